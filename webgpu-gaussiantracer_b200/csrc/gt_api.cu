@@ -229,6 +229,92 @@ static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n) {
   return GT_OK;
 }
 
+// Buffers of the per-view proxy lists (gt_stream.cu) for a launch of these
+// views, grown as needed and kept by the context (at most kListBudget bytes).
+// Entries: 24 per proxy and view to begin with (a proxy meets 2 to 4 bins of a
+// 1080p view of the 1M-Gaussian scene), more once a call that was waited for
+// has reported a larger need; the tiles of bins whose lists do not fit are
+// traced by the warp-per-ray kernel.  Views the lists cannot serve, and
+// launches whose projection records or bins alone would take half the
+// budget, get none (the hierarchy kernels trace them).
+constexpr uint64_t kListBudget = 8ull << 30;
+static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
+                              const LaunchShape& shape, Lists* out, Handoff* hand) {
+  *out = Lists{};
+  if (shape.packet != 2 || !stream_views(views, n, total_tiles, ctx->faces)) return GT_OK;
+  const StreamPlan plan = stream_plan(rays, ctx->num_sms);
+  if (plan.rays == 0) return GT_OK;
+  const uint64_t bins = total_tiles >> plan.shift;
+  uint64_t recs = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    views[i].rec_begin = (uint32_t)recs;
+    recs += views[i].s.n_kept;
+  }
+  constexpr uint64_t kRec = 3 * sizeof(float4) + sizeof(float), kEnt = sizeof(float4) + sizeof(uint2);
+  constexpr uint64_t kBin = (4ull << kListBucketBits) + 4;
+  const uint64_t fixed = recs * kRec + bins * kBin;
+  if (fixed > kListBudget / 2 || recs >= (1ull << 31)) return GT_OK;
+  uint64_t want = std::max<uint64_t>(recs * 24 + (1u << 20), ctx->lists_need + ctx->lists_need / 4ull);
+  want = std::min<uint64_t>(std::min<uint64_t>(want, (kListBudget - fixed) / kEnt), 1ull << 30);
+  Lists& L = ctx->lists;
+  if (n > ctx->lists_views || recs > ctx->lists_recs || bins > ctx->lists_bins || want > L.cap ||
+      rays > ctx->redo_cap) {
+    cudaStreamSynchronize(ctx->stream);
+    drop_graphs(ctx);  // captured graphs hold the old addresses
+    auto grow = [](auto** p, uint64_t count) {
+      cudaFree(*p);
+      *p = nullptr;
+      return cudaMalloc(p, count * sizeof(**p));
+    };
+    cudaError_t e = cudaSuccess;
+    if (n > ctx->lists_views) {
+      ctx->lists_views = 0;
+      const uint32_t c = n + n / 2;
+      e = grow(&L.views, c);
+      if (e == cudaSuccess) e = grow(&L.range, 2ull * c);
+      if (e == cudaSuccess) ctx->lists_views = c;
+    }
+    if (e == cudaSuccess && recs > ctx->lists_recs) {
+      ctx->lists_recs = 0;
+      e = grow(&L.rec, 2 * recs);
+      if (e == cudaSuccess) e = grow(&L.box, recs);
+      if (e == cudaSuccess) e = grow(&L.far, recs);
+      if (e == cudaSuccess) ctx->lists_recs = recs;
+    }
+    if (e == cudaSuccess && bins > ctx->lists_bins) {
+      ctx->lists_bins = 0;
+      e = grow(&L.cells, bins << kListBucketBits);
+      if (e == cudaSuccess) e = grow(&L.bin_base, bins + 1);
+      if (e == cudaSuccess) ctx->lists_bins = bins;
+    }
+    if (e == cudaSuccess && want > L.cap) {
+      L.cap = 0;
+      e = grow(&L.ent_box, want);
+      if (e == cudaSuccess) e = grow(&L.ent, want);
+      if (e == cudaSuccess) L.cap = (uint32_t)want;
+    }
+    if (e == cudaSuccess && !L.spill) {  // 16 warps an SM of 32 rays each
+      const uint64_t b = (uint64_t)ctx->num_sms * 16u * kStreamSpill * 32u * sizeof(unsigned long long);
+      e = cudaMalloc(&L.spill, b);
+      if (e == cudaSuccess) L.spill_bytes = b;
+    }
+    if (e == cudaSuccess && rays > ctx->redo_cap) {
+      ctx->redo_cap = 0;
+      e = grow(&ctx->d_redo, rays);
+      if (e == cudaSuccess) ctx->redo_cap = rays;
+    }
+    if (e != cudaSuccess) {  // (no room: the hierarchy kernels)
+      (void)cudaGetLastError();
+      return GT_OK;
+    }
+  }
+  *out = L;
+  out->shift = plan.shift;
+  out->rays = plan.rays;
+  hand->redo = ctx->d_redo;
+  return GT_OK;
+}
+
 static SceneDev scene_dev(const gt_scene* s) {
   SceneDev d;
   d.nodes8 = s->b.nodes8;
@@ -284,7 +370,7 @@ static void fill_stats(const DevCounters& c, gt_render_stats* st) {
   st->node_visits = c.node_visits;
   st->anyhits = c.anyhits;
   st->status_flags = c.status;
-  st->handed = c.handoff;
+  st->handed = c.handoff + c.redo;
 }
 
 static std::tuple<uint64_t, uint32_t, uint32_t, uint32_t> tune_key(const gt_scene* s, uint32_t w, uint32_t h,
@@ -293,9 +379,15 @@ static std::tuple<uint64_t, uint32_t, uint32_t, uint32_t> tune_key(const gt_scen
                          (uint32_t)log2((double)std::max<uint64_t>((uint64_t)w * h, 1)), kmax_for(k), 0u);
 }
 
+// gt_tune_result::_pad of a result that stands for the default launch over
+// per-view lists (gt_set_tune takes it back; the other fields then count only
+// for launches that the lists cannot serve).
+constexpr uint32_t kTuneLists = 0x4C495354u;
+
 // The launch shape a tuning result stands for.
 static LaunchShape shape_of(const gt_tune_result& r) {
   LaunchShape sh;
+  if (r._pad == kTuneLists) return sh;
   // block_threads 32: tile packets with this k-buffer; 128: a warp per ray
   sh.packet = r.block_threads == 32 ? 1u : 0u;
   if (sh.packet)
@@ -327,6 +419,10 @@ LaunchShape api_batch_shape_for(gt_context* ctx, const gt_scene* const* scenes, 
 void api_fill_stats(const DevCounters& c, gt_render_stats* st) { fill_stats(c, st); }
 gt_status api_ensure_views(gt_context* ctx, uint32_t n) { return ensure_views(ctx, n); }
 gt_status api_ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out) { return ensure_handoff(ctx, rays, out); }
+gt_status api_ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
+                           const LaunchShape& shape, Lists* lists, Handoff* hand) {
+  return ensure_lists(ctx, views, n, total_tiles, rays, shape, lists, hand);
+}
 gt_status api_assign_colours(gt_context* ctx, ViewDev* views, uint32_t n) { return assign_colours(ctx, views, n); }
 }  // namespace gt
 
@@ -402,6 +498,10 @@ extern "C" gt_status gt_context_destroy(gt_context* ctx) {
   cudaFreeHost(ctx->h_views);
   cudaFree(ctx->staging);
   cudaFree(ctx->colours);
+  for (void* p : {(void*)ctx->lists.views, (void*)ctx->lists.rec, (void*)ctx->lists.box, (void*)ctx->lists.far, (void*)ctx->lists.range,
+                  (void*)ctx->lists.cells, (void*)ctx->lists.bin_base, (void*)ctx->lists.ent_box,
+                  (void*)ctx->lists.ent, (void*)ctx->lists.spill, (void*)ctx->d_redo})
+    cudaFree(p);
   delete ctx->copy_pool;
   for (int b = 0; b < 2; ++b) {
     if (ctx->up_pinned[b]) cudaFreeHost(ctx->up_pinned[b]);
@@ -588,6 +688,7 @@ static gt_status finish_call(gt_context* ctx, gt_render_stats* stats, uint64_t k
   API_CUDA(ctx, cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
   API_CUDA(ctx, cudaEventRecord(ctx->call1, ctx->stream));
   API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->lists_need = ctx->h_ctr->list_pairs;
   if (stats) {
     memset(stats, 0, sizeof *stats);
     fill_stats(*ctx->h_ctr, stats);
@@ -670,8 +771,11 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
   Handoff hand;
   st = ensure_handoff(ctx, (uint64_t)w * h, &hand);
   if (st != GT_OK) return st;
+  Lists lists;
+  st = ensure_lists(ctx, &v, 1, v.n_tiles, (uint64_t)w * h, shape, &lists, &hand);
+  if (st != GT_OK) return st;
   Err e = launch_trace(&v, 1, v.n_tiles, ctx->d_ctr, ctx->faces, shape, ctx->num_sms, ctx->stream, &ctx->launches,
-                       ctx->d_views, nullptr, &hand);
+                       ctx->d_views, nullptr, &hand, &lists);
   if (e.code != GT_OK) return fail(ctx, e);
   API_CUDA(ctx, cudaEventRecord(ctx->ring[2 * slot + 1], ctx->stream));
   if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !direct)
@@ -853,9 +957,13 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
   auto bt = ctx->batch_tune.find(std::make_tuple(count, total_tiles, kmax));
   LaunchShape shape = bt != ctx->batch_tune.end() ? shape_of(bt->second)
                                                   : shape_for(ctx, items[0].scene, items[0].w, items[0].h, items[0].u.k);
+  // before the graph is looked up: growing the lists drops the graphs
+  Lists lists;
+  st = ensure_lists(ctx, ctx->h_views, count, total_tiles, all_pixels, shape, &lists, &hand);
+  if (st != GT_OK) return st;
   // the view table is rebuilt on every call: it takes the shape's k-buffer
   // size and leaf batch here, and the graph's kernel matches its slot count
-  const bool packet = packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, shape, false);
+  const bool packet = !lists.cap && packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, shape, false);
   apply_shape(ctx->h_views, count, shape);
   uint32_t kb_max = 1, pkb_max = 1;
   bool any_debug = false;  // the graph's kernel is the debug-mode instantiation
@@ -867,7 +975,8 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
   // the kernels of the graph: warp-per-ray slots per lane, and with tile
   // packets their heap size and handoff
   auto key = std::make_tuple(count, total_tiles,
-                             kmax | (any_debug ? 0x10000u : 0u) | (packet ? 0x20000u : 0u) | (colours ? 0x40000u : 0u),
+                             kmax | (any_debug ? 0x10000u : 0u) | (packet ? 0x20000u : 0u) | (colours ? 0x40000u : 0u) |
+                                 (lists.cap ? (lists.rays << 20) | 0x80000u : 0u),
                              shape.blocks_per_sm,
                              ((kb_max + 31u) / 32u) | (packet ? (pkb_max << 8) | (shape.handoff_after << 16) : 0u));
   auto it = ctx->graphs.find(key);
@@ -879,7 +988,7 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
     // launch_trace re-uploads the view table; inside the graph it copies from
     // the pinned staging table, which is refreshed before every replay.
     Err e = launch_trace(ctx->h_views, count, total_tiles, ctx->d_ctr, ctx->faces, shape, ctx->num_sms, cs,
-                         &ctx->launches, ctx->d_views, nullptr, &hand);
+                         &ctx->launches, ctx->d_views, nullptr, &hand, &lists);
     cudaError_t ce = cudaStreamEndCapture(cs, &g.graph);
     if (e.code != GT_OK) return fail(ctx, e);
     if (ce != cudaSuccess) return fail(ctx, GT_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
@@ -939,6 +1048,9 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
   Handoff hand;
   st = ensure_handoff(ctx, (uint64_t)w * h, &hand);
   if (st != GT_OK) return st;
+  Lists lists;
+  st = ensure_lists(ctx, &v, 1, v.n_tiles, (uint64_t)w * h, LaunchShape(), &lists, &hand);
+  if (st != GT_OK) return st;
   // fastest of `reps` launches of one shape
   auto time_shape = [&](const LaunchShape& sh, int reps, float* out_ms) -> gt_status {
     float ms_min = 1e30f;
@@ -946,7 +1058,7 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
       API_CUDA(ctx, cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), ctx->stream));
       API_CUDA(ctx, cudaEventRecord(ctx->int0, ctx->stream));
       Err e = launch_trace(&v, 1, v.n_tiles, ctx->d_ctr, ctx->faces, sh, ctx->num_sms, ctx->stream, &ctx->launches,
-                           ctx->d_views, nullptr, &hand);
+                           ctx->d_views, nullptr, &hand, sh.packet == 2 ? &lists : nullptr);
       if (e.code != GT_OK) return fail(ctx, e);
       API_CUDA(ctx, cudaEventRecord(ctx->int1, ctx->stream));
       API_CUDA(ctx, cudaEventSynchronize(ctx->int1));
@@ -962,6 +1074,9 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
   float best = 1e30f, def = 0.0f;
   st = time_shape(LaunchShape(), 3, &def);
   if (st != GT_OK) return st;
+  float pk_best = 1e30f;
+  LaunchShape pk_sh;
+  if (lists.cap) best = def;  // 0. the default: per-view lists
   // 1. tile packets: k-buffer entries per ray, then the hand-off point of
   // the fastest
   const uint32_t pkbufs[] = {k, 24u, 32u, 48u, 64u};
@@ -974,13 +1089,17 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
     float ms = 0.0f;
     st = time_shape(sh, 3, &ms);
     if (st != GT_OK) return st;
-    if (ms < best) {
-      best = ms;
-      best_sh = sh;
+    if (ms < pk_best) {
+      pk_best = ms;
+      pk_sh = sh;
     }
   }
-  if (best_sh.packet == 1) {
-    const LaunchShape kb_sh = best_sh;
+  if (pk_best < best) {
+    best = pk_best;
+    best_sh = pk_sh;
+  }
+  if (pk_sh.packet == 1) {
+    const LaunchShape kb_sh = pk_sh;
     // (64: only once every tile of the launch is taken)
     for (uint32_t ha : {2u, 4u, 6u, 8u, 64u}) {
       LaunchShape sh = kb_sh;
@@ -1034,6 +1153,7 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
   }
   gt_tune_result r;
   memset(&r, 0, sizeof r);
+  if (best_sh.packet == 2) r._pad = kTuneLists;
   r.block_threads = best_sh.packet ? 32u : 128u;
   r.blocks_per_sm = best_sh.blocks_per_sm;
   r.tile_w = 8;
@@ -1091,13 +1211,16 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
   }
   st = assign_colours(ctx, ctx->h_views, count);  // as gt_render_batch renders it
   if (st != GT_OK) return st;
+  Lists lists;
+  st = ensure_lists(ctx, ctx->h_views, count, total_tiles, pixels, LaunchShape(), &lists, &hand);
+  if (st != GT_OK) return st;
   auto time_shape = [&](const LaunchShape& sh, int reps, float* out_ms) -> gt_status {
     float ms_min = 1e30f;
     for (int rep = 0; rep < reps; ++rep) {
       API_CUDA(ctx, cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), ctx->stream));
       API_CUDA(ctx, cudaEventRecord(ctx->int0, ctx->stream));
       Err e = launch_trace(ctx->h_views, count, total_tiles, ctx->d_ctr, ctx->faces, sh, ctx->num_sms, ctx->stream,
-                           &ctx->launches, ctx->d_views, nullptr, &hand);
+                           &ctx->launches, ctx->d_views, nullptr, &hand, sh.packet == 2 ? &lists : nullptr);
       if (e.code != GT_OK) return fail(ctx, e);
       API_CUDA(ctx, cudaEventRecord(ctx->int1, ctx->stream));
       API_CUDA(ctx, cudaEventSynchronize(ctx->int1));
@@ -1149,7 +1272,8 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
   }
   gt_tune_result r;
   memset(&r, 0, sizeof r);
-  const bool pk = packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, best_sh, false);
+  if (best_sh.packet == 2 && lists.cap) r._pad = kTuneLists;
+  const bool pk = r._pad || packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, best_sh, false);
   r.block_threads = pk ? 32u : 128u;
   r.blocks_per_sm = best_sh.blocks_per_sm;
   r.tile_w = 8;

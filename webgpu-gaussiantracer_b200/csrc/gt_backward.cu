@@ -637,6 +637,9 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
   if (sst != GT_OK) return sst;
   sst = api_assign_colours(ctx, vd.data(), count);  // as a plain render's
   if (sst != GT_OK) return sst;
+  Lists lists;
+  sst = api_ensure_lists(ctx, vd.data(), count, total_tiles, rays, shape, &lists, &hand);
+  if (sst != GT_OK) return sst;
   for (int attempt = 0; attempt < 3; ++attempt) {
     if (want > 0xFFFFFFF0ull) return api_fail(ctx, GT_ERR_OOM, "checkpoint needs more than 2^32 records");
     uint32_t m = mode == 1 ? 1u : (mode == 2 ? 2u : (want * (kCkptHeader + kCkptChunk) * 4 <= budget ? 1u : 2u));
@@ -654,7 +657,7 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     CK_TRY(cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), st));
     CK_TRY(cudaEventRecord(ctx->int0, st));
     Err e = launch_trace(vd.data(), count, total_tiles, ctx->d_ctr, ctx->faces, shape, ctx->num_sms, st,
-                         &ctx->launches, ctx->d_views, &c, &hand);
+                         &ctx->launches, ctx->d_views, &c, &hand, &lists);
     if (e.code != GT_OK) return api_fail(ctx, e.code, e.msg);
     CK_TRY(cudaEventRecord(ctx->int1, st));
     uint32_t used = 0;
@@ -662,6 +665,7 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     CK_TRY(cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
     CK_TRY(cudaStreamSynchronize(st));
     cudaEventElapsedTime(&ck.fwd_ms, ctx->int0, ctx->int1);
+    ctx->lists_need = ctx->h_ctr->list_pairs;
     sst = api_status_to_error(ctx, ctx->h_ctr->status);
     if (sst != GT_OK) return sst;
     if (stats) {

@@ -67,6 +67,11 @@ struct gt_context {
   cudaEvent_t up_done[2] = {nullptr, nullptr};
   gt::HandoffRay* d_handoff = nullptr;  // rays tile packets hand to the warp-per-ray kernel
   uint32_t handoff_cap = 0;
+  gt::Lists lists;                      // per-view proxy lists (gt_stream.cu)
+  uint32_t lists_views = 0;             // capacities: views, projection records, bins, redo slots
+  uint64_t lists_recs = 0, lists_bins = 0, redo_cap = 0;
+  uint32_t lists_need = 0;              // entries the last list launch that was waited for needed
+  uint32_t* d_redo = nullptr;
   cudaEvent_t call0 = nullptr, call1 = nullptr, timer0 = nullptr, timer1 = nullptr;
   cudaEvent_t int0 = nullptr, int1 = nullptr;  // library-internal timing (never the user's timer)
   cudaEvent_t ring[2 * gt::kEventRing];
@@ -106,6 +111,11 @@ LaunchShape api_batch_shape_for(gt_context* ctx, const gt_scene* const* scenes, 
 void api_fill_stats(const DevCounters& c, gt_render_stats* st);
 gt_status api_ensure_views(gt_context* ctx, uint32_t n);
 gt_status api_ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out);
+// Proxy lists for a launch of these views (shape.packet == 2 and views the
+// lists can serve), or lists->cap == 0; sets the views' rec_begin and the
+// handoff's redo list.
+gt_status api_ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
+                           const LaunchShape& shape, Lists* lists, Handoff* hand);
 // Colour tables for the plain-render views of a launch (ViewDev::rgb).
 gt_status api_assign_colours(gt_context* ctx, ViewDev* views, uint32_t n);
 // Checkpointing forward (gt_backward.cu): renders the views into `outs`

@@ -66,7 +66,9 @@ struct DevCounters {
   unsigned int status;
   unsigned int work;  // work-stealing tile counter
   unsigned int work2;    // the same for the second kernel of a launch
-  unsigned int handoff;  // rays the tile-packet kernel handed to the warp-per-ray kernel
+  unsigned int handoff;  // rays the tile kernels handed to the warp-per-ray kernel
+  unsigned int redo;       // rays that kernel traces from the start
+  unsigned int list_pairs; // list entries the launch needed (gt_stream.cu)
 };
 
 // Scene as the kernels see it.  Records of kept proxies are in BVH leaf
@@ -128,6 +130,7 @@ struct ViewDev {
   float4* grad;         // backward: the scene's per-particle sums of the response terms (4 float4 a particle)
   float4* grad_sh;      // backward: this view's per-particle sums of the colour weights (1 float4 a particle)
   uint64_t n_particles;
+  uint32_t rec_begin;   // first projection record of this view (gt_stream.cu)
   // this view's colour of every particle, max(0, SH(normalize(mu - camera)))
   // per channel (k_view_colours, before the trace launch), or null: the
   // trace kernels evaluate the SH per composited entry
@@ -143,9 +146,10 @@ struct LaunchShape {
   uint32_t tile_w = 8, tile_h = 4;  // pixel tile of the work order (tile_w*tile_h == 32)
   uint32_t kbuf = 64;               // k-buffer entries (raised to k when k is larger; <= kMaxKbuf)
   uint32_t leaf_batch = 32;         // leaf queue size that triggers proxy tests
-  // Plain renders (debugMode 0, no checkpoint) run one warp per 8x4 tile of
-  // rays (gt_packet.cu) when packet is 1, one warp per ray when it is 0, and
-  // by default (2) the tile packets when the launch has at least
+  // Renders of debugMode 0 run one warp per 8x4 tile of rays over the
+  // hierarchy (gt_packet.cu) when packet is 1, one warp per ray when it is 0.
+  // By default (2) they run over per-view proxy lists (gt_stream.cu) when the
+  // launch has lists, else as tile packets when it has at least
   // kPacketTilesPerSm tiles per SM.  The packet kernel's k-buffer has
   // packet_kbuf entries per ray (raised to k; <= kMaxPacketKbuf).
   uint32_t packet = 2;
@@ -262,6 +266,37 @@ struct HandoffRay {
 struct Handoff {
   HandoffRay* rays = nullptr;
   uint32_t cap = 0;
+  uint32_t* redo = nullptr;  // work slots to trace from the start (gt_stream.cu; one per ray of the launch)
+  uint32_t late = 0;         // gt_stream.cu: idle warps at which the tracing tiles hand over
+};
+
+// Per-view proxy lists (gt_stream.cu).
+constexpr int kListBucketBits = 10;                // distance buckets per bin
+constexpr int kStreamSpill = 96;                   // rows of a ray's column in global memory
+constexpr uint64_t kStreamMaxSlots = 1ull << 28;   // larger launches use the hierarchy kernels
+struct ListView {
+  double X[3], Y[3], Z[3];  // camera frame: right, up, view direction
+  double sx, sy, ox, oy;    // pixel x = u sx + ox
+  double inv_bw, inv_bh;    // 1 / bin size in pixels
+  float Xf[3], Yf[3], Zf[3];
+  uint32_t bins_x, bins_y;  // bins that cover the image
+  uint32_t bin_begin, rec_begin;
+};
+struct Lists {
+  ListView* views = nullptr;
+  float4* rec = nullptr;         // 2 per (view, proxy): (u0, v0, slope, g11), (g22, bound, bins x, bins y)
+  float4* box = nullptr;         // outline rectangle (u lo, u hi, v lo, v hi)
+  float* far = nullptr;          // per (view, proxy): no point of it is farther from the camera
+  uint32_t* range = nullptr;     // per view: bits of the smallest and largest bound
+  uint32_t* cells = nullptr;     // per bin 2^kListBucketBits counts, then places
+  uint32_t* bin_base = nullptr;  // start of each bin's list (one more than bins)
+  float4* ent_box = nullptr;     // list entries: outline rectangle
+  uint2* ent = nullptr;          // proxy, bits of its bucket's lower bound
+  unsigned long long* spill = nullptr;  // waiting hits past a ray's column in shared memory
+  uint64_t spill_bytes = 0;
+  uint32_t cap = 0;              // entries that fit
+  uint32_t shift = 4;            // tiles per bin: 2^shift
+  uint32_t rays = 32;            // rays per warp
 };
 
 // Trace launches (gt_trace.cu).  launch_trace writes the shape's k-buffer
@@ -278,7 +313,17 @@ Err launch_view_colours(const ViewDev* views, const ViewDev* d_views, uint32_t n
 Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCounters* counters,
                  const FaceTable& faces, const LaunchShape& shape, int num_sms, cudaStream_t stream,
                  uint64_t* launches, ViewDev* d_views_scratch, const Ckpt* ckpt = nullptr,
-                 const Handoff* handoff = nullptr);
+                 const Handoff* handoff = nullptr, const Lists* lists = nullptr);
+// Whether per-view lists can serve these views (gt_stream.cu).
+bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, const FaceTable& faces);
+struct StreamPlan {
+  uint32_t rays = 0;   // rays per warp (0: the hierarchy kernels are faster)
+  uint32_t shift = 4;  // bins of 2^shift tiles
+};
+StreamPlan stream_plan(uint64_t rays, int num_sms);
+Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n_views, uint32_t total_tiles,
+                        DevCounters* counters, const FaceTable& faces, int num_sms, cudaStream_t stream,
+                        uint64_t* launches, const Lists& lists, const Handoff& handoff, const Ckpt* ckpt);
 Err launch_trace_packet(const ViewDev* views, const ViewDev* d_views, uint32_t n_views, uint32_t total_tiles,
                         DevCounters* counters, const FaceTable& faces, int num_sms, cudaStream_t stream,
                         uint64_t* launches, const Handoff& handoff, uint32_t handoff_after,

@@ -298,7 +298,7 @@ __device__ __forceinline__ float4 trace_ray_warp(const ViewDev& V, const FaceTab
 // so neighbouring pixels run on neighbouring warps at the same time.  With
 // `resume`, the slots are instead the rays a tile-packet launch handed over
 // (DevCounters::handoff of them, at most resume_cap), continued from their
-// state.
+// state, and the slots of `redo` (DevCounters::redo of them), from the start.
 // 8 resident blocks (32 warps per SM, 64 registers a thread) beat 4 blocks
 // without spills by 12% on the 1M-Gaussian 1080p view: the kernel is bound by
 // dependent latencies, and more warps hide them better than the spill loads
@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_trace8(const ViewDev
                                                                   const __grid_constant__ FaceTable F,
                                                                   const uint32_t* pixels, uint32_t n_pix,
                                                                   const HitOut ho, const Ckpt ck,
-                                                                  const HandoffRay* resume, uint32_t resume_cap) {
+                                                                  const HandoffRay* resume, uint32_t resume_cap,
+                                                                  const uint32_t* redo) {
   __shared__ WarpScratch scratch[kWarpsPerBlock];
   const uint32_t lane = threadIdx.x & 31;
   WarpScratch& W = scratch[threadIdx.x >> 5];
@@ -317,7 +318,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_trace8(const ViewDev
   if (lane == 0) st = RayStats{0, 0, 0, 0, 0, 0};
   __syncwarp();
   uint32_t status = 0, rays = 0;
-  const uint32_t total = RECORD ? n_pix : (resume ? min(ctr->handoff, resume_cap) : total_tiles * 32u);
+  const uint32_t resumed = resume ? min(ctr->handoff, resume_cap) : 0u;
+  const uint32_t total = RECORD ? n_pix : (resume ? resumed + (redo ? ctr->redo : 0u) : total_tiles * 32u);
   while (true) {
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(resume ? &ctr->work2 : &ctr->work, 1u);
@@ -325,8 +327,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_trace8(const ViewDev
     if (item >= total) break;
     const HandoffRay* init = nullptr;
     if (!RECORD && resume) {
-      init = resume + item;
-      item = init->item;
+      if (redo && item >= resumed) {
+        item = redo[item - resumed];
+      } else {
+        init = resume + item;
+        item = init->item;
+      }
     }
     uint32_t vi = 0, px, py;
     if (RECORD) {
@@ -429,13 +435,19 @@ Err launch_view_colours(const ViewDev* views, const ViewDev* d_views, uint32_t n
 
 Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCounters* counters,
                  const FaceTable& faces, const LaunchShape& shape, int num_sms, cudaStream_t stream,
-                 uint64_t* launches, ViewDev* d_views, const Ckpt* ckpt, const Handoff* handoff) {
-  const bool packet = packet_launch(views, n_views, total_tiles, num_sms, shape, ckpt != nullptr);
+                 uint64_t* launches, ViewDev* d_views, const Ckpt* ckpt, const Handoff* handoff, const Lists* lists) {
+  const bool stream_lists = lists && lists->cap && handoff && handoff->rays && handoff->redo;
+  const bool packet = !stream_lists && packet_launch(views, n_views, total_tiles, num_sms, shape, ckpt != nullptr);
   apply_shape(views, n_views, shape);
   GT_CUDA_TRY(cudaMemcpyAsync(d_views, views, sizeof(ViewDev) * n_views, cudaMemcpyHostToDevice, stream));
   Err ce = launch_view_colours(views, d_views, n_views, num_sms, stream, launches);
   if (ce.code != GT_OK) return ce;
-  const bool hand = packet && handoff && handoff->rays && handoff->cap && shape.handoff_after;
+  const bool hand = stream_lists || (packet && handoff && handoff->rays && handoff->cap && shape.handoff_after);
+  if (stream_lists) {
+    Err e = launch_trace_stream(views, d_views, n_views, total_tiles, counters, faces, num_sms, stream, launches,
+                                *lists, *handoff, ckpt);
+    if (e.code != GT_OK) return e;
+  }
   if (packet) {
     Err e = launch_trace_packet(views, d_views, n_views, total_tiles, counters, faces, num_sms, stream, launches,
                                 hand ? *handoff : Handoff{}, shape.handoff_after, ckpt);
@@ -476,9 +488,10 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
   // after a tile-packet launch: the rays it handed over, one warp per ray
   const HandoffRay* resume = hand ? handoff->rays : nullptr;
   const uint32_t resume_cap = hand ? handoff->cap : 0u;
+  const uint32_t* redo = stream_lists ? handoff->redo : nullptr;
   if (hand) grid = (uint32_t)num_sms * std::max(1u, shape.blocks_per_sm);
   void* args[] = {(void*)&dv, (void*)&n_views, (void*)&total_tiles, (void*)&counters, (void*)&faces,
-                  (void*)&no_pix, (void*)&zero, (void*)&ho, (void*)&ck, (void*)&resume, (void*)&resume_cap};
+                  (void*)&no_pix, (void*)&zero, (void*)&ho, (void*)&ck, (void*)&resume, (void*)&resume_cap, (void*)&redo};
   GT_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, stream));
   ++*launches;
   GT_CUDA_TRY(cudaGetLastError());
@@ -494,7 +507,7 @@ Err launch_trace_hits(const ViewDev& view, ViewDev* d_views, const uint32_t* pix
   HitOut ho{out_pidx, out_t, out_alpha, out_count, out_rounds, out_rgba, max_entries};
   uint32_t grid = std::min<uint32_t>((n_pix + kWarpsPerBlock - 1) / kWarpsPerBlock, 148u * 8u);
   k_trace8<true, false, 1, true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(d_views, 1, 0, counters, faces, pixels, n_pix, ho,
-                                                                  Ckpt{}, nullptr, 0u);
+                                                                  Ckpt{}, nullptr, 0u, nullptr);
   ++*launches;
   GT_CUDA_TRY(cudaGetLastError());
   return Err{};
