@@ -1,26 +1,28 @@
-// gt_build.cu — GPU scene build: proxies, LBVH, shading records.
+// gt_build.cu — GPU scene build: proxies, hierarchy, shading records.
 //
 // Replaces the reference's host-side acceleration-structure build
 // (gaussianSceneToBvh, src/main.ts:30-111; Tlas.build,
 // webrtx/src/wasm_bvh_builder.ts:260-377; build_blas/build_tlas,
-// webrtx/bvh/src/lib.rs:254-347, 512-603) with a linear BVH built on the GPU:
+// webrtx/bvh/src/lib.rs:254-347, 512-603) with a hierarchy built on the GPU:
 //
-//   1. keep flags (opacity > alpha_min) and an exclusive scan  -> kept list
-//   2. per kept particle: proxy matrix M = T R diag(s*scale), world AABB of
-//      the 12 transformed icosahedron vertices, box centre, scene bounds
-//   3. 30-bit Morton codes of the box centres
-//   4. LSD radix sort of (code, kept slot), 4 passes of 8 bits, hand-written
+//   1. one pass over the packed records (k_records): keep flags (opacity >
+//      alpha_min), shading records in particle order (mean, opacity, precision
+//      matrix, SH), proxy matrix M = T R diag(s*scale) and its inverse, world
+//      AABB of the 12 transformed icosahedron vertices, bounds of the centres
+//   2. an exclusive scan of the flags, 30-bit Morton codes of the box centres
+//   3. LSD radix sort of (code, particle), 4 passes of 8 bits, hand-written
 //      (per-tile histograms, one scan, stable warp-ranked scatter)
-//   5. Karras (2012) hierarchy over the sorted codes, ties broken by index
-//   6. bottom-up refit with one atomic arrival counter per internal node
-//   7. leaf records in leaf order (world-to-object map, particle index) and
-//      shading records in particle order (mean, opacity, precision matrix, SH)
+//   4. leaf records in leaf order (world-to-object map, particle index, box)
+//   5. binary hierarchy: H-PLOC (gt_ploc.cu), or with fast_build Karras (2012)
+//      over the sorted codes, ties broken by index, and a bottom-up refit
+//   6. checks, and the greedy 8-wide collapse
 //
 // Node layout (4 x float4 per internal node; children's boxes in the parent):
 //   f0 = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)
 //   f1 = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
 //   f2 = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
 //   f3 = (child0, child1, 0, 0) as uint bits; kLeafBit | j marks leaf j.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
 
@@ -191,18 +193,6 @@ __device__ __forceinline__ void affine_inverse(const float M[12], float W[12]) {
   W[11] = -((W[2] * p.x + W[5] * p.y) + W[8] * p.z);
 }
 
-__device__ __forceinline__ const float* record(const uint8_t* packed, uint64_t i, uint32_t stride) {
-  return reinterpret_cast<const float*>(packed + i * (uint64_t)stride);
-}
-
-__global__ void k_keep_flags(const uint8_t* packed, uint64_t n, uint32_t stride, double alpha_min,
-                             const double* act64, uint32_t* flags) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double o = act64 ? act64[8 * i] : (double)record(packed, i, stride)[12];
-  flags[i] = (o > alpha_min) ? 1u : 0u;
-}
-
 // float min/max through order-preserving integer maps (for atomics)
 __device__ __forceinline__ uint32_t f2ord(float f) {
   uint32_t u = __float_as_uint(f);
@@ -212,46 +202,152 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-__global__ void k_proxy_boxes(const uint8_t* packed, uint64_t n, uint32_t stride, double alpha_min,
-                              const double* act64, const uint32_t* flags, const uint32_t* slots, const IcoVerts iv, float* box,
-                              uint32_t* kept_pidx, uint32_t* bounds_ord) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+// Everything the build takes from the packed records, in one pass over them:
+// the keep flag, and for kept particles the shading records ((mu, opacity),
+// the precision matrix A of computeResponse (6 unique entries), the SH floats
+// made tight, scale and rotation), the proxy's world-to-object map and padded
+// world box, and the bounds of the box centres.
+//
+// Bound by HBM: 320 bytes a record read, 344 written (0.66 GB for 1M).  The
+// usual 320-byte records are read as coalesced quads, whose SH part leaves
+// again as coalesced quads (the particles that are not kept included); only
+// the head goes through shared memory (rows of an odd number of words: a
+// thread a record reads without bank conflicts).  Other strides stage whole
+// records.  Three kernels with a thread a record reading it from global memory
+// took 191 + 191 + 22 us for 1M records on a B200, and the leaves' gather of
+// the records 68; this takes 115 (231 with an atomic of every warp on the
+// shared bounds).
+constexpr uint32_t kRecBlock = 64;
+
+// FULL: 320-byte records of 16 coefficients on 16-byte boundaries.
+template <bool FULL>
+__global__ void __launch_bounds__(kRecBlock) k_records(const uint8_t* __restrict__ packed, uint64_t n, uint32_t stride,
+                                                       uint32_t n_sh, double alpha_min,
+                                                       const double* __restrict__ act64, const IcoVerts iv,
+                                                       uint32_t* __restrict__ flags, float4* __restrict__ shade,
+                                                       float4* __restrict__ sh, float4* __restrict__ params,
+                                                       float4* __restrict__ w2o, float* __restrict__ box,
+                                                       uint32_t* bounds_ord) {
+  extern __shared__ float rows[];
+  __shared__ uint32_t kept_s[kRecBlock];
+  // the words of a record that are read: the head and the SH rows present
+  const uint32_t words = FULL ? 16u : min(stride / 4u, 16u + 4u * n_sh), pitch = words | 1u;
+  const uint64_t p0 = (uint64_t)blockIdx.x * kRecBlock;
+  const uint32_t cnt = (uint32_t)min((uint64_t)kRecBlock, n - p0);
+  const uint8_t* src = packed + p0 * stride;
+  if (FULL) {
+    // 20 quads a record, ten loads of a thread in flight at a time.  Four
+    // lanes hold four quads of one record: its head (quads 0-3), which goes
+    // to shared memory, or four coefficients, three floats each of 12 that
+    // leave as three quads.
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      float4 v[10];
+#pragma unroll
+      for (uint32_t i = 0; i < 10; ++i) {
+        const uint32_t at = (h * 10 + i) * kRecBlock + threadIdx.x;
+        v[i] = at < cnt * 20u ? __ldcs(reinterpret_cast<const float4*>(src) + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < 10; ++i) {
+        const uint32_t at = (h * 10 + i) * kRecBlock + threadIdx.x;
+        const uint32_t r = at / 20u, q = at % 20u, g = q / 4u, l = q % 4u;
+        const float nx = __shfl_down_sync(0xFFFFFFFFu, v[i].x, 1), ny = __shfl_down_sync(0xFFFFFFFFu, v[i].y, 1),
+                    nz = __shfl_down_sync(0xFFFFFFFFu, v[i].z, 1);
+        if (at >= cnt * 20u) continue;
+        if (g == 0) {
+          float* d = rows + r * pitch + 4u * l;
+          d[0] = v[i].x;
+          d[1] = v[i].y;
+          d[2] = v[i].z;
+          d[3] = v[i].w;
+        } else if (l < 3u) {
+          sh[12 * (p0 + r) + 3u * (g - 1u) + l] = l == 0   ? make_float4(v[i].x, v[i].y, v[i].z, nx)
+                                                  : l == 1 ? make_float4(v[i].y, v[i].z, nx, ny)
+                                                           : make_float4(v[i].z, nx, ny, nz);
+        }
+      }
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < cnt * words; i += kRecBlock) {
+      const uint32_t r = i / words, w = i - r * words;
+      rows[r * pitch + w] = __ldg(reinterpret_cast<const float*>(src + (size_t)r * stride) + w);
+    }
+  }
+  __syncthreads();
+  const uint64_t p = p0 + threadIdx.x;
   float cmin[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, cmax[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
   float bmag = 0.0f;
-  if (i < n && flags[i]) {
-    const float* rec = record(packed, i, stride);
-    float M[12];
-    proxy_o2w(rec, activation(rec, act64, i), alpha_min, M);
-    Affine A;
+  bool kept = false;
+  if (threadIdx.x < cnt) {
+    const float* rec = rows + threadIdx.x * pitch;
+    const Act64 act = activation(rec, act64, p);
+    kept = act.o > alpha_min;
+    flags[p] = kept ? 1u : 0u;
+    if (kept) {
+      const float q[4] = {rec[8], rec[9], rec[10], rec[11]};
+      const float sc[3] = {rec[4], rec[5], rec[6]};
+      float A[3][3];
+      precision_matrix(q, sc, A);
+      shade[3 * p] = make_float4(rec[0], rec[1], rec[2], rec[12]);
+      shade[3 * p + 1] = make_float4(A[0][0], A[1][0], A[2][0], A[1][1]);
+      shade[3 * p + 2] = make_float4(A[2][1], A[2][2], 0.f, 0.f);
+      params[2 * p] = make_float4(sc[0], sc[1], sc[2], 0.f);
+      params[2 * p + 1] = make_float4(q[0], q[1], q[2], q[3]);
+      float M[12], W[12];
+      proxy_o2w(rec, act, alpha_min, M);
+      affine_inverse(M, W);
+      w2o[3 * p] = make_float4(W[0], W[1], W[2], W[3]);
+      w2o[3 * p + 1] = make_float4(W[4], W[5], W[6], W[7]);
+      w2o[3 * p + 2] = make_float4(W[8], W[9], W[10], W[11]);
+      Affine T;
 #pragma unroll
-    for (int q = 0; q < 12; ++q) A.m[q] = M[q];
-    float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+      for (int c = 0; c < 12; ++c) T.m[c] = M[c];
+      float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-    for (int v = 0; v < 12; ++v) {
-      V3 w = xpoint(A, mk(iv.v[3 * v], iv.v[3 * v + 1], iv.v[3 * v + 2]));
-      lo[0] = fminf(lo[0], w.x); lo[1] = fminf(lo[1], w.y); lo[2] = fminf(lo[2], w.z);
-      hi[0] = fmaxf(hi[0], w.x); hi[1] = fmaxf(hi[1], w.y); hi[2] = fmaxf(hi[2], w.z);
+      for (int v = 0; v < 12; ++v) {
+        V3 w = xpoint(T, mk(iv.v[3 * v], iv.v[3 * v + 1], iv.v[3 * v + 2]));
+        lo[0] = fminf(lo[0], w.x); lo[1] = fminf(lo[1], w.y); lo[2] = fminf(lo[2], w.z);
+        hi[0] = fmaxf(hi[0], w.x); hi[1] = fmaxf(hi[1], w.y); hi[2] = fmaxf(hi[2], w.z);
+      }
+      float ext = fmaxf(fmaxf(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
+      float mag = 0.0f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) mag = fmaxf(mag, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
+      // conservative padding for the rounding of the vertex transform
+      float pad = __fmaf_rn(1e-5f, ext, 2e-6f * (mag + 1.0f));
+      float* b = box + 6 * p;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float b0 = lo[a] - pad, b1 = hi[a] + pad;
+        b[a] = b0;
+        b[3 + a] = b1;
+        float c = 0.5f * (b0 + b1);
+        cmin[a] = c;
+        cmax[a] = c;
+        bmag = fmaxf(bmag, fmaxf(fabsf(b0), fabsf(b1)));
+      }
     }
-    float ext = fmaxf(fmaxf(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
-    float mag = 0.0f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) mag = fmaxf(mag, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
-    // conservative padding for the rounding of the vertex transform
-    float pad = __fmaf_rn(1e-5f, ext, 2e-6f * (mag + 1.0f));
-    uint32_t s = slots[i];
-    float* b = box + 6 * (size_t)s;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      b[a] = lo[a] - pad;
-      b[3 + a] = hi[a] + pad;
-      float c = 0.5f * (b[a] + b[3 + a]);
-      cmin[a] = c;
-      cmax[a] = c;
-      bmag = fmaxf(bmag, fmaxf(fabsf(b[a]), fabsf(b[3 + a])));
-    }
-    kept_pidx[s] = (uint32_t)i;
   }
-  // warp-reduce the centre bounds, then one atomic per warp
+  if (!FULL) {
+    kept_s[threadIdx.x] = kept ? 1u : 0u;
+    __syncthreads();
+    // SH rows: float 3k + ch of a row is coefficient k, channel ch
+    for (uint32_t i = threadIdx.x; i < cnt * 12u; i += kRecBlock) {
+      const uint32_t r = i / 12u, q = i - 12u * r;
+      if (!kept_s[r]) continue;
+      const float* rec = rows + r * pitch + 16;
+      float v[4];
+#pragma unroll
+      for (uint32_t c = 0; c < 4; ++c) {
+        const uint32_t f = 4 * q + c, k = f / 3u, ch = f - 3u * k;
+        v[c] = k < n_sh ? rec[4 * k + ch] : 0.0f;
+      }
+      sh[12 * (p0 + r) + q] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+  // the block's centre bounds, and atomics only for those that move the
+  // totals (an atomic of every warp on one sector takes longer than the pass)
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
 #pragma unroll
@@ -263,12 +359,15 @@ __global__ void k_proxy_boxes(const uint8_t* packed, uint64_t n, uint32_t stride
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) bmag = fmaxf(bmag, __shfl_xor_sync(0xFFFFFFFFu, bmag, off));
   if ((threadIdx.x & 31) == 0 && cmin[0] <= cmax[0]) {
+    const uint4 now0 = __ldcg(reinterpret_cast<const uint4*>(bounds_ord)),
+                now1 = __ldcg(reinterpret_cast<const uint4*>(bounds_ord) + 1);
+    const uint32_t now[7] = {now0.x, now0.y, now0.z, now0.w, now1.x, now1.y, now1.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      atomicMin(&bounds_ord[a], f2ord(cmin[a]));
-      atomicMax(&bounds_ord[3 + a], f2ord(cmax[a]));
+      if (f2ord(cmin[a]) < now[a]) atomicMin(&bounds_ord[a], f2ord(cmin[a]));
+      if (f2ord(cmax[a]) > now[3 + a]) atomicMax(&bounds_ord[3 + a], f2ord(cmax[a]));
     }
-    atomicMax(&bounds_ord[6], f2ord(bmag));
+    if (f2ord(bmag) > now[6]) atomicMax(&bounds_ord[6], f2ord(bmag));
   }
 }
 
@@ -281,23 +380,24 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   return v;
 }
 
-__global__ void k_morton(const float* box, uint32_t m, const uint32_t* bounds_ord, uint32_t* keys,
-                         uint32_t* vals) {
-  uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
+// Morton code of every kept particle's box centre, with the particle's index.
+__global__ void k_morton(const float* box, uint64_t n, const uint32_t* flags, const uint32_t* slots,
+                         const uint32_t* bounds_ord, uint32_t* keys, uint32_t* vals) {
+  const uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (p >= n || !flags[p]) return;
   uint32_t code = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     float lo = ord2f(bounds_ord[a]), hi = ord2f(bounds_ord[3 + a]);
-    float c = 0.5f * (box[6 * (size_t)j + a] + box[6 * (size_t)j + 3 + a]);
+    float c = 0.5f * (box[6 * p + a] + box[6 * p + 3 + a]);
     float e = hi - lo;
     float u = e > 0.0f ? (c - lo) / e : 0.0f;
     u = fminf(fmaxf(u, 0.0f), 1.0f);
     uint32_t q = (uint32_t)(u * 1023.0f);
     code |= spread10(q) << (2 - a);
   }
-  keys[j] = code;
-  vals[j] = j;
+  keys[slots[p]] = code;
+  vals[slots[p]] = (uint32_t)p;
 }
 
 // ------------------------------------------------------------------ scan
@@ -516,23 +616,18 @@ __global__ void k_karras(const uint32_t* keys, int n, float4* nodes, uint32_t* p
 }
 
 // Leaf records in leaf order: world-to-object map, particle index, box.
-__global__ void k_leaves(const uint8_t* packed, uint32_t stride, double alpha_min, const double* act64,
-                         const uint32_t* sorted_slots, uint32_t m, const uint32_t* kept_pidx, const float* box_by_slot, float4* w2o,
-                         uint32_t* leaf_pidx, float* leaf_box) {
+__global__ void k_leaves(const uint32_t* sorted_pidx, uint32_t m, const float4* w2o_by_particle,
+                         const float* box_by_particle, float4* w2o, uint32_t* leaf_pidx, float* leaf_box) {
   uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= m) return;
-  uint32_t slot = sorted_slots[j];
-  uint32_t p = kept_pidx[slot];
-  float M[12], W[12];
-  const float* rec = record(packed, p, stride);
-  proxy_o2w(rec, activation(rec, act64, p), alpha_min, M);
-  affine_inverse(M, W);
-  w2o[3 * (size_t)j] = make_float4(W[0], W[1], W[2], W[3]);
-  w2o[3 * (size_t)j + 1] = make_float4(W[4], W[5], W[6], W[7]);
-  w2o[3 * (size_t)j + 2] = make_float4(W[8], W[9], W[10], W[11]);
-  leaf_pidx[j] = p;
+  const uint32_t p = sorted_pidx[j];
 #pragma unroll
-  for (int a = 0; a < 6; ++a) leaf_box[6 * (size_t)j + a] = box_by_slot[6 * (size_t)slot + a];
+  for (int q = 0; q < 3; ++q) w2o[3 * (size_t)j + q] = __ldg(w2o_by_particle + 3 * (size_t)p + q);
+  leaf_pidx[j] = p;
+  const float2* b = reinterpret_cast<const float2*>(box_by_particle) + 3 * (size_t)p;
+  float2* o = reinterpret_cast<float2*>(leaf_box) + 3 * (size_t)j;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) o[a] = __ldg(b + a);
 }
 
 __device__ __forceinline__ void child_box(uint32_t ref, const float* leaf_box, const float* ibox, float b[6]) {
@@ -571,7 +666,8 @@ __global__ void k_refit(uint32_t m, const float* leaf_box, float* ibox, float4* 
 
 // Tree check before any traversal: every child reference in range and every
 // node reached by exactly one parent (the root by none).
-__global__ void k_check_children(uint32_t m, const float4* nodes, uint32_t* refcount, uint32_t* bad) {
+__global__ void k_check_children(uint32_t m, const float4* nodes, uint32_t* refcount, const uint32_t* root,
+                                 uint32_t* bad) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i + 1 >= m) return;
   float4 f3 = nodes[4 * (size_t)i + 3];
@@ -583,14 +679,14 @@ __global__ void k_check_children(uint32_t m, const float4* nodes, uint32_t* refc
       uint32_t j = r & ~kLeafBit;
       if (j >= m) atomicOr(bad, 1u); else atomicAdd(&refcount[(m - 1) + j], 1u);
     } else {
-      if (r >= m - 1 || r == 0) atomicOr(bad, 2u); else atomicAdd(&refcount[r], 1u);
+      if (r >= m - 1 || r == *root) atomicOr(bad, 2u); else atomicAdd(&refcount[r], 1u);
     }
   }
 }
-__global__ void k_check_counts(uint32_t total, const uint32_t* refcount, uint32_t* bad) {
+__global__ void k_check_counts(uint32_t total, const uint32_t* refcount, const uint32_t* root, uint32_t* bad) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  uint32_t expect = i == 0 ? 0u : 1u;
+  uint32_t expect = i == *root ? 0u : 1u;
   if (refcount[i] != expect) atomicOr(bad, 4u);
 }
 
@@ -605,31 +701,6 @@ __global__ void k_depth(uint32_t m, const uint32_t* parent_int, const uint32_t* 
   atomicMax(depth, d);
 }
 
-// Shading records in particle order: (mu, opacity), precision matrix A of
-// computeResponse (6 unique entries), and the 48 SH floats made tight.
-__global__ void k_shade(const uint8_t* packed, uint64_t n, uint32_t stride, uint32_t n_sh, const uint32_t* flags,
-                        float4* shade, float4* sh, float4* params) {
-  uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (p >= n || !flags[p]) return;
-  const float* rec = record(packed, p, stride);
-  float q[4] = {rec[8], rec[9], rec[10], rec[11]};
-  float sc[3] = {rec[4], rec[5], rec[6]};
-  float A[3][3];
-  precision_matrix(q, sc, A);
-  shade[3 * p] = make_float4(rec[0], rec[1], rec[2], rec[12]);
-  params[2 * p] = make_float4(sc[0], sc[1], sc[2], 0.f);
-  params[2 * p + 1] = make_float4(q[0], q[1], q[2], q[3]);
-  shade[3 * p + 1] = make_float4(A[0][0], A[1][0], A[2][0], A[1][1]);
-  shade[3 * p + 2] = make_float4(A[2][1], A[2][2], 0.f, 0.f);
-  float v[48];
-#pragma unroll
-  for (int k = 0; k < 16; ++k)
-#pragma unroll
-    for (int ch = 0; ch < 3; ++ch) v[3 * k + ch] = (uint32_t)k < n_sh ? rec[16 + 4 * k + ch] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < 12; ++i) sh[12 * p + i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-}
-
 // ------------------------------------------------------------- BVH8 collapse
 // Greedy collapse of the binary hierarchy into 8-wide nodes: a node starts
 // with the two children of a binary node and repeatedly opens its internal
@@ -642,87 +713,111 @@ __global__ void k_shade(const uint8_t* packed, uint64_t n, uint32_t stride, uint
 //   f0 = (lo.x, lo.y, lo.z, hi.x), f1 = (hi.y, hi.z, ref, 0)
 // ref = kLeafBit | j for leaf j, an 8-wide node index, or kInvalid (empty
 // slot, with an empty box).
-struct Entry8 {
-  float b[6];
-  uint32_t ref;  // binary reference: kLeafBit | j or internal index
-};
-
-__device__ __forceinline__ void binary_children(const float4* bn, uint32_t i, Entry8& c0, Entry8& c1) {
-  float4 f0 = bn[4 * (size_t)i], f1 = bn[4 * (size_t)i + 1], f2 = bn[4 * (size_t)i + 2], f3 = bn[4 * (size_t)i + 3];
-  c0.b[0] = f0.x; c0.b[3] = f0.y; c0.b[1] = f0.z; c0.b[4] = f0.w; c0.b[2] = f2.x; c0.b[5] = f2.y;
-  c1.b[0] = f1.x; c1.b[3] = f1.y; c1.b[1] = f1.z; c1.b[4] = f1.w; c1.b[2] = f2.z; c1.b[5] = f2.w;
-  c0.ref = __float_as_uint(f3.x);
-  c1.ref = __float_as_uint(f3.y);
-}
-
 __device__ __forceinline__ float half_area(const float b[6]) {
   float x = b[3] - b[0], y = b[4] - b[1], z = b[5] - b[2];
   return x * y + y * z + z * x;
 }
 
-__global__ void k_collapse8(const float4* bn, const uint32_t* front_bin, const uint32_t* front_n8, uint32_t n_front,
-                            float4* nodes8, uint32_t* next_bin, uint32_t* next_n8, uint32_t* counters,
-                            uint32_t max_nodes8) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_front) return;
-  uint32_t bi = front_bin[i], n8 = front_n8[i];
-  Entry8 e[8];
-  binary_children(bn, bi, e[0], e[1]);
-  int cnt = 2;
-  while (cnt < 8) {
-    int best = -1;
-    float ba = -1.0f;
-    for (int q = 0; q < cnt; ++q) {
-      if (e[q].ref & kLeafBit) continue;
-      float a = half_area(e[q].b);
-      if (a > ba) {
-        ba = a;
-        best = q;
-      }
-    }
-    if (best < 0) break;
-    Entry8 c0, c1;
-    binary_children(bn, e[best].ref, c0, c1);
-    e[best] = c0;
-    e[cnt++] = c1;
-  }
-  float4* out = nodes8 + 16 * (size_t)n8;
-  for (int q = 0; q < 8; ++q) {
-    if (q < cnt) {
-      uint32_t ref = e[q].ref;
-      if (!(ref & kLeafBit)) {
-        uint32_t child8 = atomicAdd(&counters[0], 1u);
-        if (child8 >= max_nodes8) {
-          atomicOr(&counters[2], 1u);
-          child8 = 0;
-        } else {
-          uint32_t slot = atomicAdd(&counters[1], 1u);
-          next_bin[slot] = ref;
-          next_n8[slot] = child8;
+// Child c (0 or 1) of binary node i.
+__device__ __forceinline__ void binary_child(const float4* bn, uint32_t i, uint32_t c, float b[6], uint32_t& ref) {
+  const float4 xy = __ldg(bn + 4 * (size_t)i + c), z = __ldg(bn + 4 * (size_t)i + 2), r = __ldg(bn + 4 * (size_t)i + 3);
+  b[0] = xy.x;
+  b[3] = xy.y;
+  b[1] = xy.z;
+  b[4] = xy.w;
+  b[2] = c ? z.z : z.x;
+  b[5] = c ? z.w : z.y;
+  ref = __float_as_uint(c ? r.y : r.x);
+}
+
+// The whole collapse in one cooperative launch: level by level, eight lanes a
+// node (one entry each), the grid in step between levels.  The nodes of a
+// level follow each other, so a node's index is also its place in the work
+// list; bin_of[i] is the binary node 8-wide node i starts from.  counts: how
+// many nodes a level has made so far, three in turn.  Bound by the dependent
+// loads of up to six openings a node.  (B200, 1M proxies: a thread a node and a
+// launch and a host round trip a level took 312 us of kernels in 15 launches;
+// this takes 215 us in one.)
+__global__ void __launch_bounds__(128) k_collapse8(const float4* __restrict__ bn, float4* __restrict__ nodes8,
+                                                   const float* __restrict__ ibox, const uint32_t* root, float* root_box,
+                                                   uint32_t* bin_of, uint32_t* counts, uint32_t* out,
+                                                   uint32_t max_nodes8) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x & 31, gl = lane & 7, g0 = lane & 24;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
+  if (blockIdx.x == 0 && threadIdx.x < 6) root_box[threadIdx.x] = ibox[6 * (size_t)*root + threadIdx.x];
+  uint32_t start = 0, end = 1;
+  for (uint32_t level = 0; start < end; ++level) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[(level + 1) % 3] = 0;
+    uint32_t* made = &counts[level % 3];
+    for (uint32_t first = start + 4 * warp; first < end; first += 4 * n_warps) {
+      const uint32_t i = first + (lane >> 3);
+      const bool on = i < end;
+      float b[6] = {1e30f, 1e30f, 1e30f, -1e30f, -1e30f, -1e30f};
+      uint32_t ref = kInvalid;
+      const uint32_t bi = i == 0 ? *root : on ? __ldcg(bin_of + i) : 0u;
+      if (on && gl < 2) binary_child(bn, bi, gl, b, ref);
+      uint32_t cnt = 2;
+      for (int open = 0; open < 6; ++open) {
+        float area = ref == kInvalid || (ref & kLeafBit) ? -1.0f : half_area(b);
+        if (!(area >= 0.0f)) area = -1.0f;
+        uint32_t at = gl;
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) {
+          const float oa = __shfl_xor_sync(kAll, area, off);
+          const uint32_t ob = __shfl_xor_sync(kAll, at, off);
+          if (oa > area || (oa == area && ob < at)) {
+            area = oa;
+            at = ob;
+          }
         }
-        ref = child8;
+        const uint32_t parent = __shfl_sync(kAll, ref, g0 + at);
+        if (area >= 0.0f) {
+          if (gl == at) binary_child(bn, parent, 0, b, ref);
+          if (gl == cnt) binary_child(bn, parent, 1, b, ref);
+          ++cnt;
+        }
+        if (!__any_sync(kAll, area >= 0.0f)) break;
       }
-      out[2 * q] = make_float4(e[q].b[0], e[q].b[1], e[q].b[2], e[q].b[3]);
-      out[2 * q + 1] = make_float4(e[q].b[4], e[q].b[5], __uint_as_float(ref), 0.f);
-    } else {
-      out[2 * q] = make_float4(1e30f, 1e30f, 1e30f, -1e30f);
-      out[2 * q + 1] = make_float4(-1e30f, -1e30f, __uint_as_float(kInvalid), 0.f);
+      const bool inner = on && ref != kInvalid && !(ref & kLeafBit);
+      const uint32_t im = __ballot_sync(kAll, inner);
+      uint32_t base = 0;
+      if (lane == 0 && im) base = atomicAdd(made, (uint32_t)__popc(im));
+      base = __shfl_sync(kAll, base, 0);
+      if (inner) {
+        const uint32_t child = end + base + __popc(im & lt_mask);
+        if (child >= max_nodes8) {
+          out[1] = 1u;
+          ref = 0u;
+        } else {
+          __stcg(bin_of + child, ref);
+          ref = child;
+        }
+      }
+      if (on) {
+        float4* o = nodes8 + 16 * (size_t)i + 2 * gl;
+        o[0] = make_float4(b[0], b[1], b[2], b[3]);
+        o[1] = make_float4(b[4], b[5], __uint_as_float(ref), 0.f);
+      }
     }
+    __threadfence();
+    grid.sync();
+    start = end;
+    end = min(end + *reinterpret_cast<volatile uint32_t*>(made), max_nodes8);
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = end;
 }
 
 // Collapses the binary hierarchy (m leaves) into `*out8` (exactly sized).
-static Err collapse_bvh8(const float4* bn, const float* leaf_box, uint32_t m, cudaStream_t st, float4** out8,
-                         uint32_t* n_nodes8, uint64_t* launches) {
+static Err collapse_bvh8(const float4* bn, const float* ibox, const float* leaf_box, uint32_t m, uint32_t* bounds,
+                         cudaStream_t st, float4** out8, uint32_t* n_nodes8, uint64_t* launches) {
   uint32_t cap = std::max<uint32_t>(m > 1 ? m - 1 : 1, 1);
   float4* tmp = nullptr;
-  uint32_t *fb = nullptr, *fn = nullptr, *nb = nullptr, *nn = nullptr, *ctr = nullptr;
+  uint32_t* buf = nullptr;  // 5 words: level counts, result; then bin_of
   GT_CUDA_TRY(cudaMallocAsync(&tmp, (size_t)cap * 16 * sizeof(float4), st));
-  GT_CUDA_TRY(cudaMallocAsync(&fb, (size_t)cap * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&fn, (size_t)cap * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&nb, (size_t)cap * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&nn, (size_t)cap * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&ctr, 4 * 4, st));
+  GT_CUDA_TRY(cudaMallocAsync(&buf, ((size_t)cap + 8) * 4, st));
   uint32_t total = 1;
   if (m == 1) {
     float lb[6];
@@ -742,35 +837,32 @@ static Err collapse_bvh8(const float4* bn, const float* leaf_box, uint32_t m, cu
     }
     GT_CUDA_TRY(cudaMemcpyAsync(tmp, host, sizeof host, cudaMemcpyHostToDevice, st));
   } else {
-    uint32_t init[4] = {1u, 0u, 0u, 0u};
-    uint32_t zero = 0u;
-    GT_CUDA_TRY(cudaMemcpyAsync(ctr, init, sizeof init, cudaMemcpyHostToDevice, st));
-    GT_CUDA_TRY(cudaMemcpyAsync(fb, &zero, 4, cudaMemcpyHostToDevice, st));
-    GT_CUDA_TRY(cudaMemcpyAsync(fn, &zero, 4, cudaMemcpyHostToDevice, st));
-    uint32_t n_front = 1;
-    for (int level = 0; n_front > 0 && level < 1000; ++level) {
-      GT_CUDA_TRY(cudaMemsetAsync(ctr + 1, 0, 4, st));
-      k_collapse8<<<(n_front + 127) / 128, 128, 0, st>>>(bn, fb, fn, n_front, tmp, nb, nn, ctr, cap);
-      ++*launches;
-      GT_CUDA_TRY(cudaGetLastError());
-      uint32_t c[4];
-      GT_CUDA_TRY(cudaMemcpyAsync(c, ctr, sizeof c, cudaMemcpyDeviceToHost, st));
-      GT_CUDA_TRY(cudaStreamSynchronize(st));
-      if (c[2]) return Err{GT_ERR_CUDA, "internal error: 8-wide collapse exceeded its node bound"};
-      total = c[0];
-      n_front = c[1];
-      std::swap(fb, nb);
-      std::swap(fn, nn);
-    }
+    GT_CUDA_TRY(cudaMemsetAsync(buf, 0, 8 * 4, st));  // counts and result
+    int dev = 0, sms = 0, per_sm = 0;
+    GT_CUDA_TRY(cudaGetDevice(&dev));
+    GT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    GT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_collapse8, 128, 0));
+    // (a level has at most m / 4 or so nodes, 16 a block)
+    const unsigned grid =
+        (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)(sms * std::min(per_sm, 8)), m / 64 + 1));
+    uint32_t* counts = buf;
+    uint32_t* out = buf + 4;
+    uint32_t* bin_of = buf + 8;
+    const uint32_t* root = bounds + 8;
+    float* root_box = reinterpret_cast<float*>(bounds + 9);
+    void* args[] = {(void*)&bn, (void*)&tmp, (void*)&ibox, (void*)&root, (void*)&root_box, (void*)&bin_of, (void*)&counts, (void*)&out, (void*)&cap};
+    GT_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_collapse8, dim3(grid), dim3(128), args, 0, st));
+    ++*launches;
+    uint32_t c[2];
+    GT_CUDA_TRY(cudaMemcpyAsync(c, out, sizeof c, cudaMemcpyDeviceToHost, st));
+    GT_CUDA_TRY(cudaStreamSynchronize(st));
+    if (c[1]) return Err{GT_ERR_CUDA, "internal error: 8-wide collapse exceeded its node bound"};
+    total = c[0];
   }
   GT_CUDA_TRY(cudaMallocAsync(out8, (size_t)total * 16 * sizeof(float4), st));
   GT_CUDA_TRY(cudaMemcpyAsync(*out8, tmp, (size_t)total * 16 * sizeof(float4), cudaMemcpyDeviceToDevice, st));
   cudaFreeAsync(tmp, st);
-  cudaFreeAsync(fb, st);
-  cudaFreeAsync(fn, st);
-  cudaFreeAsync(nb, st);
-  cudaFreeAsync(nn, st);
-  cudaFreeAsync(ctr, st);
+  cudaFreeAsync(buf, st);
   *n_nodes8 = total;
   return Err{};
 }
@@ -804,11 +896,29 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   GT_CUDA_TRY(cudaMallocAsync(&b.params, n * 2 * sizeof(float4), st));
   b.bytes += n * 17 * sizeof(float4);
   uint32_t *flags = nullptr, *slots = nullptr, *bounds = nullptr;
+  float *box = nullptr;
+  float4* w2o_p = nullptr;
   GT_CUDA_TRY(cudaMallocAsync(&flags, n * 4, st));
   GT_CUDA_TRY(cudaMallocAsync(&slots, n * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&bounds, 8 * 4, st));
+  // centre bounds [0, 6), largest coordinate [6], tree check [7], binary root [8], its box [9, 15)
+  GT_CUDA_TRY(cudaMallocAsync(&bounds, 16 * 4, st));
+  GT_CUDA_TRY(cudaMallocAsync(&box, n * 6 * 4, st));
+  GT_CUDA_TRY(cudaMallocAsync(&w2o_p, n * 3 * sizeof(float4), st));
   const unsigned B = 256;
-  k_keep_flags<<<grid_for(n, B), B, 0, st>>>(packed, n, stride, alpha_min, act64, flags);
+  {
+    uint32_t init[16] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
+    GT_CUDA_TRY(cudaMemcpyAsync(bounds, init, sizeof init, cudaMemcpyHostToDevice, st));
+  }
+  IcoVerts iv;
+  ico_vertices(iv.v);
+  if (stride == 320 && (uintptr_t)packed % 16 == 0) {
+    k_records<true><<<grid_for(n, kRecBlock), kRecBlock, kRecBlock * 17 * sizeof(float), st>>>(
+        packed, n, stride, b.n_sh, alpha_min, act64, iv, flags, b.shade, b.sh, b.params, w2o_p, box, bounds);
+  } else {
+    const size_t smem = (size_t)kRecBlock * (std::min(stride / 4u, 16u + 4u * b.n_sh) | 1u) * sizeof(float);
+    k_records<false><<<grid_for(n, kRecBlock), kRecBlock, smem, st>>>(
+        packed, n, stride, b.n_sh, alpha_min, act64, iv, flags, b.shade, b.sh, b.params, w2o_p, box, bounds);
+  }
   ++*launches;
   GT_CUDA_TRY(cudaGetLastError());
   Err e = scan_exclusive(flags, slots, n, st, launches);
@@ -819,32 +929,23 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   GT_CUDA_TRY(cudaStreamSynchronize(st));
   uint32_t m = last_slot + last_flag;
   b.n_kept = m;
-  k_shade<<<grid_for(n, 128), 128, 0, st>>>(packed, n, stride, b.n_sh, flags, b.shade, b.sh, b.params);
-  ++*launches;
-  if (m == 0) {
+  auto drop_first = [&]() {
     cudaFreeAsync(flags, st);
     cudaFreeAsync(slots, st);
     cudaFreeAsync(bounds, st);
+    cudaFreeAsync(box, st);
+    cudaFreeAsync(w2o_p, st);
+  };
+  if (m == 0) {
+    drop_first();
     GT_CUDA_TRY(cudaStreamSynchronize(st));
     *out = b;
     return Err{};
   }
-  float* box = nullptr;
-  uint32_t *kept_pidx = nullptr, *keys = nullptr, *vals = nullptr;
-  GT_CUDA_TRY(cudaMallocAsync(&box, (size_t)m * 6 * 4, st));
-  GT_CUDA_TRY(cudaMallocAsync(&kept_pidx, (size_t)m * 4, st));
+  uint32_t *keys = nullptr, *vals = nullptr;
   GT_CUDA_TRY(cudaMallocAsync(&keys, (size_t)m * 4, st));
   GT_CUDA_TRY(cudaMallocAsync(&vals, (size_t)m * 4, st));
-  {
-    uint32_t init[8] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
-    GT_CUDA_TRY(cudaMemcpyAsync(bounds, init, sizeof init, cudaMemcpyHostToDevice, st));
-  }
-  IcoVerts iv;
-  ico_vertices(iv.v);
-  k_proxy_boxes<<<grid_for(n, B), B, 0, st>>>(packed, n, stride, alpha_min, act64, flags, slots, iv, box, kept_pidx,
-                                              bounds);
-  ++*launches;
-  k_morton<<<grid_for(m, B), B, 0, st>>>(box, m, bounds, keys, vals);
+  k_morton<<<grid_for(n, B), B, 0, st>>>(box, n, flags, slots, bounds, keys, vals);
   ++*launches;
   GT_CUDA_TRY(cudaGetLastError());
   e = radix_sort(keys, vals, m, st, launches);
@@ -865,8 +966,7 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   GT_CUDA_TRY(cudaMallocAsync(&depth, 4, st));
   GT_CUDA_TRY(cudaMemsetAsync(arrive, 0, (size_t)std::max<uint32_t>(n_int, 1) * 4, st));
   GT_CUDA_TRY(cudaMemsetAsync(depth, 0, 4, st));
-  k_leaves<<<grid_for(m, B), B, 0, st>>>(packed, stride, alpha_min, act64, vals, m, kept_pidx, box, b.w2o, b.leaf_pidx,
-                                          leaf_box);
+  k_leaves<<<grid_for(m, B), B, 0, st>>>(vals, m, w2o_p, box, b.w2o, b.leaf_pidx, leaf_box);
   ++*launches;
   if (m > 1) {
     if (fast_build) {
@@ -874,7 +974,7 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
       k_refit<<<grid_for(m, B), B, 0, st>>>(m, leaf_box, ibox, b.nodes, parent_int, parent_leaf, arrive);
       *launches += 2;
     } else {
-      Err pe = build_ploc(leaf_box, m, st, b.nodes, ibox, parent_int, parent_leaf, launches);
+      Err pe = build_ploc(keys, leaf_box, m, st, b.nodes, ibox, parent_int, parent_leaf, bounds + 8, launches);
       if (pe.code != GT_OK) return pe;
     }
     k_depth<<<grid_for(m, B), B, 0, st>>>(m, parent_int, parent_leaf, depth);
@@ -883,9 +983,8 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
     uint32_t* refc = nullptr;
     GT_CUDA_TRY(cudaMallocAsync(&refc, (size_t)(2 * m - 1) * 4, st));
     GT_CUDA_TRY(cudaMemsetAsync(refc, 0, (size_t)(2 * m - 1) * 4, st));
-    GT_CUDA_TRY(cudaMemsetAsync(bounds + 7, 0, 4, st));
-    k_check_children<<<grid_for(n_int, B), B, 0, st>>>(m, b.nodes, refc, bounds + 7);
-    k_check_counts<<<grid_for(2 * m - 1, B), B, 0, st>>>(2 * m - 1, refc, bounds + 7);
+    k_check_children<<<grid_for(n_int, B), B, 0, st>>>(m, b.nodes, refc, bounds + 8, bounds + 7);
+    k_check_counts<<<grid_for(2 * m - 1, B), B, 0, st>>>(2 * m - 1, refc, bounds + 8, bounds + 7);
     *launches += 2;
     cudaFreeAsync(refc, st);
     b.root = 0;
@@ -894,7 +993,7 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   }
   GT_CUDA_TRY(cudaGetLastError());
   {
-    Err ce = collapse_bvh8(b.nodes, leaf_box, m, st, &b.nodes8, &b.n_nodes8, launches);
+    Err ce = collapse_bvh8(b.nodes, ibox, leaf_box, m, bounds, st, &b.nodes8, &b.n_nodes8, launches);
     if (ce.code != GT_OK) return ce;
     b.bytes += (uint64_t)b.n_nodes8 * 16 * sizeof(float4);
     // traversal reads only the 8-wide nodes: the binary hierarchy goes
@@ -903,20 +1002,17 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
     b.bytes -= (uint64_t)std::max<uint32_t>(n_int, 1) * 4 * sizeof(float4);
   }
   float rb[6];
-  uint32_t bo[8];
-  GT_CUDA_TRY(cudaMemcpyAsync(rb, m > 1 ? ibox : leaf_box, sizeof rb, cudaMemcpyDeviceToHost, st));
+  uint32_t bo[16];
+  if (m == 1) GT_CUDA_TRY(cudaMemcpyAsync(rb, leaf_box, sizeof rb, cudaMemcpyDeviceToHost, st));
   GT_CUDA_TRY(cudaMemcpyAsync(&b.depth, depth, 4, cudaMemcpyDeviceToHost, st));
   GT_CUDA_TRY(cudaMemcpyAsync(bo, bounds, sizeof bo, cudaMemcpyDeviceToHost, st));
   GT_CUDA_TRY(cudaStreamSynchronize(st));
+  if (m > 1) memcpy(rb, bo + 9, sizeof rb);
   for (int a = 0; a < 6; ++a) b.bounds[a] = rb[a];
   float mag = 0.0f;
   for (int a = 0; a < 6; ++a) mag = std::max(mag, std::fabs(rb[a]));
   b.scene_mag = mag;
-  cudaFreeAsync(flags, st);
-  cudaFreeAsync(slots, st);
-  cudaFreeAsync(bounds, st);
-  cudaFreeAsync(box, st);
-  cudaFreeAsync(kept_pidx, st);
+  drop_first();
   cudaFreeAsync(keys, st);
   cudaFreeAsync(vals, st);
   cudaFreeAsync(leaf_box, st);
@@ -932,6 +1028,8 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   }
   if (b.depth > kMaxDepth) {
     free_scene(&b, st);
+    // (the radix tree is at most 30 code bits and 31 index bits deep)
+    if (!fast_build) return build_scene(packed_dev, n, stride, alpha_min, st, out, launches, true, act64);
     return Err{GT_ERR_UNSUPPORTED, "BVH deeper than the traversal stack allows"};
   }
   *out = b;
