@@ -251,7 +251,7 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
     recs += views[i].s.n_kept;
   }
   constexpr uint64_t kRec = 3 * sizeof(float4) + sizeof(float), kEnt = sizeof(float4) + sizeof(uint2);
-  constexpr uint64_t kBin = (4ull << kListBucketBits) + 4;
+  constexpr uint64_t kBin = (4ull << kListBucketBits) + 8;
   const uint64_t fixed = recs * kRec + bins * kBin;
   if (fixed > kListBudget / 2 || recs >= (1ull << 31)) return GT_OK;
   uint64_t want = std::max<uint64_t>(recs * 24 + (1u << 20), ctx->lists_need + ctx->lists_need / 4ull);
@@ -285,6 +285,7 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
       ctx->lists_bins = 0;
       e = grow(&L.cells, bins << kListBucketBits);
       if (e == cudaSuccess) e = grow(&L.bin_base, bins + 1);
+      if (e == cudaSuccess) e = grow(&L.order, bins);
       if (e == cudaSuccess) ctx->lists_bins = bins;
     }
     if (e == cudaSuccess && want > L.cap) {
@@ -499,7 +500,7 @@ extern "C" gt_status gt_context_destroy(gt_context* ctx) {
   cudaFree(ctx->staging);
   cudaFree(ctx->colours);
   for (void* p : {(void*)ctx->lists.views, (void*)ctx->lists.rec, (void*)ctx->lists.box, (void*)ctx->lists.far, (void*)ctx->lists.range,
-                  (void*)ctx->lists.cells, (void*)ctx->lists.bin_base, (void*)ctx->lists.ent_box,
+                  (void*)ctx->lists.cells, (void*)ctx->lists.bin_base, (void*)ctx->lists.order, (void*)ctx->lists.ent_box,
                   (void*)ctx->lists.ent, (void*)ctx->lists.spill, (void*)ctx->d_redo})
     cudaFree(p);
   delete ctx->copy_pool;

@@ -291,6 +291,7 @@ struct Lists {
   uint32_t* range = nullptr;     // per view: bits of the smallest and largest bound
   uint32_t* cells = nullptr;     // per bin 2^kListBucketBits counts, then places
   uint32_t* bin_base = nullptr;  // start of each bin's list (one more than bins)
+  uint32_t* order = nullptr;     // bins in the order in which their tiles are traced
   float4* ent_box = nullptr;     // list entries: outline rectangle
   uint2* ent = nullptr;          // proxy, bits of its bucket's lower bound
   unsigned long long* spill = nullptr;  // waiting hits past a ray's column in shared memory

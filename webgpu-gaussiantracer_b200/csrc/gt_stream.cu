@@ -296,8 +296,16 @@ __device__ __forceinline__ float bin_bound(const ProxySlab& S, float u0, float u
 // The two passes of the counting sort over (bin, bucket) cells: SCATTER
 // false counts each cell's entries, true writes them (a cell then holds the
 // next free place of its bin's list).
+// A warp takes 32 proxies and shares their pairs with bins out evenly (a proxy
+// meets one bin or hundreds: with a lane a proxy 158 + 260 us for 1080p and 1M
+// proxies, 74 + 137 so).
+constexpr uint32_t kPassBlock = 128;
+struct PassRow {
+  ProxySlab slab;
+  uint32_t bx, by, nx;  // bins: the first, and how many across
+};
 template <bool SCATTER>
-__global__ void __launch_bounds__(256) k_list_pass(const ViewDev* __restrict__ views,
+__global__ void __launch_bounds__(kPassBlock) k_list_pass(const ViewDev* __restrict__ views,
                                                    const ListView* __restrict__ lviews, float r_circ,
                                                    const Lists L) {
   const ViewDev& V = views[blockIdx.y];
@@ -308,7 +316,7 @@ __global__ void __launch_bounds__(256) k_list_pass(const ViewDev* __restrict__ v
   const float bw = 1.0f / (float)P.inv_bw, bh = 1.0f / (float)P.inv_bh;
   const float isx = (float)(1.0 / P.sx), isy = (float)(1.0 / P.sy), ox = (float)P.ox, oy = (float)P.oy;
   const V3 o = mk(V.u.tw[12], V.u.tw[13], V.u.tw[14]);
-  auto put = [&](uint32_t bx, uint32_t by, const ProxySlab& S, float4 bb, uint32_t j) {
+  auto put = [&](uint32_t bx, uint32_t by, const ProxySlab& S, uint32_t j) {
     const uint32_t bin = P.bin_begin + bin_index(bx, by, L.shift, bpr);
     // the bin's image-plane rectangle, a little larger
     const float u0 = ((float)bx * bw - 0.1f - ox) * isx, u1 = ((float)(bx + 1) * bw + 0.1f - ox) * isx;
@@ -318,29 +326,31 @@ __global__ void __launch_bounds__(256) k_list_pass(const ViewDev* __restrict__ v
     if (SCATTER) {
       const uint32_t pos = L.bin_base[bin] + atomicAdd(cell, 1u);
       if (pos < L.cap) {
-        L.ent_box[pos] = bb;
+        L.ent_box[pos] = __ldg(L.box + (size_t)P.rec_begin + j);
         L.ent[pos] = make_uint2(j, bucket_edge(B, bucket));
       }
     } else {
       atomicAdd(cell, 1u);
     }
   };
+  __shared__ PassRow rows_s[kPassBlock];
+  __shared__ uint32_t first_s[kPassBlock + kPassBlock / 32];
+  PassRow* rows = rows_s + (threadIdx.x & ~31u);
+  uint32_t* first = first_s + 33u * (threadIdx.x >> 5);
   for (uint32_t base = blockIdx.x * blockDim.x; base < V.s.n_kept; base += gridDim.x * blockDim.x) {
     const uint32_t j = base + threadIdx.x;
-    uint32_t rx = 0xFFFFFFFFu, ry = 0;
-    float4 bb = make_float4(0.f, 0.f, 0.f, 0.f);
-    ProxySlab S{};
+    uint32_t total = 0;
     if (j < V.s.n_kept) {
       const size_t at = (size_t)P.rec_begin + j;
       const float4 r1 = __ldg(L.rec + 2 * at + 1);
-      rx = __float_as_uint(r1.z);
-      ry = __float_as_uint(r1.w);
+      const uint32_t rx = __float_as_uint(r1.z), ry = __float_as_uint(r1.w);
       if (rx != 0xFFFFFFFFu) {
+        PassRow& Q = rows[lane];
         const float4 r0 = __ldg(L.rec + 2 * at);
+        ProxySlab S;
         S.u = r0.x;
         S.v = r0.y;
         S.tb = r1.y;
-        if (SCATTER) bb = __ldg(L.box + at);
         const Affine W = load_affine(V.s.w2o + 3 * (size_t)j);
         S.oo = xpoint(W, o);
         const float l1o = fabsf(S.oo.x) + fabsf(S.oo.y) + fabsf(S.oo.z);
@@ -350,37 +360,34 @@ __global__ void __launch_bounds__(256) k_list_pass(const ViewDev* __restrict__ v
         S.wx = xdir(W, mk(P.Xf[0], P.Xf[1], P.Xf[2]));
         S.wy = xdir(W, mk(P.Yf[0], P.Yf[1], P.Yf[2]));
         S.wz = xdir(W, mk(P.Zf[0], P.Zf[1], P.Zf[2]));
+        Q.slab = S;
+        Q.bx = rx & 0xFFFFu;
+        Q.by = ry & 0xFFFFu;
+        Q.nx = (rx >> 16) - (rx & 0xFFFFu) + 1;
+        total = Q.nx * ((ry >> 16) - (ry & 0xFFFFu) + 1);
       }
     }
-    const uint32_t nx = (rx >> 16) - (rx & 0xFFFFu) + 1, ny = (ry >> 16) - (ry & 0xFFFFu) + 1;
-    const uint32_t total = rx == 0xFFFFFFFFu ? 0u : nx * ny;
-    const bool big = total > 16u;
-    if (!big) {
-      for (uint32_t q = 0, bx = rx & 0xFFFFu, by = ry & 0xFFFFu; q < total; ++q) {
-        put(bx, by, S, bb, j);
-        if (++bx > (rx >> 16)) {
-          bx = rx & 0xFFFFu;
-          ++by;
-        }
-      }
-    }
-    // proxies in many bins: the warp's lanes share the bins
-    uint32_t bm = __ballot_sync(kFull, big);
-    while (bm) {
-      const int src = __ffs(bm) - 1;
-      bm &= bm - 1;
-      const uint32_t srx = __shfl_sync(kFull, rx, src), sry = __shfl_sync(kFull, ry, src);
-      const uint32_t snx = __shfl_sync(kFull, nx, src), st = __shfl_sync(kFull, total, src);
-      const uint32_t sj = __shfl_sync(kFull, j, src);
-      const float4 sbb = make_float4(__shfl_sync(kFull, bb.x, src), __shfl_sync(kFull, bb.y, src),
-                                     __shfl_sync(kFull, bb.z, src), __shfl_sync(kFull, bb.w, src));
-      ProxySlab Q;
-      const float* f = reinterpret_cast<const float*>(&S);
-      float* g = reinterpret_cast<float*>(&Q);
+    // the warp's (proxy, bin) pairs, shared out evenly
+    uint32_t end = total;
 #pragma unroll
-      for (int i = 0; i < (int)(sizeof(ProxySlab) / 4); ++i) g[i] = __shfl_sync(kFull, f[i], src);
-      for (uint32_t q = lane; q < st; q += 32) put((srx & 0xFFFFu) + q % snx, (sry & 0xFFFFu) + q / snx, Q, sbb, sj);
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, end, off);
+      if ((int)lane >= off) end += y;
     }
+    first[lane] = end - total;
+    const uint32_t pairs = __shfl_sync(kFull, end, 31);
+    __syncwarp();
+    for (uint32_t t = lane; t < pairs; t += 32) {
+      uint32_t src = 0;  // the last row whose first pair is not past t
+#pragma unroll
+      for (uint32_t step = 16; step > 0; step >>= 1)
+        if (first[src + step] <= t) src += step;
+      const PassRow& Q = rows[src];
+      const uint32_t q = t - first[src], dy = q / Q.nx;
+      const uint32_t jj = base + (threadIdx.x & ~31u) + src;
+      put(Q.bx + (q - dy * Q.nx), Q.by + dy, Q.slab, jj);
+    }
+    __syncwarp();
   }
 }
 
@@ -414,16 +421,22 @@ __global__ void __launch_bounds__(128) k_list_rows(const Lists L) {
   }
 }
 
-// One block: the bins' lengths become the starts of their lists.
+// One block: the bins' lengths become the starts of their lists, and the bins
+// are ordered by length (in powers of two, longest first).  Tiles of long lists
+// take longest, and the launch's end waits on those taken last (256x256 of 16k
+// Gaussians 483 -> 435 us, 960x540 of 1M 3.86 -> 3.67 ms, 1080p unchanged).
 __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bins, DevCounters* ctr) {
   __shared__ uint32_t ws[32];
   __shared__ uint32_t carry;
+  __shared__ uint32_t place[33];  // bins per class, then their first places
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0;
+  if (threadIdx.x < 33) place[threadIdx.x] = 0;
   __syncthreads();
   for (uint32_t base = 0; base < n_bins; base += 1024) {
     const uint32_t i = base + threadIdx.x;
     const uint32_t v = i < n_bins ? L.bin_base[i] : 0u;
+    if (i < n_bins) atomicAdd(&place[__clz(v)], 1u);
     uint32_t x = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -451,6 +464,17 @@ __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bi
   if (threadIdx.x == 0) {
     L.bin_base[n_bins] = carry;
     atomicMax(&ctr->list_pairs, carry);
+    uint32_t at = 0;
+    for (int c = 0; c < 33; ++c) {
+      const uint32_t k = place[c];
+      place[c] = at;
+      at += k;
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n_bins; i += 1024) {
+    const uint32_t v = L.bin_base[i + 1] - L.bin_base[i];
+    L.order[atomicAdd(&place[__clz(v)], 1u)] = i;
   }
 }
 
@@ -661,7 +685,9 @@ __global__ void __launch_bounds__(32, 16) k_trace_stream(const ViewDev* __restri
     if (lane == 0) item = atomicAdd(&ctr->work, 1u);
     item = __shfl_sync(kFull, item, 0);
     if (item >= total) break;
-    const uint32_t tile = item / kParts, part = item % kParts;
+    const uint32_t part = item % kParts;
+    uint32_t tile = item / kParts;
+    tile = (__ldg(L.order + (tile >> L.shift)) << L.shift) | (tile & ((1u << L.shift) - 1u));
     const uint32_t vi = n_views == 1 ? 0u : find_view(views, n_views, tile);
     const ViewDev& V = views[vi];
     // R = 32: the tile; 8: its 4x2 quarter (part & 1, part >> 1)
@@ -1119,7 +1145,10 @@ static Err launch_stream_r(const ViewDev* d_views, uint32_t n_views, uint32_t to
   const uint32_t items = total_tiles * (32 / R);
   if (grid > items) grid = std::max(1u, items);
   grid = std::min(grid, (uint32_t)(L.spill_bytes / (sizeof(unsigned long long) * kStreamSpill * R)));
-  hand.late = grid / 4 * 3;
+  // (idle warps at which the tiles still tracing hand over, 50 / 75 / 90 / 95 %
+  // / never: 481x271 of 1M Gaussians 2.14 / 2.00 / 2.09 / 2.04 / 2.79 ms,
+  // 256x256 of 16k 440 / 444 / 435 / 418 / 420 us, 1080p within 1 %)
+  hand.late = grid / 10 * 9;
   k_trace_stream<R, CKPT><<<grid, 32, smem, stream>>>(d_views, L.views, n_views, total_tiles, counters, faces, L,
                                                       hand, ck);
   ++*launches;
@@ -1166,12 +1195,12 @@ bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, 
 // as warp per ray / 8 rays per warp / 32 rays per warp, bins of 16x8 pixels for
 // 8 rays and 32x16 for 32:
 //   rays          uniform 16k k 6   clusters 200k k 8   clusters 1M k 16
-//   64x64         197 /  290 /  314    245 /  536 /  525     704 / 2015 / 1287
-//   128x96        308 /  314 /  376    289 /  453 /  550     888 / 1489 / 1681
-//   200x150       565 /  338 /  430    480 /  438 /  555    1443 / 1449 / 1618
-//   256x256       974 /  430 /  477    845 /  503 /  601    2183 / 1845 / 1917
-//   400x300      1945 /  662 /  534   1512 /  612 /  622    3985 / 2199 / 1892
-//   800x600      7464 / 1982 / 1201   5589 / 1426 /  998   15023 / 5211 / 3543
+//   64x64         203 /  315 /  368    242 /  517 /  710     750 / 2462 / 2660
+//   128x96        314 /  316 /  429    294 /  462 /  561     910 / 1574 / 1942
+//   200x150       566 /  331 /  434    479 /  463 /  552    1500 / 1525 / 1711
+//   256x256       983 /  390 /  472    841 /  499 /  589    2174 / 2009 / 1954
+//   400x300      1946 /  646 /  501   1491 /  559 /  614    3951 / 2138 / 1916
+//   800x600      7472 / 1980 / 1155   5542 / 1362 /  970   14931 / 5222 / 3504
 // With few tiles the warps with the most hits decide the time, so fewer rays
 // share one; below 160 rays an SM even those are too few warps.
 StreamPlan stream_plan(uint64_t rays, int num_sms) {
@@ -1193,10 +1222,12 @@ Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n
   GT_CUDA_TRY(cudaMemsetAsync(L.cells, 0, ((size_t)n_bins << kListBucketBits) * 4, stream));
   k_list_views<<<(n_views + 63) / 64, 64, 0, stream>>>(d_views, n_views, L.views, L);
   k_list_project<<<dim3(std::max(1u, (kept + 127) / 128), n_views), 128, 0, stream>>>(d_views, L.views, faces.r_circ, L);
-  k_list_pass<false><<<dim3(std::max(1u, (kept + 255) / 256), n_views), 256, 0, stream>>>(d_views, L.views, faces.r_circ, L);
+  k_list_pass<false><<<dim3(std::max(1u, (kept + kPassBlock - 1) / kPassBlock), n_views), kPassBlock, 0, stream>>>(
+      d_views, L.views, faces.r_circ, L);
   k_list_rows<<<n_bins, 128, 0, stream>>>(L);
   k_list_bins<<<1, 1024, 0, stream>>>(L, n_bins, counters);
-  k_list_pass<true><<<dim3(std::max(1u, (kept + 255) / 256), n_views), 256, 0, stream>>>(d_views, L.views, faces.r_circ, L);
+  k_list_pass<true><<<dim3(std::max(1u, (kept + kPassBlock - 1) / kPassBlock), n_views), kPassBlock, 0, stream>>>(
+      d_views, L.views, faces.r_circ, L);
   *launches += 6;
   GT_CUDA_TRY(cudaGetLastError());
   const Ckpt ck = ckpt ? *ckpt : Ckpt{};
