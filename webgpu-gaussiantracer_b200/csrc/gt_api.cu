@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
+#include <new>
 #include <map>
 #include <mutex>
 #include <set>
@@ -23,7 +24,10 @@
 // much as a chunk's copy.  The calling thread takes a share as well.
 struct CopyPool {
   explicit CopyPool(unsigned workers) {
-    for (unsigned t = 0; t < workers; ++t) th_.emplace_back([this, t] { run(t); });
+    try {
+      for (unsigned t = 0; t < workers; ++t) th_.emplace_back([this, t] { run(t); });
+    } catch (...) {  // (fewer threads than asked for)
+    }
   }
   ~CopyPool() {
     {
@@ -527,30 +531,58 @@ extern "C" gt_status gt_last_error(const gt_context* ctx, char* buf, size_t len)
 }
 
 // ================================================================ scene
-// Host-to-device copy of a host buffer through two pinned 16 MB chunks of the
-// context: the host copies chunk i into one pinned buffer (several threads)
-// while the DMA engine moves chunk i-1 out of the other, so a pageable
-// source streams at close to host memcpy speed instead of the driver's
-// staged pageable copy.  Each chunk is one cudaMemcpyAsync on the context
-// stream.
-constexpr size_t kUploadChunk = 16u << 20;
+// Uploads of pageable memory go through two pinned 16 MB chunks of the context:
+// the copy threads fill one while the DMA engine empties the other, where the
+// driver's own staged copy runs on one thread (25 MB of a PLY file: 100k
+// vertices to the first frame 4.3 -> 2.8 ms, with its buffers from the pool).
+// Each chunk is one cudaMemcpyAsync on the context stream.  Page-locked buffers
+// and small copies go straight to the DMA engine.  Downloads stay with the
+// driver: emptying a pinned chunk by these threads was slower (a 3.9 MB gradient
+// 1.44 -> 2.2 ms a call: the page faults of a new output buffer), and so were
+// threads that queue their own 1 MB chunks (21 MB upload 2.4 -> 2.7 ms a call).
+constexpr size_t kCopyChunk = 16u << 20;
+constexpr size_t kDirectCopy = 4u << 20;
 
-static gt_status upload_host(gt_context* ctx, void* dst_dev, const void* src_host, size_t bytes) {
-  if (bytes == 0) return GT_OK;
+static bool page_locked(const void* p) {
+  cudaPointerAttributes pa;
+  if (cudaPointerGetAttributes(&pa, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return pa.type == cudaMemoryTypeHost;
+}
+
+static gt_status ensure_chunks(gt_context* ctx) {
   if (!ctx->copy_pool) {
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    ctx->copy_pool = new CopyPool(std::min(hw, 8u) - 1);
+    ctx->copy_pool = new (std::nothrow) CopyPool(std::min(hw, 8u) - 1);
+    if (!ctx->copy_pool) return fail(ctx, GT_ERR_OOM, "copy threads");
   }
   for (int b = 0; b < 2; ++b) {
     if (!ctx->up_pinned[b])
-      API_CUDA(ctx, cudaHostAlloc((void**)&ctx->up_pinned[b], kUploadChunk, cudaHostAllocDefault));
+      API_CUDA(ctx, cudaHostAlloc((void**)&ctx->up_pinned[b], kCopyChunk, cudaHostAllocDefault));
     if (!ctx->up_done[b]) API_CUDA(ctx, cudaEventCreateWithFlags(&ctx->up_done[b], cudaEventDisableTiming));
   }
-  const unsigned char* src = static_cast<const unsigned char*>(src_host);
-  unsigned char* dst = static_cast<unsigned char*>(dst_dev);
-  for (size_t off = 0, i = 0; off < bytes; off += kUploadChunk, ++i) {
+  return GT_OK;
+}
+
+namespace gt {
+gt_status api_upload(gt_context* ctx, void* dev, const void* host, size_t bytes) {
+  if (bytes == 0) return GT_OK;
+  const bool locked = page_locked(host);
+  if (bytes <= kDirectCopy || locked) {
+    API_CUDA(ctx, cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    // (a page-locked source is read by the DMA engine, not staged by the call)
+    if (locked) API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return GT_OK;
+  }
+  gt_status st = ensure_chunks(ctx);
+  if (st != GT_OK) return st;
+  const unsigned char* src = static_cast<const unsigned char*>(host);
+  unsigned char* dst = static_cast<unsigned char*>(dev);
+  for (size_t off = 0, i = 0; off < bytes; off += kCopyChunk, ++i) {
     const int b = (int)(i & 1);
-    const size_t len = std::min(kUploadChunk, bytes - off);
+    const size_t len = std::min(kCopyChunk, bytes - off);
     API_CUDA(ctx, cudaEventSynchronize(ctx->up_done[b]));  // the chunk's previous copy has left
     ctx->copy_pool->copy(ctx->up_pinned[b], src + off, len);
     API_CUDA(ctx, cudaMemcpyAsync(dst + off, ctx->up_pinned[b], len, cudaMemcpyHostToDevice, ctx->stream));
@@ -558,6 +590,12 @@ static gt_status upload_host(gt_context* ctx, void* dst_dev, const void* src_hos
   }
   return GT_OK;
 }
+
+gt_status api_download(gt_context* ctx, void* host, const void* dev, size_t bytes) {
+  if (bytes) API_CUDA(ctx, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  return GT_OK;
+}
+}  // namespace gt
 
 extern "C" gt_status gt_scene_create(gt_context* ctx, const void* packed, uint64_t n, uint32_t stride_bytes,
                                      double alpha_min, uint32_t flags, gt_scene** out) {
@@ -588,7 +626,7 @@ extern "C" gt_status gt_scene_create_ex(gt_context* ctx, const void* packed, uin
   const auto up0 = std::chrono::steady_clock::now();
   if (n > 0 && !(flags & GT_FLAG_INPUT_DEVICE)) {
     API_CUDA(ctx, cudaMallocAsync(&tmp, n * (uint64_t)stride_bytes, ctx->stream));
-    gt_status ust = upload_host(ctx, tmp, packed, n * (uint64_t)stride_bytes);
+    gt_status ust = gt::api_upload(ctx, tmp, packed, n * (uint64_t)stride_bytes);
     if (ust != GT_OK) {
       drop_tmps();
       return ust;
@@ -604,7 +642,7 @@ extern "C" gt_status gt_scene_create_ex(gt_context* ctx, const void* packed, uin
       return fail(ctx, e == cudaErrorMemoryAllocation ? GT_ERR_OOM : GT_ERR_CUDA,
                   std::string("upload of the activated values: ") + cudaGetErrorString(e));
     }
-    gt_status ust = upload_host(ctx, act_tmp, activated, n * 8 * sizeof(double));
+    gt_status ust = gt::api_upload(ctx, act_tmp, activated, n * 8 * sizeof(double));
     if (ust != GT_OK) {
       drop_tmps();
       return ust;
@@ -721,11 +759,11 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
   // A page-locked host buffer of this GPU (cudaHostAlloc, cudaMallocHost or
   // cudaHostRegister with a device mapping) is written by the trace kernels
   // directly: each tile's pixels cross the host link when the tile is done,
-  // instead of the whole image in one copy after the render.  Anti-aliased
-  // frames (which read the previous average) and checkpointing renders take
-  // the staging buffer.
+  // instead of the whole image in one copy after the render (and, for
+  // anti-aliased frames, the previous average in one before).  Checkpointing
+  // renders take the staging buffer.
   bool direct = false;
-  if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !aa && !(flags & GT_FLAG_CHECKPOINT)) {
+  if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !(flags & GT_FLAG_CHECKPOINT)) {
     cudaPointerAttributes pa;
     if (cudaPointerGetAttributes(&pa, out_rgba) == cudaSuccess) {
       if (pa.type == cudaMemoryTypeHost && pa.device == ctx->device && pa.devicePointer &&
@@ -742,8 +780,10 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
     if (st != GT_OK) return st;
     out = ctx->staging;
     // the running average of the earlier frames is blended on the device
-    if (aa && u->accumulated_frames != 0)
-      API_CUDA(ctx, cudaMemcpyAsync(out, out_rgba, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (aa && u->accumulated_frames != 0) {
+      st = gt::api_upload(ctx, out, out_rgba, bytes);
+      if (st != GT_OK) return st;
+    }
   }
   if (flags & GT_FLAG_CHECKPOINT) {
     if (flags & GT_FLAG_ASYNC) return fail(ctx, GT_ERR_INVALID_ARG, "a checkpointing render is synchronous");
@@ -751,8 +791,10 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
     API_CUDA(ctx, cudaEventRecord(ctx->call0, ctx->stream));
     st = api_forward_ckpt(ctx, &scene, u, &w, &h, &out, 1, 0, 0, 0, stats);
     if (st != GT_OK) return st;
-    if (!(flags & GT_FLAG_OUTPUT_DEVICE))
-      API_CUDA(ctx, cudaMemcpyAsync(out_rgba, out, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (!(flags & GT_FLAG_OUTPUT_DEVICE)) {
+      st = gt::api_download(ctx, out_rgba, out, bytes);
+      if (st != GT_OK) return st;
+    }
     API_CUDA(ctx, cudaEventRecord(ctx->call1, ctx->stream));
     API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (stats) cudaEventElapsedTime(&stats->total_ms, ctx->call0, ctx->call1);
@@ -779,8 +821,10 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
                        ctx->d_views, nullptr, &hand, &lists);
   if (e.code != GT_OK) return fail(ctx, e);
   API_CUDA(ctx, cudaEventRecord(ctx->ring[2 * slot + 1], ctx->stream));
-  if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !direct)
-    API_CUDA(ctx, cudaMemcpyAsync(out_rgba, out, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !direct) {
+    st = gt::api_download(ctx, out_rgba, out, bytes);
+    if (st != GT_OK) return st;
+  }
   if (flags & GT_FLAG_ASYNC) return GT_OK;
   return finish_call(ctx, stats, slot);
 }
@@ -912,9 +956,10 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
     st = api_forward_ckpt(ctx, sc.data(), us.data(), ws.data(), hs.data(), os.data(), count, 0, 0, 0, stats);
     if (st != GT_OK) return st;
     if (!(flags & GT_FLAG_OUTPUT_DEVICE))
-      for (uint32_t i = 0; i < count; ++i)
-        API_CUDA(ctx, cudaMemcpyAsync(items[i].out_rgba, os[i], (size_t)ws[i] * hs[i] * sizeof(float4),
-                                      cudaMemcpyDeviceToHost, ctx->stream));
+      for (uint32_t i = 0; i < count; ++i) {
+        st = gt::api_download(ctx, items[i].out_rgba, os[i], (size_t)ws[i] * hs[i] * sizeof(float4));
+        if (st != GT_OK) return st;
+      }
     API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return GT_OK;
   }
@@ -942,9 +987,10 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
     ctx->h_views[q] = make_view(it.scene, it.u, it.w, it.h, out, total_tiles);
     ctx->h_views[q].u.aa = aa ? 1u : 0u;
     total_tiles += ctx->h_views[q].n_tiles;
-    if (aa && it.u.accumulated_frames != 0 && !(flags & GT_FLAG_OUTPUT_DEVICE))
-      API_CUDA(ctx, cudaMemcpyAsync(out, it.out_rgba, (size_t)it.w * it.h * sizeof(float4), cudaMemcpyHostToDevice,
-                                    ctx->stream));
+    if (aa && it.u.accumulated_frames != 0 && !(flags & GT_FLAG_OUTPUT_DEVICE)) {
+      st = gt::api_upload(ctx, out, it.out_rgba, (size_t)it.w * it.h * sizeof(float4));
+      if (st != GT_OK) return st;
+    }
   }
   st = assign_colours(ctx, ctx->h_views, count);
   if (st != GT_OK) return st;
@@ -1003,8 +1049,8 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
     size_t o2 = 0;
     for (uint32_t i = 0; i < count; ++i) {
       size_t px = (size_t)items[i].w * items[i].h;
-      API_CUDA(ctx, cudaMemcpyAsync(items[i].out_rgba, ctx->staging + o2, px * sizeof(float4), cudaMemcpyDeviceToHost,
-                                    ctx->stream));
+      st = gt::api_download(ctx, items[i].out_rgba, ctx->staging + o2, px * sizeof(float4));
+      if (st != GT_OK) return st;
       o2 += px;
     }
   }

@@ -620,14 +620,10 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     rays += (uint64_t)ws[i] * hs[i];
   }
   const uint64_t slots = (uint64_t)total_tiles * 32u;
-  if (budget == 0) {
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    budget = free_b / 2 + ck.pool_bytes;  // the pool we hold counts as available
-  }
   // first guess of the records: the last call's count, else 4 a ray
   uint64_t want = ck.last_records ? ck.last_records + ck.last_records / 8 + 1024 : rays * 4 + 1024;
   if (cap) want = std::max<uint64_t>(want, rays * (uint64_t)cap);
+  const bool own_budget = budget == 0;
   if (!ck.pool_next) CK_TRY(cudaMalloc(&ck.pool_next, 4));
   sst = grow(ctx, (void**)&ck.head, &ck.head_bytes, slots * 4);
   if (sst != GT_OK) return sst;
@@ -642,6 +638,17 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
   if (sst != GT_OK) return sst;
   for (int attempt = 0; attempt < 3; ++attempt) {
     if (want > 0xFFFFFFF0ull) return api_fail(ctx, GT_ERR_OOM, "checkpoint needs more than 2^32 records");
+    if (own_budget && want * (kCkptHeader + kCkptChunk) * 4 > budget) {
+      // half of the free memory, the pool we hold counted as free; records
+      // that fit the pool as it is fit that, whatever is free (the query takes
+      // 0.1 ms or more)
+      budget = ck.pool_bytes;
+      if (want * (kCkptHeader + kCkptChunk) * 4 > budget) {
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        budget += free_b / 2;
+      }
+    }
     uint32_t m = mode == 1 ? 1u : (mode == 2 ? 2u : (want * (kCkptHeader + kCkptChunk) * 4 <= budget ? 1u : 2u));
     const uint32_t kc = m == 1 ? kCkptChunk : 0u;
     sst = grow(ctx, (void**)&ck.pool, &ck.pool_bytes, want * (kCkptHeader + kc) * 4);
@@ -771,7 +778,11 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
     if (flags & GT_FLAG_INPUT_DEVICE) {
       vd[i].dL = reinterpret_cast<const float4*>(bv.dL);
     } else {
-      BWD_TRY(cudaMemcpyAsync(dl_dev + off, bv.dL, px * sizeof(float4), cudaMemcpyHostToDevice, st));
+      const gt_status us = api_upload(ctx, dl_dev + off, bv.dL, px * sizeof(float4));
+      if (us != GT_OK) {
+        cleanup();
+        return us;
+      }
       vd[i].dL = dl_dev + off;
     }
     uint32_t s = 0;
@@ -786,10 +797,16 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
   std::vector<float4*> G(n_scenes, nullptr);
   for (uint32_t s = 0; s < n_scenes; ++s)
     BWD_TRY(talloc((void**)&G[s], (size_t)std::max<uint64_t>(scenes[s]->n, 1) * 4 * sizeof(float4)));
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const size_t gs_budget =
-      (opts && opts->mem_budget) ? (size_t)opts->mem_budget : std::max<size_t>((size_t)256 << 20, free_b / 4);
+  // a quarter of the free memory, at least 256 MB (queried only when the sums need more)
+  size_t gs_budget = (opts && opts->mem_budget) ? (size_t)opts->mem_budget : (size_t)256 << 20;
+  size_t gs_all_bytes = 0;
+  for (uint32_t i = 0; i < count; ++i)
+    gs_all_bytes += (size_t)std::max<uint64_t>(scenes[vscene[i]]->n, 1) * sizeof(float4);
+  if (!(opts && opts->mem_budget) && gs_all_bytes > gs_budget) {
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    gs_budget = std::max<size_t>(gs_budget, free_b / 4);
+  }
   std::vector<uint32_t> group_end;
   size_t gs_max = 0;
   {
@@ -829,8 +846,13 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
     dev_out[s] = outs[s];
     if (n == 0 || (flags & GT_FLAG_OUTPUT_DEVICE)) continue;
     BWD_TRY(talloc((void**)&dev_out[s], n * GT_PARAMS_PER_PARTICLE * 4));
-    if (flags & GT_FLAG_ACCUMULATE)
-      BWD_TRY(cudaMemcpyAsync(dev_out[s], outs[s], n * GT_PARAMS_PER_PARTICLE * 4, cudaMemcpyHostToDevice, st));
+    if (flags & GT_FLAG_ACCUMULATE) {
+      sst = api_upload(ctx, dev_out[s], outs[s], n * GT_PARAMS_PER_PARTICLE * 4);
+      if (sst != GT_OK) {
+        cleanup();
+        return sst;
+      }
+    }
   }
   float bwd_ms = 0.f;
   BWD_TRY(cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), st));
@@ -904,7 +926,11 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
   for (uint32_t s = 0; s < n_scenes; ++s) {
     const uint64_t n = scenes[s]->n;
     if (n == 0 || (flags & GT_FLAG_OUTPUT_DEVICE)) continue;
-    BWD_TRY(cudaMemcpyAsync(outs[s], dev_out[s], n * GT_PARAMS_PER_PARTICLE * 4, cudaMemcpyDeviceToHost, st));
+    sst = api_download(ctx, outs[s], dev_out[s], n * GT_PARAMS_PER_PARTICLE * 4);
+    if (sst != GT_OK) {
+      cleanup();
+      return sst;
+    }
   }
   BWD_TRY(cudaEventRecord(ctx->int1, st));
   BWD_TRY(cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));

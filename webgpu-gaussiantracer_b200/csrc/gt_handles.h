@@ -61,8 +61,8 @@ struct gt_context {
   // per-view particle colour tables of the render calls (ViewDev::rgb)
   float4* colours = nullptr;
   uint64_t colours_cap = 0;  // float4 entries
-  // pinned chunks through which host records are uploaded (double-buffered)
-  struct CopyPool* copy_pool = nullptr;  // host threads of the pinned uploads (gt_api.cu)
+  // pinned chunks of the uploads, and the threads that fill them (gt_api.cu)
+  struct CopyPool* copy_pool = nullptr;
   unsigned char* up_pinned[2] = {nullptr, nullptr};
   cudaEvent_t up_done[2] = {nullptr, nullptr};
   gt::HandoffRay* d_handoff = nullptr;  // rays tile packets hand to the warp-per-ray kernel
@@ -108,6 +108,11 @@ LaunchShape api_shape_for(gt_context* ctx, const gt_scene* s, uint32_t w, uint32
 // shape, else the per-view choice of the first view.
 LaunchShape api_batch_shape_for(gt_context* ctx, const gt_scene* const* scenes, const gt_uniforms* us,
                                 const uint32_t* ws, const uint32_t* hs, uint32_t count, uint32_t total_tiles);
+// Copies between host memory (pageable or page-locked) and the device, ordered
+// on the context stream: the upload's source may be reused when the call
+// returns; the download has arrived once the stream is waited for.
+gt_status api_upload(gt_context* ctx, void* dev, const void* host, size_t bytes);
+gt_status api_download(gt_context* ctx, void* host, const void* dev, size_t bytes);
 void api_fill_stats(const DevCounters& c, gt_render_stats* st);
 gt_status api_ensure_views(gt_context* ctx, uint32_t n);
 gt_status api_ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out);

@@ -391,18 +391,21 @@ static Err ply_to_device(gt_context* ctx, const uint8_t* data, const PlyLayout& 
   uint8_t* body = nullptr;
   float* packed = nullptr;
   const uint64_t body_bytes = L.n * (uint64_t)L.row_bytes;
-  GT_CUDA_TRY(cudaMalloc(&body, body_bytes));
-  cudaError_t e = cudaMalloc(&packed, L.n * (uint64_t)L.stride);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(body, data + L.data_offset, body_bytes, cudaMemcpyHostToDevice, ctx->stream);
+  // stream-ordered buffers: the context's pool keeps their memory
+  GT_CUDA_TRY(cudaMallocAsync(&body, body_bytes, ctx->stream));
+  cudaError_t e = cudaMallocAsync(&packed, L.n * (uint64_t)L.stride, ctx->stream);
   Err r;
-  if (e != cudaSuccess) {
+  const gt_status up = e == cudaSuccess ? api_upload(ctx, body, data + L.data_offset, body_bytes) : GT_OK;
+  if (up != GT_OK) {
+    r = Err{up, ctx->err};
+  } else if (e != cudaSuccess) {
     r = Err{e == cudaErrorMemoryAllocation ? GT_ERR_OOM : GT_ERR_CUDA,
             std::string("PLY upload: ") + cudaGetErrorString(e)};
   } else {
     r = launch_ply_pack(L, body, packed, ctx->num_sms, ctx->stream, &ctx->launches);
     if (r.code == GT_OK && act_dev) {
       double* act = nullptr;
-      e = cudaMalloc(&act, L.n * 8 * sizeof(double));
+      e = cudaMallocAsync(&act, L.n * 8 * sizeof(double), ctx->stream);
       if (e != cudaSuccess) {
         r = Err{e == cudaErrorMemoryAllocation ? GT_ERR_OOM : GT_ERR_CUDA,
                 std::string("PLY activations: ") + cudaGetErrorString(e)};
@@ -417,23 +420,19 @@ static Err ply_to_device(gt_context* ctx, const uint8_t* data, const PlyLayout& 
         ++ctx->launches;
         e = cudaGetLastError();
         if (e != cudaSuccess) {
-          cudaFree(act);
+          cudaFreeAsync(act, ctx->stream);
           r = Err{GT_ERR_CUDA, std::string("PLY activations: ") + cudaGetErrorString(e)};
         } else {
           *act_dev = act;
         }
       }
     }
-    if (r.code == GT_OK) {
-      e = cudaStreamSynchronize(ctx->stream);
-      if (e != cudaSuccess) r = Err{GT_ERR_CUDA, std::string("PLY pack: ") + cudaGetErrorString(e)};
-    }
   }
-  cudaFree(body);
+  cudaFreeAsync(body, ctx->stream);
   if (r.code != GT_OK) {
-    cudaFree(packed);
+    if (packed) cudaFreeAsync(packed, ctx->stream);
     if (act_dev && *act_dev) {
-      cudaFree(*act_dev);
+      cudaFreeAsync(*act_dev, ctx->stream);
       *act_dev = nullptr;
     }
     return r;
@@ -518,11 +517,14 @@ extern "C" gt_status gt_ply_pack(gt_context* ctx, const void* data, uint64_t len
   e = ply_to_device(ctx, static_cast<const uint8_t*>(data), L, &packed);
   if (e.code != GT_OK) return api_fail(ctx, e.code, e.msg);
   cudaEventRecord(ctx->int1, ctx->stream);
-  ce = cudaMemcpyAsync(out_packed, packed, need,
-                       (flags & GT_FLAG_OUTPUT_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                       ctx->stream);
+  gt_status cs = GT_OK;
+  if (flags & GT_FLAG_OUTPUT_DEVICE)
+    ce = cudaMemcpyAsync(out_packed, packed, need, cudaMemcpyDeviceToDevice, ctx->stream);
+  else
+    cs = api_download(ctx, out_packed, packed, need);
+  cudaFreeAsync(packed, ctx->stream);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
-  cudaFree(packed);
+  if (cs != GT_OK) return cs;
   if (ce != cudaSuccess) return api_fail(ctx, GT_ERR_CUDA, std::string("PLY output copy: ") + cudaGetErrorString(ce));
   if (info) cudaEventElapsedTime(&info->ingest_ms, ctx->int0, ctx->int1);
   return GT_OK;
@@ -551,8 +553,8 @@ extern "C" gt_status gt_scene_create_from_ply(gt_context* ctx, const void* data,
   // the proxies come from the activated values in double, as the reference's do
   gt_status s = gt_scene_create_ex(ctx, packed, L.n, L.stride, alpha_min, act,
                                    (flags & GT_FLAG_FAST_BUILD) | GT_FLAG_INPUT_DEVICE, out);
-  cudaFree(packed);
-  cudaFree(act);
+  cudaFreeAsync(packed, ctx->stream);
+  if (act) cudaFreeAsync(act, ctx->stream);
   if (s == GT_OK && info) cudaEventElapsedTime(&info->ingest_ms, ctx->int0, ctx->int1);
   return s;
 }

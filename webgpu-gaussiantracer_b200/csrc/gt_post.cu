@@ -83,8 +83,13 @@ extern "C" gt_status gt_tonemap(gt_context* ctx, const float* rgba, uint64_t n_p
   };
   if (!(flags & GT_FLAG_INPUT_DEVICE)) {
     e = cudaMallocAsync(&in_tmp, n_pixels * sizeof(float4), ctx->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(in_tmp, rgba, n_pixels * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) {
+      const gt_status st = api_upload(ctx, in_tmp, rgba, n_pixels * sizeof(float4));
+      if (st != GT_OK) {
+        cleanup();
+        return st;
+      }
+    }
     src = in_tmp;
   }
   if (e == cudaSuccess && !(flags & GT_FLAG_OUTPUT_DEVICE)) {
@@ -101,8 +106,13 @@ extern "C" gt_status gt_tonemap(gt_context* ctx, const float* rgba, uint64_t n_p
   k_tonemap<<<(unsigned)blocks, 256, 0, ctx->stream>>>(src, n_pixels, mode, exposure, dst);
   ++ctx->launches;
   e = cudaGetLastError();
-  if (e == cudaSuccess && !(flags & GT_FLAG_OUTPUT_DEVICE))
-    e = cudaMemcpyAsync(out_rgba8, out_tmp, n_pixels * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess && !(flags & GT_FLAG_OUTPUT_DEVICE)) {
+    const gt_status st = api_download(ctx, out_rgba8, out_tmp, n_pixels * sizeof(uint32_t));
+    if (st != GT_OK) {
+      cleanup();
+      return st;
+    }
+  }
   cleanup();
   if (e == cudaSuccess && !(flags & GT_FLAG_ASYNC)) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return api_fail(ctx, GT_ERR_CUDA, std::string("tone map: ") + cudaGetErrorString(e));
