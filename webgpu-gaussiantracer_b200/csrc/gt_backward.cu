@@ -3,11 +3,12 @@
 // README.md:69); the forward it differentiates is tracePath
 // (src/GS_shader.ts:192-273) as implemented in gt_trace.cu.
 //
-// Scheme.  A forward pass writes, per ray and round, t_curr and the
-// transmittance T at the round's start (and, in checkpoint mode, the round's
-// particle indices).  The adjoint then walks each ray's rounds from the last
-// to the first, one warp per ray:
-//   * the round's entries come from the checkpoint, or are found again by a
+// Scheme.  A forward pass writes records per ray (see Ckpt): in checkpoint mode
+// the particle indices of its next 16 contributing entries and the
+// transmittance before them, in replay mode each round's t_curr and
+// transmittance.  The adjoint walks each ray's records from the last to the
+// first, half a warp a ray (replay mode: a warp):
+//   * a record's entries come from the checkpoint, or are found again by a
 //     traversal from the stored t_curr (replay mode; the set is the same: it is
 //     the k closest front-face hits beyond t_curr);
 //   * lanes recompute alpha_i and the SH colour c_i of one entry each, and the
@@ -105,9 +106,9 @@ __device__ __forceinline__ void sh_basis(V3 d, uint32_t deg, float B[16], float 
 //   for every ray of a view (all primary rays start at the camera).
 //   T: transmittance before the entry; a: its alpha; resp: exp(E); craw: SH
 //   colour before the clamp; ga: dL/dalpha; g: dL/dpixel (rgb).
-__device__ __forceinline__ void entry_terms(const SceneDev& S, uint32_t p, const Shade& sd, V3 o, V3 dr, float T,
-                                            float a, float resp, const float craw[3], float ga, const float g[3],
-                                            float v[20]) {
+//   qa: its rotation (w, x, y, z)
+__device__ __forceinline__ void entry_terms(const float4 qa, const Shade& sd, V3 o, V3 dr, float T, float a, float resp,
+                                            const float craw[3], float ga, const float g[3], float v[20]) {
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) v[16 + ch] = craw[ch] > 0.f ? T * a * g[ch] : 0.f;
   v[19] = 0.f;
@@ -133,7 +134,6 @@ __device__ __forceinline__ void entry_terms(const SceneDev& S, uint32_t p, const
     aqd[2] = a02 * qd[0] + a12 * qd[1] + a22 * qd[2];
   }
   const float q[3] = {(float)qd[0], (float)qd[1], (float)qd[2]};
-  const float4 qa = __ldg(S.params + 2 * (size_t)p + 1);
   const float qw = qa.x, qx = qa.y, qy = qa.z, qz = qa.w;
   // rotation of the quaternion (rows); computeResponse's matrix is its transpose
   const float R[3][3] = {{1.f - 2.f * (qy * qy + qz * qz), 2.f * (qx * qy - qw * qz), 2.f * (qx * qz + qw * qy)},
@@ -161,49 +161,72 @@ __device__ __forceinline__ void entry_terms(const SceneDev& S, uint32_t p, const
 }
 
 // Per-warp table of per-particle sums.  The rays of one 8x4 tile composite
-// mostly the same particles, so the warp adds its tile's entry terms here
-// (shared-memory atomics; the entries of one round are distinct particles
-// but for shared-edge duplicates) and each particle's sums reach global
-// memory once per tile: 5 vector atomics per particle and tile instead of
-// per entry.
+// mostly the same particles, so the warp adds its tile's entry terms here and
+// each particle's sums reach global memory once per tile: 5 vector atomics per
+// particle and tile instead of per entry.
 constexpr int kAggSlots = 64;
 struct AggTable {
-  uint32_t key[kAggSlots];     // particle index, kInvalid when empty
-  float val[20][kAggSlots];    // sum i of slot h at val[i][h]: the 16 response sums, the 3 colour sums, 0
+  float4 val[kAggSlots][5];  // the 16 response sums, the 3 colour sums, 0 (16-byte accesses, 80 bytes a slot)
+  uint32_t key[kAggSlots];   // particle index, kInvalid when empty
 };
-// (component-major: lanes adding to different slots meet in one bank only
-// when their slots are 32 apart)
 
 __device__ __forceinline__ void agg_clear(AggTable& A, uint32_t lane) {
   for (uint32_t i = lane; i < (uint32_t)kAggSlots; i += 32) {
     A.key[i] = kInvalid;
 #pragma unroll
-    for (int c = 0; c < 20; ++c) A.val[c][i] = 0.f;
+    for (int c = 0; c < 5; ++c) A.val[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncwarp();
 }
 
-// Adds the terms v of particle p; returns whether p took an empty slot.  The
-// caller keeps at most kAggSlots particles in the table, so the probe finds
-// p or an empty slot within kAggSlots steps; past them (never) the terms go
-// straight to global memory.
-__device__ __forceinline__ bool agg_add(AggTable& A, uint32_t p, const float v[20], float4* G, float4* GS) {
+// Adds the terms v of particle p of every lane that has one (`on`); returns
+// how many particles took an empty slot.  The caller keeps at most kAggSlots
+// particles in the table, so the probe finds p or an empty slot within
+// kAggSlots steps; past them (never) the terms go straight to global memory.
+// Lanes of one particle take turns, so the sums are plain loads and stores of
+// whole slots: atomic adds of 19 floats a lane are as many loops of a load, a
+// compare-and-swap and its round trip (k_backward of 200k Gaussians at 800x800
+// 1.29 ms with them).
+__device__ __forceinline__ uint32_t agg_add(AggTable& A, bool on, uint32_t p, const float v[20], float4* G, float4* GS,
+                                            uint32_t lane) {
   uint32_t h = (p * 2654435761u) >> 26;
-  for (int step = 0; step < kAggSlots; ++step) {
-    const uint32_t prev = atomicCAS(&A.key[h], kInvalid, p);
-    if (prev == kInvalid || prev == p) {
-#pragma unroll
-      for (int i = 0; i < 19; ++i)
-        if (v[i] != 0.f) atomicAdd(&A.val[i][h], v[i]);
-      return prev == kInvalid;
+  bool fresh = false, found = false;
+  if (on) {
+    for (int step = 0; step < kAggSlots; ++step) {
+      const uint32_t prev = atomicCAS(&A.key[h], kInvalid, p);
+      if (prev == kInvalid || prev == p) {
+        fresh = prev == kInvalid;
+        found = true;
+        break;
+      }
+      h = (h + 1) & (kAggSlots - 1);
     }
-    h = (h + 1) & (kAggSlots - 1);
-  }
+    if (!found) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-    atomicAdd(G + 4 * (size_t)p + c, make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
-  atomicAdd(GS + p, make_float4(v[16], v[17], v[18], 0.f));
-  return false;
+      for (int c = 0; c < 4; ++c)
+        atomicAdd(G + 4 * (size_t)p + c, make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
+      atomicAdd(GS + p, make_float4(v[16], v[17], v[18], 0.f));
+    }
+  }
+  const uint32_t peers = __match_any_sync(kFull, found ? h : (uint32_t)kAggSlots + lane);
+  const uint32_t turn = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  const uint32_t turns = __reduce_max_sync(kFull, found ? turn + 1u : 0u);
+  for (uint32_t i = 0; i < turns; ++i) {
+    if (found && turn == i) {
+      float4* q = A.val[h];
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+        float4 x = q[c];
+        x.x += v[4 * c];
+        x.y += v[4 * c + 1];
+        x.z += v[4 * c + 2];
+        x.w += v[4 * c + 3];
+        q[c] = x;
+      }
+    }
+    __syncwarp();
+  }
+  return (uint32_t)__popc(__ballot_sync(kFull, fresh));
 }
 
 // Adds the table to the scene's response sums G and the view's colour sums
@@ -215,39 +238,245 @@ __device__ __forceinline__ void agg_flush(AggTable& A, float4* G, float4* GS, ui
     if (p == kInvalid) continue;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-      const float4 x = make_float4(A.val[4 * c][i], A.val[4 * c + 1][i], A.val[4 * c + 2][i], A.val[4 * c + 3][i]);
+      const float4 x = A.val[i][c];
       if (x.x != 0.f || x.y != 0.f || x.z != 0.f || x.w != 0.f) atomicAdd(c < 4 ? G + 4 * (size_t)p + c : GS + p, x);
-      A.val[4 * c][i] = 0.f;
-      A.val[4 * c + 1][i] = 0.f;
-      A.val[4 * c + 2][i] = 0.f;
-      A.val[4 * c + 3][i] = 0.f;
+      A.val[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     A.key[i] = kInvalid;
   }
   __syncwarp();
 }
 
-// The adjoint, one warp per 8x4 tile of ray slots (the forward's slot
-// numbering): the tiles [tile_begin, tile_end) of the launch's views.  The
-// warp splits into 32 / SEG segments of SEG lanes, each walking one of the
-// tile's rays (a record's up to SEG contributing entries across its lanes);
-// the tile's per-particle sums gather in the warp's table.  Replay mode (a
-// round's entries found again by a warp-wide traversal) runs with SEG = 32.
-template <bool CKPT_PIDX, int SEG>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) k_backward(const ViewDev* __restrict__ views,
-                                                                    uint32_t n_views, uint32_t tile_begin,
-                                                                    uint32_t tile_end, DevCounters* ctr,
-                                                                    const __grid_constant__ FaceTable F,
-                                                                    const Ckpt ck) {
-  static_assert(SEG == 8 || SEG == 16 || SEG == 32, "segment width");
-  static_assert(CKPT_PIDX || SEG == 32, "replay traverses with the whole warp");
-  constexpr uint32_t kGroups = 32 / SEG;
+// One step of a ray's adjoint, SEG lanes a ray, one entry a lane in
+// compositing order: the transmittance before each entry (an exclusive product
+// scan of 1 - alpha from Tstart), dL/dalpha and the entry's terms into the
+// table.  S: g . R, the colour composited behind the step's entries (normalised
+// by the transmittance there), dotted with dL/dpixel; updated to before them.
+template <int SEG>
+__device__ __forceinline__ void adjoint_step(const ViewDev& V, AggTable& A, uint32_t& nfill, bool valid, uint32_t p,
+                                             V3 o, V3 d, const float g[3], float Tstart, float& S, uint32_t lane,
+                                             uint32_t& cballot) {
+  const uint32_t sl_lane = lane % SEG;
+  float alpha = 0.f, resp = 0.f;
+  float craw[3] = {0.f, 0.f, 0.f};
+  Shade sd{};
+  float4 qa = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool contrib = false;
+  if (valid) {
+    sd = load_shade(V.s.shade, p);
+    // (requested together: each is a gather of its own)
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (V.rgb) q = __ldg(V.rgb + p);
+    qa = __ldg(V.s.params + 2 * (size_t)p + 1);
+    resp = response(sd, o, d);
+    alpha = resp * sd.opacity;
+    contrib = V.u.alpha_min < alpha;
+    if (contrib) {
+      if (V.rgb) {
+        // the view's colour table holds max(0, craw): the same signs
+        // and clamped values, which is all the adjoint uses of craw
+        craw[0] = q.x;
+        craw[1] = q.y;
+        craw[2] = q.z;
+      } else {
+        sh_radiance(V.s.sh, p, vnorm(vsub(sd.mu, o)), V.u.deg, craw);
+      }
+    }
+  }
+  cballot = __ballot_sync(kFull, contrib);
+  const float keep = contrib ? 1.0f - alpha : 1.0f;
+  float pre = keep;
+#pragma unroll
+  for (int off = 1; off < SEG; off <<= 1) {
+    const float x = __shfl_up_sync(kFull, pre, off, SEG);
+    if ((int)sl_lane >= off) pre *= x;
+  }
+  float ahead = __shfl_up_sync(kFull, pre, 1, SEG);
+  if (sl_lane == 0) ahead = 1.0f;
+  const float Tme = Tstart * ahead;
+  // dL/dalpha of entry e: T_e (g.c_e - g.R_e), R_e the colour composited
+  // behind e (normalised by T_e (1 - a_e)), i.e. the entries after e in
+  // this step and the later steps' S.  Behind-colours follow
+  // x -> a_e s_e + (1 - a_e) x from the back, so they are an inclusive
+  // suffix scan of these affine maps (composed through shuffles).
+  float sv = 0.f;
+  if (contrib) {
+    const float c0 = craw[0] > 0.f ? craw[0] : 0.f, c1 = craw[1] > 0.f ? craw[1] : 0.f,
+                c2 = craw[2] > 0.f ? craw[2] : 0.f;
+    sv = g[0] * c0 + g[1] * c1 + g[2] * c2;
+  }
+  float fm = keep, fb = contrib ? alpha * sv : 0.f;  // map of entries e.. (from e to the step's end)
+#pragma unroll
+  for (int off = 1; off < SEG; off <<= 1) {
+    const float xm = __shfl_down_sync(kFull, fm, off, SEG);
+    const float xb = __shfl_down_sync(kFull, fb, off, SEG);
+    if ((int)sl_lane + off < SEG) {
+      fb = __fmaf_rn(fm, xb, fb);
+      fm = fm * xm;
+    }
+  }
+  float nm = __shfl_down_sync(kFull, fm, 1, SEG), nb = __shfl_down_sync(kFull, fb, 1, SEG);
+  if ((int)sl_lane + 1 >= SEG) {
+    nm = 1.0f;
+    nb = 0.0f;
+  }
+  const float ga = contrib ? Tme * (sv - __fmaf_rn(nm, S, nb)) : 0.f;
+  S = __fmaf_rn(__shfl_sync(kFull, fm, 0, SEG), S, __shfl_sync(kFull, fb, 0, SEG));
+  // room for this step's particles (all segments) in the table
+  if (nfill + (uint32_t)__popc(cballot) > (uint32_t)kAggSlots) {
+    agg_flush(A, V.grad, V.grad_sh, lane);
+    nfill = 0;
+  }
+  float v[20];
+  if (contrib) entry_terms(qa, sd, o, d, Tme, alpha, resp, craw, ga, g, v);
+  nfill += agg_add(A, contrib, p, v, V.grad, V.grad_sh, lane);
+}
+
+// The adjoint from checkpoint records, one warp per 8x4 tile of ray slots (the
+// forward's slot numbering): the tiles [tile_begin, tile_end) of the launch's
+// views.  Half a warp walks one ray's records back to front (a record's 16
+// contributing entries across its lanes); a half that is done takes the tile's
+// next ray at once, and the next record, of the same ray or the next one, is
+// requested before the current one is worked on.
+//
+// Bound by dependent gathers (record, shading record) and the turns in the
+// table (issue 44 %).  200k Gaussians, 800x800, B200: 0.58 ms (1.29 ms with the
+// halves in step, a record's loads exposed, and atomic adds in the table).
+constexpr int kAdjWarps = 4;
+constexpr int kAdjBlocks = 4;  // an SM (3: 0.69 ms, 5 and 6 spill: 0.74 and 0.85, all with 0.06 around the kernel)
+__global__ void __launch_bounds__(kAdjWarps * 32, kAdjBlocks) k_adjoint(const ViewDev* __restrict__ views, uint32_t n_views,
+                                                               uint32_t tile_begin, uint32_t tile_end,
+                                                               uint32_t parts, DevCounters* ctr, const Ckpt ck) {
+  constexpr int SEG = (int)kCkptChunk;
+  static_assert(SEG == 16, "two rays a warp");
+  __shared__ AggTable tables[kAdjWarps];
+  __shared__ RayStats stats[kAdjWarps];
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t seg = lane / SEG, sl_lane = lane % SEG;
+  AggTable& A = tables[threadIdx.x >> 5];
+  RayStats& st = stats[threadIdx.x >> 5];
+  if (lane == 0) st = RayStats{0, 0, 0, 0, 0, 0};
+  agg_clear(A, lane);
+  uint32_t rays = 0, n_rounds = 0, n_entries = 0, n_contrib = 0;
+  while (true) {
+    uint32_t tile = 0;
+    if (lane == 0) tile = atomicAdd(&ctr->work, 1u);
+    tile = __shfl_sync(kFull, tile, 0);
+    const uint32_t part = tile % parts;
+    tile /= parts;
+    if (tile >= tile_end - tile_begin) break;
+    tile += tile_begin;
+    const uint32_t vi = n_views == 1 ? 0u : find_view(views, n_views, tile);
+    const ViewDev& V = views[vi];
+    // the tile's rays, one a lane
+    uint32_t px, py;
+    tile_pixel(V.tiles_x, tile - V.tile_begin, lane, px, py);
+    uint32_t head = kInvalid;
+    float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (px < V.w && py < V.h) {
+      head = __ldg(ck.head + 32u * tile + lane);
+      g4 = __ldg(V.dL + (size_t)py * V.w + px);
+      if ((g4.x == 0.f && g4.y == 0.f && g4.z == 0.f) || lane % parts != part) head = kInvalid;
+    }
+    uint32_t todo = __ballot_sync(kFull, head != kInvalid);  // rays not yet taken
+    if (todo == 0) continue;
+    rays += lane == 0 ? (uint32_t)__popc(todo) : 0u;
+    V3 o, d_own;
+    ray_gen(V.u, V.w, V.h, head != kInvalid ? px : 0u, head != kInvalid ? py : 0u, o, d_own);
+    // the record a half takes next: its index, its ray, whether it is the ray's last record
+    uint32_t rec = kInvalid, ray = 0;
+    bool last = false;
+    auto take = [&](bool want) {  // halves without a next record take a ray each
+      const uint32_t wm = __ballot_sync(kFull, want);
+#pragma unroll
+      for (uint32_t q = 0; q < 2; ++q) {
+        if (!((wm >> (q * SEG)) & 1u) || todo == 0) continue;
+        const int next = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t h = __shfl_sync(kFull, head, next);
+        if (seg == q) {
+          rec = h;
+          ray = (uint32_t)next;
+          last = true;
+        }
+      }
+    };
+    take(true);
+    // that record's fields
+    float nT = 0.f;
+    uint32_t np = 0, nn = 0, nprev = kInvalid;
+    auto fetch = [&]() {
+      if (rec != kInvalid) {
+        const uint32_t* rr = ck.pool + (size_t)rec * (kCkptHeader + kCkptChunk);
+        const uint4 h = __ldg(reinterpret_cast<const uint4*>(rr));
+        np = __ldg(rr + kCkptHeader + sl_lane);
+        nT = __uint_as_float(h.y);
+        nprev = h.z;
+        nn = h.w;
+      }
+    };
+    fetch();
+    uint32_t nfill = 0;  // particles in the table
+    float S = 0.f;
+    V3 d = mk(0.f, 0.f, 1.f);
+    float g[3] = {0.f, 0.f, 0.f};
+    for (uint32_t guard = 0; guard < 2u * 32u + ck.pool_cap; ++guard) {
+      const bool active = rec != kInvalid;
+      if (!__any_sync(kFull, active)) break;
+      const float T = nT;
+      const uint32_t p = np, n = nn, prev = nprev;
+      {
+        const bool start = active && last;
+        const float dx = __shfl_sync(kFull, d_own.x, (int)ray), dy = __shfl_sync(kFull, d_own.y, (int)ray),
+                    dz = __shfl_sync(kFull, d_own.z, (int)ray);
+        const float gx = __shfl_sync(kFull, g4.x, (int)ray), gy = __shfl_sync(kFull, g4.y, (int)ray),
+                    gz = __shfl_sync(kFull, g4.z, (int)ray);
+        if (start) {
+          d = mk(dx, dy, dz);
+          g[0] = gx;
+          g[1] = gy;
+          g[2] = gz;
+          S = 0.f;
+        }
+      }
+      // the next record on its way
+      rec = active ? prev : kInvalid;
+      last = false;
+      take(rec == kInvalid);
+      fetch();
+      const bool valid = active && sl_lane < n && p != kInvalid;
+      uint32_t cb;
+      adjoint_step<SEG>(V, A, nfill, valid, p, o, d, g, T, S, lane, cb);
+      if (active && sl_lane == 0) {
+        ++n_rounds;
+        n_entries += n;
+        n_contrib += (uint32_t)__popc((cb >> (seg * SEG)) & ((1u << SEG) - 1u));
+      }
+    }
+    // the next tile may be another view's (other colour sums) or scene's
+    agg_flush(A, V.grad, V.grad_sh, lane);
+  }
+  const uint32_t r_ = __reduce_add_sync(kFull, n_rounds), e_ = __reduce_add_sync(kFull, n_entries),
+                 c_ = __reduce_add_sync(kFull, n_contrib);
+  if (lane == 0) {
+    st.rounds += r_;
+    st.entries += e_;
+    st.contributing += c_;
+  }
+  __syncwarp();
+  flush_stats(ctr, st, __reduce_add_sync(kFull, rays), 0u);
+}
+
+// The adjoint in replay mode, one warp per tile and ray: each round's entries
+// are found again by a warp-wide traversal from the round's t_curr.
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) k_adjoint_replay(const ViewDev* __restrict__ views,
+                                                                          uint32_t n_views, uint32_t tile_begin,
+                                                                          uint32_t tile_end, DevCounters* ctr,
+                                                                          const __grid_constant__ FaceTable F,
+                                                                          const Ckpt ck) {
   __shared__ WarpScratch scratch[kWarpsPerBlock];
   __shared__ AggTable tables[kWarpsPerBlock];
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t seg = lane / SEG, sl_lane = lane % SEG;
-  const uint32_t seg_shift = seg * SEG;
-  const uint32_t seg_bits = SEG == 32 ? kFull : ((1u << SEG) - 1u);
   WarpScratch& W = scratch[threadIdx.x >> 5];
   AggTable& A = tables[threadIdx.x >> 5];
   RayStats& st = W.stats;
@@ -264,160 +493,52 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) k_backward(const ViewD
     const ViewDev& V = views[vi];
     const uint32_t k = V.u.k;
     uint32_t nfill = 0;  // particles in the table
-    for (uint32_t base = 0; base < 32; base += kGroups) {
-      // this segment's ray
-      const uint32_t sl = base + seg;
-      const uint32_t item = 32u * tile + sl;
+    for (uint32_t sl = 0; sl < 32; ++sl) {
       uint32_t px, py;
       tile_pixel(V.tiles_x, tile - V.tile_begin, sl, px, py);
-      uint32_t rec = kInvalid;
-      float g[3] = {0.f, 0.f, 0.f};
-      if (px < V.w && py < V.h) {
-        const float4 g4 = V.dL[(size_t)py * V.w + px];
-        if (g4.x != 0.f || g4.y != 0.f || g4.z != 0.f) {
-          rec = ck.head[item];
-          g[0] = g4.x;
-          g[1] = g4.y;
-          g[2] = g4.z;
-        }
-      }
-      V3 o = mk(0.f, 0.f, 0.f), d = mk(0.f, 0.f, 1.f);
-      if (rec != kInvalid) ray_gen(V.u, V.w, V.h, px, py, o, d);
+      if (px >= V.w || py >= V.h) continue;
+      const float4 g4 = V.dL[(size_t)py * V.w + px];
+      if (g4.x == 0.f && g4.y == 0.f && g4.z == 0.f) continue;
+      uint32_t rec = ck.head[32u * tile + sl];
+      if (rec == kInvalid) continue;
+      const float g[3] = {g4.x, g4.y, g4.z};
+      V3 o, d;
+      ray_gen(V.u, V.w, V.h, px, py, o, d);
       const BoxRay br = make_boxray(o, d, V.s.scene_mag);
-      if (rec != kInvalid && sl_lane == 0) ++rays;
-      float S = 0.f;  // g.R: the colour composited behind the current round, dotted with g
-      // records from the last to the first along their links, all segments
-      // in step (a segment whose ray is done idles)
-      for (uint32_t guard = 0; guard < ck.pool_cap; ++guard) {
-        const bool active = rec != kInvalid;
-        if (!__any_sync(kFull, active)) break;
-        uint32_t p = kInvalid, nrec = 0;
-        float2 ri = make_float2(0.f, 0.f);
-        bool valid = false;
-        if (CKPT_PIDX) {
-          if (active) {
-            const uint32_t* rr = ck.pool + (size_t)rec * (kCkptHeader + ck.kc);
-            ri = make_float2(__uint_as_float(rr[0]), __uint_as_float(rr[1]));
-            nrec = rr[3];
-            p = sl_lane < ck.kc ? rr[kCkptHeader + sl_lane] : kInvalid;
-            valid = sl_lane < nrec && p != kInvalid;
-            rec = rr[2];
-          }
-        } else {
-          const uint32_t* rr = ck.pool + (size_t)rec * (kCkptHeader + ck.kc);
-          ri = make_float2(__uint_as_float(rr[0]), __uint_as_float(rr[1]));
-          nrec = rr[3];
-          KBuf<1> kb;
-          kbuf_init(kb, V.u.t_max);
-          traverse8<kCollect>(V.s, F, W, o, d, br, ri.x, V.u.t_max, kb, st, status, lane, (int)k, V.leaf_batch);
-          if (__reduce_or_sync(kFull, status) & (kStatusStackOverflow | kStatusVisitCap | kStatusHitOverflow)) {
-            rec = kInvalid;
-            break;
-          }
-          valid = lane < k && lane < nrec && kb.p[0] != kInvalid;
-          p = kb.p[0];
-          rec = rr[2];
-        }
-        const uint32_t vmask = (__ballot_sync(kFull, valid) >> seg_shift) & seg_bits;
-        const int n = __popc(vmask);
-        float alpha = 0.f, resp = 0.f;
-        float craw[3] = {0.f, 0.f, 0.f};
-        Shade sd;
-        bool contrib = false;
-        if (valid) {
-          sd = load_shade(V.s.shade, p);
-          resp = response(sd, o, d);
-          alpha = resp * sd.opacity;
-          contrib = V.u.alpha_min < alpha;
-          if (contrib) {
-            if (V.rgb) {
-              // the view's colour table holds max(0, craw): the same signs
-              // and clamped values, which is all the adjoint uses of craw
-              const float4 q = __ldg(V.rgb + p);
-              craw[0] = q.x;
-              craw[1] = q.y;
-              craw[2] = q.z;
-            } else {
-              sh_radiance(V.s.sh, p, vnorm(vsub(sd.mu, o)), V.u.deg, craw);
-            }
-          }
-        }
-        const uint32_t cballot = __ballot_sync(kFull, contrib);
-        const uint32_t cmask = (cballot >> seg_shift) & seg_bits;
-        // transmittance before each entry: the round's starting T times the
-        // product of (1 - alpha) over the contributing entries ahead of it
-        // (an exclusive product scan across the segment's lanes)
-        const float keep = contrib ? 1.0f - alpha : 1.0f;
-        float pre = keep;
-#pragma unroll
-        for (int off = 1; off < SEG; off <<= 1) {
-          const float x = __shfl_up_sync(kFull, pre, off, SEG);
-          if ((int)sl_lane >= off) pre *= x;
-        }
-        float ahead = __shfl_up_sync(kFull, pre, 1, SEG);
-        if (sl_lane == 0) ahead = 1.0f;
-        const float Tme = ri.y * ahead;
-        // dL/dalpha of entry e: T_e (g.c_e - g.R_e), R_e the colour composited
-        // behind e (normalised by T_e (1 - a_e)), i.e. the entries after e in
-        // this round and the later rounds' S.  Behind-colours follow
-        // x -> a_e s_e + (1 - a_e) x from the back, so they are an inclusive
-        // suffix scan of these affine maps (composed through shuffles).
-        float sv = 0.f;
-        if (contrib) {
-          const float c0 = craw[0] > 0.f ? craw[0] : 0.f, c1 = craw[1] > 0.f ? craw[1] : 0.f,
-                      c2 = craw[2] > 0.f ? craw[2] : 0.f;
-          sv = g[0] * c0 + g[1] * c1 + g[2] * c2;
-        }
-        float fm = keep, fb = contrib ? alpha * sv : 0.f;  // map of entries e.. (from e to the round's end)
-#pragma unroll
-        for (int off = 1; off < SEG; off <<= 1) {
-          const float xm = __shfl_down_sync(kFull, fm, off, SEG);
-          const float xb = __shfl_down_sync(kFull, fb, off, SEG);
-          if ((int)sl_lane + off < SEG) {
-            fb = __fmaf_rn(fm, xb, fb);
-            fm = fm * xm;
-          }
-        }
-        float nm = __shfl_down_sync(kFull, fm, 1, SEG), nb = __shfl_down_sync(kFull, fb, 1, SEG);
-        if ((int)sl_lane + 1 >= SEG) {
-          nm = 1.0f;
-          nb = 0.0f;
-        }
-        const float ga = contrib ? Tme * (sv - __fmaf_rn(nm, S, nb)) : 0.f;
-        S = __fmaf_rn(__shfl_sync(kFull, fm, 0, SEG), S, __shfl_sync(kFull, fb, 0, SEG));
-        // room for this step's particles (all segments) in the table
-        const uint32_t nc_all = (uint32_t)__popc(cballot);
-        if (nfill + nc_all > (uint32_t)kAggSlots) {
-          agg_flush(A, V.grad, V.grad_sh, lane);
-          nfill = 0;
-        }
-        bool fresh = false;
-        if (contrib) {
-          float v[20];
-          entry_terms(V.s, p, sd, o, d, Tme, alpha, resp, craw, ga, g, v);
-          fresh = agg_add(A, p, v, V.grad, V.grad_sh);
-        }
-        nfill += (uint32_t)__popc(__ballot_sync(kFull, fresh));
-        if (active && sl_lane == 0) {
+      if (lane == 0) ++rays;
+      float S = 0.f;
+      // rounds from the last to the first along their links
+      for (uint32_t guard = 0; guard < ck.pool_cap && rec != kInvalid; ++guard) {
+        const uint32_t* rr = ck.pool + (size_t)rec * (kCkptHeader + ck.kc);
+        const float t_curr = __uint_as_float(rr[0]), T = __uint_as_float(rr[1]);
+        const uint32_t nrec = rr[3];
+        KBuf<1> kb;
+        kbuf_init(kb, V.u.t_max);
+        traverse8<kCollect>(V.s, F, W, o, d, br, t_curr, V.u.t_max, kb, st, status, lane, (int)k, V.leaf_batch);
+        if (__reduce_or_sync(kFull, status) & (kStatusStackOverflow | kStatusVisitCap | kStatusHitOverflow)) break;
+        const bool valid = lane < k && lane < nrec && kb.p[0] != kInvalid;
+        rec = rr[2];
+        const uint32_t vmask = __ballot_sync(kFull, valid);
+        uint32_t cb;
+        adjoint_step<32>(V, A, nfill, valid, kb.p[0], o, d, g, T, S, lane, cb);
+        if (lane == 0) {
           ++n_rounds;
-          n_entries += (uint32_t)n;
-          n_contrib += (uint32_t)__popc(cmask);
+          n_entries += (uint32_t)__popc(vmask);
+          n_contrib += (uint32_t)__popc(cb);
         }
       }
     }
     // the next tile may be another view's (other colour sums) or scene's
     agg_flush(A, V.grad, V.grad_sh, lane);
   }
-  {
-    const uint32_t r_ = __reduce_add_sync(kFull, n_rounds), e_ = __reduce_add_sync(kFull, n_entries),
-                   c_ = __reduce_add_sync(kFull, n_contrib);
-    if (lane == 0) {
-      st.rounds += r_;
-      st.entries += e_;
-      st.contributing += c_;
-    }
-    __syncwarp();
+  const uint32_t r_ = __reduce_add_sync(kFull, n_rounds), e_ = __reduce_add_sync(kFull, n_entries),
+                 c_ = __reduce_add_sync(kFull, n_contrib);
+  if (lane == 0) {
+    st.rounds += r_;
+    st.entries += e_;
+    st.contributing += c_;
   }
+  __syncwarp();
   flush_stats(ctr, st, __reduce_add_sync(kFull, rays), status);
 }
 
@@ -688,6 +809,8 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
       ck.kc = kc;
       ck.mode = m;
       ck.total_tiles = total_tiles;
+      ck.coloured = true;
+      for (const ViewDev& v : vd) ck.coloured = ck.coloured && v.rgb != nullptr;
       ck.key.resize(count);
       for (uint32_t i = 0; i < count; ++i) ck.key[i] = CkptKey{scenes[i], us[i], ws[i], hs[i]};
       ck.valid = true;
@@ -834,6 +957,8 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
     cleanup();
     return sst;
   }
+  bool filled = cs.coloured;
+  for (const ViewDev& v : vd) filled = filled && v.rgb != nullptr;
   Ckpt ck;
   ck.head = cs.head;
   ck.pool = cs.pool;
@@ -873,7 +998,7 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
       BWD_TRY(cudaMemsetAsync(G[s], 0, (size_t)std::max<uint64_t>(scenes[s]->n, 1) * 4 * sizeof(float4), st));
     BWD_TRY(cudaMemsetAsync(gs_all, 0, gs_off * sizeof(float4), st));
     BWD_TRY(cudaMemcpyAsync(ctx->d_views, vd.data(), sizeof(ViewDev) * count, cudaMemcpyHostToDevice, st));
-    if (gi == 0) {
+    if (gi == 0 && !(filled && !reuse)) {  // (else this call's forward has just filled these tables)
       Err ce = launch_view_colours(vd.data(), ctx->d_views, count, ctx->num_sms, st, &ctx->launches);
       if (ce.code != GT_OK) {
         cleanup();
@@ -884,19 +1009,18 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
     {
       const uint32_t tile0 = vd[g0].tile_begin;
       const uint32_t tile1 = vd[g1 - 1].tile_begin + vd[g1 - 1].n_tiles;
-      uint32_t block = kWarpsPerBlock * 32;
-      uint32_t grid = (uint32_t)ctx->num_sms * 4u;  // 4 resident blocks an SM (launch bounds)
-      uint64_t max_grid = ((uint64_t)(tile1 - tile0) + kWarpsPerBlock - 1) / kWarpsPerBlock;
+      const bool replay = cs.mode != 1;
+      const uint32_t warps = replay ? (uint32_t)kWarpsPerBlock : (uint32_t)kAdjWarps;
+      uint32_t grid = (uint32_t)ctx->num_sms * (replay ? 4u : (uint32_t)kAdjBlocks);  // the resident blocks (launch bounds)
+      // few tiles: a quarter of a tile's rays a warp (the tiles with the most
+      // entries decide the time; three 97x75 views of 16k Gaussians 265 -> 45 us)
+      const uint32_t parts = replay || tile1 - tile0 > 2 * grid * warps ? 1u : 4u;
+      const uint64_t max_grid = ((uint64_t)(tile1 - tile0) * parts + warps - 1) / warps;
       if (grid > max_grid) grid = (uint32_t)std::max<uint64_t>(1, max_grid);
-      // lanes per ray: the record's entry slots
-      if (cs.mode == 1 && cs.kc <= 8)
-        k_backward<true, 8><<<grid, block, 0, st>>>(ctx->d_views, count, tile0, tile1, ctx->d_ctr, ctx->faces, ck);
-      else if (cs.mode == 1 && cs.kc <= 16)
-        k_backward<true, 16><<<grid, block, 0, st>>>(ctx->d_views, count, tile0, tile1, ctx->d_ctr, ctx->faces, ck);
-      else if (cs.mode == 1)
-        k_backward<true, 32><<<grid, block, 0, st>>>(ctx->d_views, count, tile0, tile1, ctx->d_ctr, ctx->faces, ck);
+      if (replay)
+        k_adjoint_replay<<<grid, warps * 32, 0, st>>>(ctx->d_views, count, tile0, tile1, ctx->d_ctr, ctx->faces, ck);
       else
-        k_backward<false, 32><<<grid, block, 0, st>>>(ctx->d_views, count, tile0, tile1, ctx->d_ctr, ctx->faces, ck);
+        k_adjoint<<<grid, warps * 32, 0, st>>>(ctx->d_views, count, tile0, tile1, parts, ctx->d_ctr, ck);
       ++ctx->launches;
       BWD_TRY(cudaGetLastError());
     }

@@ -39,6 +39,7 @@ struct CkptStore {
   uint64_t last_records = 0;      // records the last forward needed
   uint32_t total_tiles = 0;
   bool valid = false;
+  bool coloured = false;          // every view of the forward had its colour table
   std::vector<CkptKey> key;
   float fwd_ms = 0.f;
 };
