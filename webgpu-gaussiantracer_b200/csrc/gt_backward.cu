@@ -481,6 +481,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) k_adjoint_replay(const
   AggTable& A = tables[threadIdx.x >> 5];
   RayStats& st = W.stats;
   if (lane == 0) st = RayStats{0, 0, 0, 0, 0, 0};
+  load_face_rows(F, W.faces, lane);
   agg_clear(A, lane);
   uint32_t status = 0, rays = 0, n_rounds = 0, n_entries = 0, n_contrib = 0;
   while (true) {

@@ -72,6 +72,7 @@ struct PacketScratch {
   float tlo[32], thi[32];          // ray intervals; thi = far bound
   uint8_t hn[32];                  // heap sizes
   float4 nbuf[16];                 // the node being visited
+  FaceRows faces;
   RayStats stats;
 };
 // 12.7 KB for 32-entry heaps (16 one-warp blocks an SM: each of the SM's four
@@ -424,7 +425,7 @@ __device__ __forceinline__ void packet_traverse(const SceneDev& S, const FaceTab
             if (nh < kMaxHitsPerProxy) W.hq[nh][lane] = t;
             ++nh;
           };
-          proxy_test<true, decltype(on_hit)&, false>(F, S.w2o, j, o, d, W.tlo[r], tb, on_hit);
+          proxy_faces(F, W.faces, S.w2o, j, o, d, W.tlo[r], tb, on_hit);
           if (nh > kMaxHitsPerProxy) {
             status |= kStatusHitOverflow;
             nh = kMaxHitsPerProxy;
@@ -502,6 +503,7 @@ __global__ void __launch_bounds__(32) k_trace_packet(const ViewDev* __restrict__
   PacketScratch<KB>& W = *reinterpret_cast<PacketScratch<KB>*>(smem_raw);
   const uint32_t lane = threadIdx.x & 31;
   if (lane == 0) W.stats = RayStats{0, 0, 0, 0, 0, 0};
+  load_face_rows(F, W.faces, lane);
   __syncwarp();
   uint32_t status = 0, rays = 0;
   uint32_t n_rounds = 0, n_entries = 0, n_contrib = 0;

@@ -296,7 +296,7 @@ __device__ __forceinline__ float bin_bound(const ProxySlab& S, float u0, float u
 // The two passes of the counting sort over (bin, bucket) cells: SCATTER
 // false counts each cell's entries, true writes them (a cell then holds the
 // next free place of its bin's list).
-// A warp takes 32 proxies and shares their pairs with bins out evenly (a proxy
+// A warp takes 32 proxies (8 of a small scene) and shares their pairs with bins out evenly (a proxy
 // meets one bin or hundreds: with a lane a proxy 158 + 260 us for 1080p and 1M
 // proxies, 74 + 137 so).
 constexpr uint32_t kPassBlock = 128;
@@ -307,7 +307,7 @@ struct PassRow {
 template <bool SCATTER>
 __global__ void __launch_bounds__(kPassBlock) k_list_pass(const ViewDev* __restrict__ views,
                                                    const ListView* __restrict__ lviews, float r_circ,
-                                                   const Lists L) {
+                                                   uint32_t per_warp, const Lists L) {
   const ViewDev& V = views[blockIdx.y];
   const ListView& P = lviews[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
@@ -337,10 +337,11 @@ __global__ void __launch_bounds__(kPassBlock) k_list_pass(const ViewDev* __restr
   __shared__ uint32_t first_s[kPassBlock + kPassBlock / 32];
   PassRow* rows = rows_s + (threadIdx.x & ~31u);
   uint32_t* first = first_s + 33u * (threadIdx.x >> 5);
-  for (uint32_t base = blockIdx.x * blockDim.x; base < V.s.n_kept; base += gridDim.x * blockDim.x) {
-    const uint32_t j = base + threadIdx.x;
+  const uint32_t warps = gridDim.x * (kPassBlock / 32);
+  for (uint32_t w = blockIdx.x * (kPassBlock / 32) + (threadIdx.x >> 5); (uint64_t)w * per_warp < V.s.n_kept; w += warps) {
+    const uint32_t base = w * per_warp, j = base + lane;
     uint32_t total = 0;
-    if (j < V.s.n_kept) {
+    if (lane < per_warp && j < V.s.n_kept) {
       const size_t at = (size_t)P.rec_begin + j;
       const float4 r1 = __ldg(L.rec + 2 * at + 1);
       const uint32_t rx = __float_as_uint(r1.z), ry = __float_as_uint(r1.w);
@@ -384,8 +385,7 @@ __global__ void __launch_bounds__(kPassBlock) k_list_pass(const ViewDev* __restr
         if (first[src + step] <= t) src += step;
       const PassRow& Q = rows[src];
       const uint32_t q = t - first[src], dy = q / Q.nx;
-      const uint32_t jj = base + (threadIdx.x & ~31u) + src;
-      put(Q.bx + (q - dy * Q.nx), Q.by + dy, Q.slab, jj);
+      put(Q.bx + (q - dy * Q.nx), Q.by + dy, Q.slab, base + src);
     }
     __syncwarp();
   }
@@ -491,7 +491,7 @@ constexpr uint32_t kStreamStep = 10;
 
 template <int R>
 struct StreamScratch {
-  float4 face[20][3];                   // (n, p0.x), (p0.yz, e1.xy), (e1.z, e0) of the icosahedron's faces
+  FaceRows faces;
   unsigned long long hk[kStreamKb][R];  // 4-ary min-heap of ray r in column r
   float4 ca[32];                        // outlines of the current survivors: u0, v0, slope, g11
   float cg[32];                         // g22
@@ -508,81 +508,6 @@ struct StreamScratch {
   uint32_t sh[R], sf[R];             // (checkpointing: its record and that record's entries)
   RayStats stats;
 };
-
-// The front-face hits of proxy j (proxy_test<true> without its prefilters on
-// t): the candidate faces of the ray's last plane crossing among the faces
-// that look at it, then the exact triangle test of each.
-//   * The faces are planes n . x = c in antipodal pairs, so the ray enters
-//     pair q's slab at t_q = -(c + s n_q . o) / |n_q . d|, s = sign(n_q . d).
-//     Only faces f with (t_e - t_f) |dn_e| |dn_f| <= gbound, e the face
-//     entered last, can pass the triangle test (proxy_test has the reason; the
-//     bound is 128 u |od|_1 (|oo|_1 + 2), where the first misses were found
-//     below 8, which leaves room for the approximate reciprocals here); pairs
-//     that graze the ray (|n . d| <= tau) send both faces to it.
-//   * The triangle test reads its face from shared memory: lanes test
-//     different faces, and a kernel parameter serves one address at a time.
-template <int R, class OnHit>
-__device__ __forceinline__ void stream_faces(const FaceTable& F, const StreamScratch<R>& S, const float4* w2o,
-                                             uint32_t j, V3 o, V3 d, float t_min, float t_max, OnHit&& on_hit) {
-  const Affine W = load_affine(w2o + 3 * (size_t)j);
-  const V3 oo = xpoint(W, o), od = xdir(W, d);
-  const float l1o = fabsf(oo.x) + fabsf(oo.y) + fabsf(oo.z);
-  const float* m = W.m;
-  const float s = fabsf(d.x) * (fabsf(m[0]) + fabsf(m[1]) + fabsf(m[2])) +
-                  fabsf(d.y) * (fabsf(m[3]) + fabsf(m[4]) + fabsf(m[5])) +
-                  fabsf(d.z) * (fabsf(m[6]) + fabsf(m[7]) + fabsf(m[8]));
-  const float tau = 1e-5f * F.nmax * s;
-  const float gbound = 7.62939453125e-6f * (fabsf(od.x) + fabsf(od.y) + fabsf(od.z)) * (l1o + 2.0f);
-  float dn[10], num[10];
-  float te = -CUDART_INF_F, re = 0.0f, least = CUDART_INF_F;
-#pragma unroll
-  for (int q = 0; q < 10; ++q) {
-    const float nx = F.pn[q][0], ny = F.pn[q][1], nz = F.pn[q][2];
-    dn[q] = __fmaf_rn(nx, od.x, __fmaf_rn(ny, od.y, nz * od.z));
-    const float no = __fmaf_rn(nx, oo.x, __fmaf_rn(ny, oo.y, nz * oo.z));
-    // distance of the origin in front of the pair's front face: -(c + s no)
-    num[q] = -__uint_as_float(__float_as_uint(no) ^ (__float_as_uint(dn[q]) & 0x80000000u)) - F.pca[q];
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(dn[q])));
-    const float t = num[q] * r;
-    if (t > te) {
-      te = t;
-      re = r;
-    }
-    least = fminf(least, fabsf(dn[q]));
-  }
-  uint32_t cand = 0;
-  if (least > 1.01f * tau && te < 1e30f) {
-    const float slack = gbound * re;
-#pragma unroll
-    for (int q = 0; q < 10; ++q)
-      if (!(__fmaf_rn(te, fabsf(dn[q]), -num[q]) > slack)) cand |= 1u << (dn[q] < 0.0f ? F.pa[q] : F.pb[q]);
-  } else {
-    // some pair grazes the ray: its faces and all that may face the ray
-#pragma unroll 1
-    for (int f = 0; f < 20; ++f) {
-      const float4 a = S.face[f][0];
-      if (!((a.x * od.x + a.y * od.y) + a.z * od.z > tau)) cand |= 1u << f;
-    }
-  }
-#pragma unroll 1
-  while (cand) {
-    const int f = __ffs(cand) - 1;
-    cand &= cand - 1;
-    const float4 a = S.face[f][0], b = S.face[f][1], c = S.face[f][2];
-    const V3 n = mk(a.x, a.y, a.z);
-    const float dnf = vdot(n, od);
-    // tri_test
-    const float r = __frcp_rn(dnf);
-    const V3 e2 = vscale(r, vsub(mk(a.w, b.x, b.y), oo));
-    const float t = vdot(n, e2);
-    if (t <= t_min || t_max <= t || t != t) continue;
-    const V3 i = vcross(od, e2);
-    const float beta = vdot(i, mk(b.z, b.w, c.x)), gamma = vdot(i, mk(c.y, c.z, c.w));
-    if (!(beta >= 0.0f && gamma >= 0.0f && beta + gamma <= 1.0f)) continue;
-    if (fabsf(dnf) > tau ? dnf < 0.0f : front_facing(F, f, load_affine(w2o + 3 * (size_t)j), d)) on_hit(t, f);
-  }
-}
 
 // Key of hit (t, p): ordered like (t, p); -0 is folded into +0.
 __device__ __forceinline__ uint32_t s_ord(float x) {
@@ -670,12 +595,7 @@ __global__ void __launch_bounds__(32, 16) k_trace_stream(const ViewDev* __restri
   const uint32_t lt_mask = (1u << lane) - 1u;
   unsigned long long* sp = L.spill + (size_t)blockIdx.x * (kStreamSpill * R);
   if (lane == 0) W.stats = RayStats{0, 0, 0, 0, 0, 0};
-  if (lane < 20) {
-    const float *n = F.n[lane], *p = F.p0[lane], *e1 = F.e1[lane], *e0 = F.e0[lane];
-    W.face[lane][0] = make_float4(n[0], n[1], n[2], p[0]);
-    W.face[lane][1] = make_float4(p[1], p[2], e1[0], e1[1]);
-    W.face[lane][2] = make_float4(e1[2], e0[0], e0[1], e0[2]);
-  }
+  load_face_rows(F, W.faces, lane);
   __syncwarp();
   uint32_t status = 0, rays = 0;
   uint32_t n_rounds = 0, n_entries = 0, n_contrib = 0;
@@ -805,7 +725,7 @@ __global__ void __launch_bounds__(32, 16) k_trace_stream(const ViewDev* __restri
               atomicMin(reinterpret_cast<int*>(&W.lim[pr]), __float_as_int(t < done ? -CUDART_INF_F : t));
             ++nh;
           };
-          stream_faces(F, W, V.s.w2o, j, o, mk(W.dx[pr], W.dy[pr], W.dz[pr]), t_min, t_max, on_hit);
+          proxy_faces(F, W.faces, V.s.w2o, j, o, mk(W.dx[pr], W.dy[pr], W.dz[pr]), t_min, t_max, on_hit);
         }
         const uint32_t found = __reduce_add_sync(kFull, nh);
         if (lane == 0) W.stats.anyhits += found;
@@ -1222,12 +1142,14 @@ Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n
   GT_CUDA_TRY(cudaMemsetAsync(L.cells, 0, ((size_t)n_bins << kListBucketBits) * 4, stream));
   k_list_views<<<(n_views + 63) / 64, 64, 0, stream>>>(d_views, n_views, L.views, L);
   k_list_project<<<dim3(std::max(1u, (kept + 127) / 128), n_views), 128, 0, stream>>>(d_views, L.views, faces.r_circ, L);
-  k_list_pass<false><<<dim3(std::max(1u, (kept + kPassBlock - 1) / kPassBlock), n_views), kPassBlock, 0, stream>>>(
-      d_views, L.views, faces.r_circ, L);
+  // proxies per warp: fewer where they would leave the GPU short of warps
+  const uint32_t per_warp = (uint64_t)kept * n_views >= 32u * 16u * (uint64_t)num_sms ? 32u : 8u;
+  const dim3 pass_grid(std::max(1u, (kept + per_warp * (kPassBlock / 32) - 1) / (per_warp * (kPassBlock / 32))),
+                       n_views);
+  k_list_pass<false><<<pass_grid, kPassBlock, 0, stream>>>(d_views, L.views, faces.r_circ, per_warp, L);
   k_list_rows<<<n_bins, 128, 0, stream>>>(L);
   k_list_bins<<<1, 1024, 0, stream>>>(L, n_bins, counters);
-  k_list_pass<true><<<dim3(std::max(1u, (kept + kPassBlock - 1) / kPassBlock), n_views), kPassBlock, 0, stream>>>(
-      d_views, L.views, faces.r_circ, L);
+  k_list_pass<true><<<pass_grid, kPassBlock, 0, stream>>>(d_views, L.views, faces.r_circ, per_warp, L);
   *launches += 6;
   GT_CUDA_TRY(cudaGetLastError());
   const Ckpt ck = ckpt ? *ckpt : Ckpt{};

@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_trace8(const ViewDev
   WarpScratch& W = scratch[threadIdx.x >> 5];
   RayStats& st = W.stats;
   if (lane == 0) st = RayStats{0, 0, 0, 0, 0, 0};
+  load_face_rows(F, W.faces, lane);
   __syncwarp();
   uint32_t status = 0, rays = 0;
   const uint32_t resumed = resume ? min(ctr->handoff, resume_cap) : 0u;

@@ -66,29 +66,25 @@ __device__ __forceinline__ BoxRay make_boxray(V3 o, V3 d, float scene_mag) {
   return b;
 }
 
-// Ray/proxy test.  Calls on_hit(t, face) for every face hit by the reference
-// triangle test with t in (tlo, thi) that is front-facing (CULL) or any
-// (!CULL).  Four exact filters run before that test; each skips only work
-// whose outcome is already known:
-//   * bounding sphere: every triangle lies inside the circumsphere, and the
-//     triangle test cannot report a point farther than its rounding error
-//     (covered by the 1e-3 + 1e-5 |o_obj| margin) from its triangle;
-//   * facing: dot(n, d_obj) and the reference's world-space facing product
-//     both approximate n^T W2O d within tau = 1e-5 * nmax * sum(|W2O||d|), so
-//     a face whose dot(n, d_obj) exceeds tau is back-facing.  Faces come in
-//     antipodal pairs with n_b == -n_a bit for bit, so dot(n_b, d) ==
-//     -dot(n_a, d) exactly and one dot product serves both;
-//   * t range: the triangle test's t times dn lies within
-//     E = 10 u nmax (|p0|_1 + |o|_1) of num = n.p0 - n.o (u = 2^-24), so a
-//     face with num >= tlo*dn + M or num <= thi*dn - M (dn < 0) has its t
-//     outside (tlo, thi); M = 3e-5 nmax (|o|_1 + 2) + 1e-6 (|tlo|+|thi|)|dn|
-//     is ~50x that error;
-//   * candidate faces (CULL): of the front faces, only those whose plane
-//     crossing lies within the triangle test's rounding reach of the latest
-//     crossing can pass it (the proxy is convex; see the bound below), so
-//     the triangle test runs on about 1.6 faces a proxy instead of 6.7.
-// The bounding-sphere filter of proxy_test on its own: false only when the
-// ray certainly misses proxy j.
+// The icosahedron's faces in shared memory, for lanes that test different faces
+// (a kernel parameter serves one address at a time): (n, p0.x), (p0.yz, e1.xy),
+// (e1.z, e0).
+struct FaceRows {
+  float4 row[20][3];
+};
+// Fills the rows (lane of a warp; the caller synchronises).
+__device__ __forceinline__ void load_face_rows(const FaceTable& F, FaceRows& S, uint32_t lane) {
+  if (lane >= 20) return;
+  const float *n = F.n[lane], *p = F.p0[lane], *e1 = F.e1[lane], *e0 = F.e0[lane];
+  S.row[lane][0] = make_float4(n[0], n[1], n[2], p[0]);
+  S.row[lane][1] = make_float4(p[1], p[2], e1[0], e1[1]);
+  S.row[lane][2] = make_float4(e1[2], e0[0], e0[1], e0[2]);
+}
+
+// The bounding-sphere filter of a proxy: false only when the ray certainly
+// misses proxy j.  Every triangle lies inside the circumsphere, and the
+// triangle test cannot report a point farther than its rounding error (covered
+// by the 1e-3 + 1e-5 |o_obj| margin) from its triangle.
 __device__ __forceinline__ bool proxy_sphere(const FaceTable& F, const float4* w2o, uint32_t j, V3 o, V3 d) {
   Affine W = load_affine(w2o + 3 * (size_t)j);
   V3 oo = xpoint(W, o), od = xdir(W, d);
@@ -102,119 +98,106 @@ __device__ __forceinline__ bool proxy_sphere(const FaceTable& F, const float4* w
   return (r2 <= rp * rp) || !(dd == dd && r2 == r2);
 }
 
-template <bool CULL, class OnHit, bool SPHERE = true>
-__device__ __forceinline__ void proxy_test(const FaceTable& F, const float4* w2o, uint32_t j, V3 o, V3 d, float tlo,
-                                           float thi, OnHit&& on_hit) {
-  Affine W = load_affine(w2o + 3 * (size_t)j);
-  V3 oo = xpoint(W, o), od = xdir(W, d);
-  float l1o = fabsf(oo.x) + fabsf(oo.y) + fabsf(oo.z);
-  if (SPHERE) {
-    float dd = __fmaf_rn(od.x, od.x, __fmaf_rn(od.y, od.y, od.z * od.z));
-    float ox = __fmaf_rn(oo.x, od.x, __fmaf_rn(oo.y, od.y, oo.z * od.z));
-    float tc = -__fdividef(ox, dd);
-    float cx = __fmaf_rn(tc, od.x, oo.x), cy = __fmaf_rn(tc, od.y, oo.y), cz = __fmaf_rn(tc, od.z, oo.z);
-    float r2 = __fmaf_rn(cx, cx, __fmaf_rn(cy, cy, cz * cz));
-    float rp = __fmaf_rn(1e-5f, l1o, F.r_circ + 1e-3f);
-    if (!(r2 <= rp * rp)) {
-      if (dd == dd && r2 == r2) return;  // NaN falls through to the exact test
-    }
+// The faces of proxy j that the reference triangle test hits with t in (tlo,
+// thi), whatever their facing (debugMode 1), as calls on_hit(t, face).
+template <class OnHit>
+__device__ __forceinline__ void proxy_any_face(const FaceTable& F, const float4* w2o, uint32_t j, V3 o, V3 d, float tlo,
+                                               float thi, OnHit&& on_hit) {
+  const Affine W = load_affine(w2o + 3 * (size_t)j);
+  const V3 oo = xpoint(W, o), od = xdir(W, d);
+#pragma unroll 1
+  for (int f = 0; f < 20; ++f) {
+    float dn = vdot(mk(F.n[f][0], F.n[f][1], F.n[f][2]), od);
+    float t;
+    if (tri_test(F, f, oo, tlo, od, thi, dn, t)) on_hit(t, f);
   }
-  if (!CULL) {
+}
+
+// The front-face hits of proxy j: calls on_hit(t, face) for every face that the
+// reference triangle test hits with t in (tlo, thi) and that faces the ray.
+// Two exact filters run before that test; each skips only work whose outcome
+// is already known:
+//   * facing: dot(n, d_obj) and the reference's world-space facing product
+//     both approximate n^T W2O d within tau = 1e-5 * nmax * sum(|W2O||d|), so
+//     a face whose dot(n, d_obj) exceeds tau is back-facing, and one below
+//     -tau is front-facing (the product is within 12 u nmax s of it, u =
+//     2^-24); only faces in between need the product computed;
+//   * candidate faces.  For front faces e, f (dn < -tau) with plane crossings
+//     t_e >= t_f, the ray at t_f lies outside plane e by (t_e - t_f)|dn_e|/|n|
+//     while triangle f lies inside it (the proxy is convex), so the crossing
+//     X_f is at least that far from triangle f.  The reference's triangle test
+//     accepts points only within its rounding of the triangle, about
+//     10 u |od| |p0 - oo| / |dn_f| in barycentric units.  Hence a face can pass
+//     only if (t_e - t_f) |dn_e| |dn_f| stays below a few tens of u |od|_1
+//     (|oo|_1 + 2); faces above 128 u times that are skipped (a CPU check of
+//     4e7 adversarial rays, edges, vertices and grazing faces, found the first
+//     misses below 8, which leaves room for the approximate reciprocals here).
+// The faces are planes n . x = c in antipodal pairs (n_b == -n_a bit for bit),
+// so the ray enters pair q's slab at t_q = -(c + s n_q . o) / |n_q . d|, s =
+// sign(n_q . d): one pass finds the latest entry, a second the faces within
+// the bound of it.  1080p, 1M Gaussians, list tracer: 17.1 -> 14.2 ms against a
+// single pass with products instead of reciprocals, t-range prefilters and the
+// faces in kernel parameters.
+template <class OnHit>
+__device__ __forceinline__ void proxy_faces(const FaceTable& F, const FaceRows& S, const float4* w2o, uint32_t j, V3 o,
+                                            V3 d, float tlo, float thi, OnHit&& on_hit) {
+  const Affine W = load_affine(w2o + 3 * (size_t)j);
+  const V3 oo = xpoint(W, o), od = xdir(W, d);
+  const float l1o = fabsf(oo.x) + fabsf(oo.y) + fabsf(oo.z);
+  const float* m = W.m;
+  const float s = fabsf(d.x) * (fabsf(m[0]) + fabsf(m[1]) + fabsf(m[2])) +
+                  fabsf(d.y) * (fabsf(m[3]) + fabsf(m[4]) + fabsf(m[5])) +
+                  fabsf(d.z) * (fabsf(m[6]) + fabsf(m[7]) + fabsf(m[8]));
+  const float tau = 1e-5f * F.nmax * s;
+  const float gbound = 7.62939453125e-6f * (fabsf(od.x) + fabsf(od.y) + fabsf(od.z)) * (l1o + 2.0f);
+  float dn[10], num[10];
+  float te = -CUDART_INF_F, re = 0.0f, least = CUDART_INF_F;
+#pragma unroll
+  for (int q = 0; q < 10; ++q) {
+    const float nx = F.pn[q][0], ny = F.pn[q][1], nz = F.pn[q][2];
+    dn[q] = __fmaf_rn(nx, od.x, __fmaf_rn(ny, od.y, nz * od.z));
+    const float no = __fmaf_rn(nx, oo.x, __fmaf_rn(ny, oo.y, nz * oo.z));
+    // distance of the origin in front of the pair's front face: -(c + s no)
+    num[q] = -__uint_as_float(__float_as_uint(no) ^ (__float_as_uint(dn[q]) & 0x80000000u)) - F.pca[q];
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(dn[q])));
+    const float t = num[q] * r;
+    if (t > te) {
+      te = t;
+      re = r;
+    }
+    least = fminf(least, fabsf(dn[q]));
+  }
+  uint32_t cand = 0;
+  if (least > 1.01f * tau && te < 1e30f) {
+    const float slack = gbound * re;
+#pragma unroll
+    for (int q = 0; q < 10; ++q)
+      if (!(__fmaf_rn(te, fabsf(dn[q]), -num[q]) > slack)) cand |= 1u << (dn[q] < 0.0f ? F.pa[q] : F.pb[q]);
+  } else {
+    // some pair grazes the ray: its faces and all that may face the ray
 #pragma unroll 1
     for (int f = 0; f < 20; ++f) {
-      float dn = vdot(mk(F.n[f][0], F.n[f][1], F.n[f][2]), od);
-      float t;
-      if (tri_test(F, f, oo, tlo, od, thi, dn, t)) on_hit(t, f);
-    }
-    return;
-  }
-  const float* m = W.m;
-  float s = fabsf(d.x) * (fabsf(m[0]) + fabsf(m[1]) + fabsf(m[2])) +
-            fabsf(d.y) * (fabsf(m[3]) + fabsf(m[4]) + fabsf(m[5])) +
-            fabsf(d.z) * (fabsf(m[6]) + fabsf(m[7]) + fabsf(m[8]));
-  const float tau = 1e-5f * F.nmax * s;
-  const float mbase = 3e-5f * F.nmax * (l1o + 2.0f);
-  const float trange = 1e-6f * (fabsf(tlo) + fminf(fabsf(thi), 1e30f));
-  // Candidate faces.  For front faces e, f (dn < -tau) with plane crossings
-  // t_e >= t_f, the ray at t_f lies outside plane e by (t_e - t_f)|dn_e|/|n|
-  // while triangle f lies inside it (the proxy is convex), so the crossing
-  // X_f is at least that far from triangle f.  The reference's triangle test
-  // accepts points only within its rounding of the triangle, about
-  // 10 u |od| |p0 - oo| / |dn_f| in barycentric units (u = 2^-24).  Hence a
-  // face can pass only if G = num_e dn_f - num_f dn_e = (t_e - t_f) dn_e dn_f
-  // stays below a few tens of u |od|_1 (|oo|_1 + 2); faces above 128 u times
-  // that are skipped (a CPU check of 4e7 adversarial rays, edges, vertices
-  // and grazing faces, found the first misses below 8).  One pass keeps the
-  // face with the largest crossing so far and every face within the bound of
-  // the face that was largest when it was seen, a superset of the faces the
-  // final largest allows; grazing pairs keep both faces.
-  const float gbound = 7.62939453125e-6f * (fabsf(od.x) + fabsf(od.y) + fabsf(od.z)) * (l1o + 2.0f);
-  uint32_t cand = 0;
-  int best = -1;
-  float bnum = 0.0f, bdn = 0.0f;
-#pragma unroll
-  for (int pair = 0; pair < 10; ++pair) {
-    const int fa = F.pa[pair];
-    const V3 na = mk(F.pn[pair][0], F.pn[pair][1], F.pn[pair][2]);
-    const float dna = vdot(na, od);
-    if (fabsf(dna) > tau) {
-      // exactly one face of the pair can face the ray
-      // the pair's values sit at fixed offsets of the table (the loop is
-      // unrolled): no indexed loads, and the pairs' independent products
-      // can overlap
-      const int fb = F.pb[pair];
-      const float ca = F.pca[pair], cb = F.pcb[pair];
-      const int f = dna < 0.0f ? fa : fb;
-      const float dn = dna < 0.0f ? dna : -dna;
-      const float no = __fmaf_rn(na.x, oo.x, __fmaf_rn(na.y, oo.y, na.z * oo.z));
-      const float num = (dna < 0.0f ? ca : cb) - (dna < 0.0f ? no : -no);
-      if (best < 0) {
-        best = f;
-        bnum = num;
-        bdn = dn;
-        cand |= 1u << f;
-      } else {
-        const float G = bnum * dn - num * bdn;
-        if (G < 0.0f) {  // f crosses its plane later: the new largest
-          if (-G > gbound) cand &= ~(1u << best);
-          best = f;
-          bnum = num;
-          bdn = dn;
-          cand |= 1u << f;
-        } else if (G <= gbound) {
-          cand |= 1u << f;
-        }
-      }
-    } else {
-      // grazing pair: both faces go to the exact test
-      cand |= (1u << fa) | (1u << F.pb[pair]);
+      const float4 a = S.row[f][0];
+      if (!((a.x * od.x + a.y * od.y) + a.z * od.z > tau)) cand |= 1u << f;
     }
   }
-  // the exact tests of the candidates: t-range prefilter (faces whose facing
-  // is certain), then the reference's triangle test and facing rule.  The
-  // candidates of non-grazing pairs have dn < -tau: the reference's facing
-  // product (within 12 u nmax s of dn, tau = 1e-5 nmax s) is then negative,
-  // so only the grazing pairs' faces need it computed.
 #pragma unroll 1
   while (cand) {
     const int f = __ffs(cand) - 1;
     cand &= cand - 1;
-    const V3 nf = mk(F.n[f][0], F.n[f][1], F.n[f][2]);
-    const float dn = vdot(nf, od);
-    const bool sure = fabsf(dn) > tau;
-    if (sure) {
-      // the t-range test: t times dn lies within E = 10 u nmax (|p0|_1 +
-      // |o|_1) of num = n.p0 - n.o, so a face with num >= tlo*dn + M or
-      // num <= thi*dn - M (dn < 0) has its t outside (tlo, thi)
-      const float no = __fmaf_rn(nf.x, oo.x, __fmaf_rn(nf.y, oo.y, nf.z * oo.z));
-      const float num = F.c[f] - no;
-      const float mg = __fmaf_rn(trange, fabsf(dn), mbase);
-      if (num >= __fmaf_rn(tlo, dn, mg) || num <= __fmaf_rn(thi, dn, -mg)) continue;
-    }
-    float t;
-    if (tri_test(F, f, oo, tlo, od, thi, dn, t) &&
-        (sure ? dn < 0.0f : front_facing(F, f, load_affine(w2o + 3 * (size_t)j), d)))
-      on_hit(t, f);
+    const float4 a = S.row[f][0], b = S.row[f][1], c = S.row[f][2];
+    const V3 n = mk(a.x, a.y, a.z);
+    const float dnf = vdot(n, od);
+    // tri_test
+    const float r = __frcp_rn(dnf);
+    const V3 e2 = vscale(r, vsub(mk(a.w, b.x, b.y), oo));
+    const float t = vdot(n, e2);
+    if (t <= tlo || thi <= t || t != t) continue;
+    const V3 i = vcross(od, e2);
+    const float beta = vdot(i, mk(b.z, b.w, c.x)), gamma = vdot(i, mk(c.y, c.z, c.w));
+    if (!(beta >= 0.0f && gamma >= 0.0f && beta + gamma <= 1.0f)) continue;
+    if (fabsf(dnf) > tau ? dnf < 0.0f : front_facing(F, f, load_affine(w2o + 3 * (size_t)j), d)) on_hit(t, f);
   }
 }
 

@@ -37,6 +37,7 @@ struct WarpScratch {
   uint32_t pop[4];  // nodes taken by the current pop (lanes 8s..8s+7 test pop[s])
   float hq[kMaxHitsPerProxy][32];  // hits of each lane's proxy, column per lane
   RayStats stats;                  // the warp's work counters (lane 0 writes)
+  FaceRows faces;                  // the caller fills them
   float rs[4];                     // warp-uniform ray state parked during a traversal
   uint32_t ru[8];
 };
@@ -357,7 +358,7 @@ __device__ __forceinline__ void traverse8(const SceneDev& S, const FaceTable& F,
             if (nh < kMaxHitsPerProxy) W.hq[nh][lane] = t;
             ++nh;
           };
-          proxy_test<true, decltype(on_hit)&, false>(F, S.w2o, j, o, d, tlo, tb, on_hit);
+          proxy_faces(F, W.faces, S.w2o, j, o, d, tlo, tb, on_hit);
           if (nh > kMaxHitsPerProxy) {
             status |= kStatusHitOverflow;
             nh = kMaxHitsPerProxy;
@@ -416,10 +417,16 @@ __device__ __forceinline__ void traverse8(const SceneDev& S, const FaceTable& F,
       if (lane == 0) st.proxy_tests += (unsigned)__popc(tested);
       if (have) {
         const float tb = MODE == kCountFront ? t_max : fminf(next_up(thi), t_max);
-        proxy_test<MODE != kClosestAny>(F, S.w2o, j, o, d, tlo, tb, [&](float t, int) {
+        auto on_hit = [&](float t, int) {
           if (nh < kMaxHitsPerProxy) W.hq[nh][lane] = t;
           ++nh;
-        });
+        };
+        if (proxy_sphere(F, S.w2o, j, o, d)) {
+          if (MODE == kClosestAny)
+            proxy_any_face(F, S.w2o, j, o, d, tlo, tb, on_hit);
+          else
+            proxy_faces(F, W.faces, S.w2o, j, o, d, tlo, tb, on_hit);
+        }
         if (nh > kMaxHitsPerProxy) {
           status |= kStatusHitOverflow;
           nh = kMaxHitsPerProxy;
