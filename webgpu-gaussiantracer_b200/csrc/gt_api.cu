@@ -478,7 +478,7 @@ extern "C" gt_status gt_context_create(int device, gt_context** out) {
   make_face_table(&ctx->faces);
   if (ctx->faces.npairs != 10) {
     gt_context_destroy(ctx);
-    return fail(nullptr, GT_ERR_CUDA, "internal error: icosahedron face table has no antipodal pairing");
+    return fail(nullptr, GT_ERR_CUDA, "internal error: icosahedron face table without the expected symmetry");
   }
   *out = ctx;
   return GT_OK;

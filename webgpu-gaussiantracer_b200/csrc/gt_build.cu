@@ -110,6 +110,18 @@ void make_face_table(FaceTable* F) {
       }
     }
   }
+  // the structure pair_dots builds on: one plane offset, the normals' signs and zeros
+  {
+    const float a = F->n[5][0], bb = F->n[1][1], cc = F->n[1][2];
+    const float want[10][3] = {{-a, a, a}, {0, bb, cc},  {0, bb, -cc},  {-a, a, -a}, {-bb, cc, 0},
+                               {a, a, a},  {-cc, 0, bb}, {-bb, -cc, 0}, {-cc, 0, -bb}, {a, a, -a}};
+    bool same = q == 10;
+    for (int r = 0; r < q && same; ++r) {
+      for (int x = 0; x < 3; ++x) same = same && F->n[F->pa[r]][x] == want[r][x];
+      same = same && F->c[F->pa[r]] == F->c[0] && F->c[F->pb[r]] == F->c[0];
+    }
+    if (!same) q = 0;  // (the context is not created)
+  }
   F->npairs = q;
   for (int r = 0; r < q; ++r) {
     for (int a = 0; a < 3; ++a) F->pn[r][a] = F->n[F->pa[r]][a];

@@ -171,8 +171,7 @@ __device__ __forceinline__ bool tri_test(const FaceTable& F, int f, V3 o, float 
 
 // Facing (webrtx/src/glsl/trace.glsl:154-164): n_world = n * W2O, front iff
 // dot(n_world, d_world) < 0.
-__device__ __forceinline__ bool front_facing(const FaceTable& F, int f, const Affine& W, V3 d) {
-  V3 n = mk(F.n[f][0], F.n[f][1], F.n[f][2]);
+__device__ __forceinline__ bool front_facing(V3 n, const Affine& W, V3 d) {
   const float* m = W.m;
   V3 nw = mk(vdot(n, mk(m[0], m[1], m[2])), vdot(n, mk(m[3], m[4], m[5])), vdot(n, mk(m[6], m[7], m[8])));
   return vdot(nw, d) < 0.0f;
