@@ -61,3 +61,16 @@ def test_record_strides_and_alignment(ctx, n, stride, offset):
         b.close()
     finally:
         ctx.device_free(dev)
+
+
+@pytest.mark.parametrize("n", [239, 255, 256, 257, 272, 273, 274, 511, 512, 513])
+@pytest.mark.parametrize("spread", [1.0, 0.0])
+def test_clustering_tasks_at_block_edges(ctx, n, spread):
+    """Nodes whose leaves straddle two blocks of the search for the clusterings
+    to start with; with spread 0 all codes are equal and only the positions in
+    the sorted order tell the leaves apart."""
+    rec = small_scene(n=n, seed=97).gaussiansBuffer.copy()
+    rec[:, 0:3] *= spread
+    s = Scene(ctx, rec, 0.01)
+    _check(s, rec, 0.01)
+    s.close()

@@ -13,21 +13,25 @@
 // that reaches it merges mutual nearest neighbours until at most kPlocKeep
 // remain (one at the root).  One launch, no host round trip.
 //
-// The warp's 32 lanes each climb from one leaf (Apetrei, "Fast and Simple
-// Agglomerative LBVH Construction", 2014: the second child to arrive at a
-// node goes on); when a lane's node holds more than kPlocKeep leaves, the
-// whole warp merges its clusters, one per lane, by shuffles.
+// The nodes of more than kPlocKeep leaves whose children have no more, at most
+// m / (kPlocKeep + 1), each start a warp, which merges the node's clusters, one
+// per lane, and climbs (Apetrei, "Fast and Simple Agglomerative LBVH
+// Construction", 2014: the second child to arrive at a node goes on).
 //
-// Determinism: which clusters merge depends only on the codes, a tie in area
-// goes to the smaller index.  A cluster is labelled by a leaf (the left
+// Determinism: which clusters merge depends only on the codes and boxes, a tie in
+// area goes to the smaller index.  A cluster is labelled by a leaf (the left
 // cluster's label stays), so the label a merge retires numbers its node: the
 // tree and its layout are the same on every run, and no counter is shared (with
 // one atomic counter: 726 us).
 //
-// Bound by the instructions of the climb and of the neighbour search (48 % of
-// issue slots, 29 % of warps resident: most lanes stop after a few nodes).
-// B200, 1M proxies: the clustering loop took about 8 ms (3.5 ms of kernels and
-// 117 host round trips), this kernel takes 660 us; rays visit as many nodes.
+// Bound by instructions while all tasks run and by the longest climb after that
+// (25 nodes, 144 rounds of merges, about 1 us each).  B200, 1M proxies: a
+// clustering loop over the array took about 8 ms (3.5 ms of kernels and 117 host
+// round trips).  One warp for 32 leaves that climbed lane by lane, boxes passed by
+// shuffles: 650 us (a warp's lanes wait for one another, SMs idle 40 %); a warp
+// for each task: 529 us; boxes read from shared memory, the nearest neighbour as
+// the least of 16 integer keys, clusters stored with their boxes: 366 us, and
+// 16 us to find the tasks.
 #include <math_constants.h>
 
 #include <algorithm>
@@ -38,182 +42,236 @@ namespace gt {
 
 constexpr uint32_t kPlocKeep = 16;   // clusters a node leaves to its parent
 constexpr uint32_t kPlocRadius = 8;  // neighbours searched on either side
-constexpr int kPlocBlock = 64;
+constexpr int kPlocBlock = 32;  // (a warp's work varies: 64 threads 583 us, 32 threads 529)
 
+// The warp's clusters in shared memory: (lo, hi.x), (hi.yz), (reference, label).
+// Rows from the number of clusters on hold a box too large to merge with.
 struct PlocWarp {
-  float b[6][32];
-  uint32_t ref[32], label[32];
+  float4 b0[32 + kPlocRadius];
+  float2 b1[32 + kPlocRadius];
+  uint2 id[32];
 };
+constexpr float kPlocFar = 1e30f;  // squared: infinity
 
 __device__ __forceinline__ unsigned long long ploc_delta(const uint32_t* __restrict__ keys, uint32_t i) {
   // codes made distinct by their position
   return ((unsigned long long)(keys[i] ^ keys[i + 1]) << 32) | (i ^ (i + 1));
 }
 
+// One thread a boundary i | i + 1: the radix tree's node that splits there spans
+// the leaves around it whose deltas are smaller, found by at most kPlocKeep + 1
+// steps to either side.  A node of more than kPlocKeep leaves (or the root) whose
+// children have no more each is a task, (lo, hi, split); a child that small whose
+// sibling is larger counts as arrived.
+constexpr int kFindBlock = 256;
+__global__ void __launch_bounds__(kFindBlock) k_hploc_find(const uint32_t* __restrict__ keys, uint32_t m,
+                                                           uint32_t* link, uint4* tasks, uint32_t* count) {
+  constexpr int kHalo = (int)kPlocKeep + 1;
+  __shared__ unsigned long long delta[kFindBlock + 2 * kHalo];  // ~0 past the ends
+  const int64_t first = (int64_t)blockIdx.x * kFindBlock - kHalo;
+  for (int x = threadIdx.x; x < kFindBlock + 2 * kHalo; x += kFindBlock) {
+    const int64_t b = first + x;
+    delta[x] = b >= 0 && b + 1 < (int64_t)m ? ploc_delta(keys, (uint32_t)b) : ~0ull;
+  }
+  __syncthreads();
+  const uint32_t i = blockIdx.x * kFindBlock + threadIdx.x;
+  bool found = false;
+  uint32_t nl = 1, nr = 1;  // leaves on either side, kPlocKeep + 1 for more than kPlocKeep
+  if (i + 1 < m) {
+    const unsigned long long* at = delta + kHalo + threadIdx.x;
+    const unsigned long long mine = *at;
+    while (nl <= kPlocKeep && at[-(int)nl] < mine) ++nl;
+    while (nr <= kPlocKeep && at[nr] < mine) ++nr;
+    const bool sl = nl <= kPlocKeep, sr = nr <= kPlocKeep;
+    found = sl && sr && (nl + nr > kPlocKeep || nl + nr == m);
+    link[i] = sl == sr ? kInvalid : sl ? i + 1 - nl : i + nr;
+  }
+  // places in the block, then one atomic a block (one a warp: 31 us for 1M leaves)
+  __shared__ uint32_t in_block, base;
+  if (threadIdx.x == 0) in_block = 0;
+  __syncthreads();
+  uint32_t place = 0;
+  if (found) place = atomicAdd(&in_block, 1u);
+  __syncthreads();
+  if (threadIdx.x == 0 && in_block) base = atomicAdd(count, in_block);
+  __syncthreads();
+  if (found) tasks[base + place] = make_uint4(i + 1 - nl, i + nr, i + 1, 0u);
+}
+
 __global__ void __launch_bounds__(kPlocBlock) k_hploc(const uint32_t* __restrict__ keys, uint32_t m,
-                                                      const float* __restrict__ leaf_box, uint2* cluster,
-                                                      uint32_t* link, float4* nodes, float* ibox,
+                                                      const float* __restrict__ leaf_box, float4* cluster,
+                                                      uint32_t* link, const uint4* __restrict__ tasks,
+                                                      const uint32_t* __restrict__ count, float4* nodes, float* ibox,
                                                       uint32_t* parent_int, uint32_t* parent_leaf, uint32_t* root) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
   __shared__ PlocWarp scratch[kPlocBlock / 32];
   PlocWarp& S = scratch[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = j < m;
-  uint32_t lo = j, hi = j, split = 0;
-  // (every pass moves each active lane one node up: at most m of them)
-  while (__any_sync(kAll, active)) {
-    if (active) {
-      uint32_t other;
-      if (lo == 0 || (hi != m - 1 && ploc_delta(keys, hi) < ploc_delta(keys, lo - 1))) {
-        other = atomicExch(&link[hi], lo);  // this node is the left child
-        if (other != kInvalid) {
-          split = hi + 1;
-          hi = other;
-        }
-      } else {
-        other = atomicExch(&link[lo - 1], hi);
-        if (other != kInvalid) {
-          split = lo;
-          lo = other;
-        }
-      }
-      if (other == kInvalid) active = false;  // its sibling goes on
-    }
-    uint32_t todo = __ballot_sync(kAll, active && (hi - lo + 1 > kPlocKeep || hi - lo + 1 == m));
-    if (todo) __threadfence();  // the arrivals before the reads of what they announced
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t L = __shfl_sync(kAll, lo, src), H = __shfl_sync(kAll, hi, src), P = __shfl_sync(kAll, split, src);
-      const uint32_t keep = H - L + 1 == m ? 1u : kPlocKeep;
-      // the children's clusters, left then right, one per lane
-      uint32_t ref = kInvalid, label = 0;
-      const uint32_t nl_max = min(P - L, kPlocKeep), nr_max = min(H - P + 1, kPlocKeep);
-      if (lane < nl_max) {
-        const uint2 c = __ldcg(cluster + L + lane);
-        ref = c.x;
-        label = c.y;
-      }
-      const uint32_t nl = __popc(__ballot_sync(kAll, ref != kInvalid));
-      if (lane >= nl) {
-        const uint2 c = lane - nl < nr_max ? __ldcg(cluster + P + (lane - nl)) : make_uint2(kInvalid, 0u);
-        ref = c.x;
-        label = c.y;
-      }
-      uint32_t n = __popc(__ballot_sync(kAll, ref != kInvalid));
-      float b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (lane < n) {
-        const float* s = (ref & kLeafBit) ? leaf_box + 6 * (size_t)(ref & ~kLeafBit) : ibox + 6 * (size_t)ref;
-#pragma unroll
-        for (int a = 0; a < 6; ++a) b[a] = __ldcg(s + a);
-      }
-      while (n > keep) {
-        // nearest neighbour within the radius (a tie keeps the smaller index)
-        float best = CUDART_INF_F;
-        uint32_t nn = lane > 0 ? lane - 1 : 1u;
-#pragma unroll
-        for (uint32_t r = kPlocRadius; r >= 1; --r) {
-          float o[6];
-#pragma unroll
-          for (int a = 0; a < 6; ++a) o[a] = __shfl_down_sync(kAll, b[a], r);
-          const float x = fmaxf(b[3], o[3]) - fminf(b[0], o[0]), y = fmaxf(b[4], o[4]) - fminf(b[1], o[1]),
-                      z = fmaxf(b[5], o[5]) - fminf(b[2], o[2]);
-          const float d = x * y + y * z + z * x;
-          const float e = __shfl_up_sync(kAll, d, r);  // the pair (lane - r, lane)
-          if (lane + r < n && (d < best || (d == best && lane + r < nn))) {
-            best = d;
-            nn = lane + r;
-          }
-          if (lane >= r && lane < n && (e < best || (e == best && lane - r < nn))) {
-            best = e;
-            nn = lane - r;
-          }
-        }
-        const uint32_t back = __shfl_sync(kAll, nn, nn & 31u);
-        bool mutual = lane < n && nn < n && back == lane;
-        if (__ballot_sync(kAll, mutual) == 0) {  // (no order among the areas, as with NaN: the first two)
-          mutual = lane < 2;
-          nn = lane ^ 1u;
-        }
-        const bool merge = mutual && lane < nn, gone = mutual && nn < lane;
-        // the partner's box and reference
-        float o[6];
-#pragma unroll
-        for (int a = 0; a < 6; ++a) o[a] = __shfl_sync(kAll, b[a], nn & 31u);
-        const uint32_t rb = __shfl_sync(kAll, ref, nn & 31u);
-        const uint32_t retired = __shfl_sync(kAll, label, nn & 31u);
-        if (merge) {
-          const uint32_t id = retired - 1u;  // (label 0 is never retired)
-          // binary node: child boxes as (lo.x, hi.x, lo.y, hi.y) x 2, (lo.z, hi.z) x 2, refs
-          nodes[4 * (size_t)id + 0] = make_float4(b[0], b[3], b[1], b[4]);
-          nodes[4 * (size_t)id + 1] = make_float4(o[0], o[3], o[1], o[4]);
-          nodes[4 * (size_t)id + 2] = make_float4(b[2], b[5], o[2], o[5]);
-          nodes[4 * (size_t)id + 3] = make_float4(__uint_as_float(ref), __uint_as_float(rb), 0.f, 0.f);
-          if (ref & kLeafBit) parent_leaf[ref & ~kLeafBit] = id; else parent_int[ref] = id;
-          if (rb & kLeafBit) parent_leaf[rb & ~kLeafBit] = id; else parent_int[rb] = id;
-#pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            b[a] = fminf(b[a], o[a]);
-            b[3 + a] = fmaxf(b[3 + a], o[3 + a]);
-          }
-#pragma unroll
-          for (int a = 0; a < 6; ++a) ibox[6 * (size_t)id + a] = b[a];
-          ref = id;
-        }
-        // close the gaps, in order
-        const uint32_t km = __ballot_sync(kAll, lane < n && !gone);
-        if (lane < n && !gone) {
-          const uint32_t q = __popc(km & lt_mask);
-#pragma unroll
-          for (int a = 0; a < 6; ++a) S.b[a][q] = b[a];
-          S.ref[q] = ref;
-          S.label[q] = label;
-        }
-        n = __popc(km);
-        __syncwarp();
-        if (lane < n) {
-#pragma unroll
-          for (int a = 0; a < 6; ++a) b[a] = S.b[a][lane];
-          ref = S.ref[lane];
-          label = S.label[lane];
-        }
-        __syncwarp();
-      }
-      if (keep == 1u) {
-        if (lane == 0) {
-          *root = ref;
-          parent_int[ref] = kInvalid;
-        }
-      } else if (lane < kPlocKeep && L + lane <= H) {
-        cluster[L + lane] = make_uint2(lane < n ? ref : kInvalid, label);
-      }
-      __threadfence();  // the clusters before the next arrival
-      __syncwarp();
-    }
+  const uint32_t task = blockIdx.x * (kPlocBlock / 32) + (threadIdx.x >> 5);
+  if (task >= *count) return;
+  uint32_t L = tasks[task].x, H = tasks[task].y, P = tasks[task].z;
+  if (lane < kPlocRadius) {
+    S.b0[32 + lane] = make_float4(-kPlocFar, -kPlocFar, -kPlocFar, kPlocFar);
+    S.b1[32 + lane] = make_float2(kPlocFar, kPlocFar);
   }
-}
-
-__global__ void k_hploc_init(uint32_t m, uint2* cluster, uint32_t* link) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  cluster[j] = make_uint2(kLeafBit | j, j);
-  link[j] = kInvalid;
+  uint32_t back_code[kPlocRadius];  // of the neighbour r before; larger than any area where there is none
+#pragma unroll
+  for (uint32_t r = 1; r <= kPlocRadius; ++r) back_code[r - 1] = (kPlocRadius - r) | (lane < r ? 0x7FFFFFF0u : 0u);
+  // (every pass moves the warp one node up: at most m of them)
+  while (true) {
+    // which child of its parent the node is
+    const bool left = L == 0 || (H != m - 1 && ploc_delta(keys, H) < ploc_delta(keys, L - 1));
+    const uint32_t keep = H - L + 1 == m ? 1u : kPlocKeep;
+    // the children's clusters: the left child's by lanes 0..15, the right one's by
+    // 16..31.  A child of at most kPlocKeep leaves has these for clusters.
+    uint32_t ref = kInvalid, label = 0, n;
+    float4 b0;
+    float2 b1;
+    {
+      const uint32_t from = lane < kPlocKeep ? L : P, to = lane < kPlocKeep ? P : H + 1;
+      const uint32_t at = from + (lane & (kPlocKeep - 1u));
+      if (to - from > kPlocKeep) {
+        const float4 v0 = __ldcg(cluster + 2 * (size_t)at), v1 = __ldcg(cluster + 2 * (size_t)at + 1);
+        ref = __float_as_uint(v0.x);
+        label = __float_as_uint(v0.y);
+        b0 = make_float4(v0.z, v0.w, v1.x, v1.y);
+        b1 = make_float2(v1.z, v1.w);
+      } else if (at < to) {
+        const float2* s = reinterpret_cast<const float2*>(leaf_box + 6 * (size_t)at);
+        const float2 v0 = __ldg(s), v1 = __ldg(s + 1);
+        ref = kLeafBit | at;
+        label = at;
+        b0 = make_float4(v0.x, v0.y, v1.x, v1.y);
+        b1 = __ldg(s + 2);
+      }
+      const uint32_t have = __ballot_sync(kAll, ref != kInvalid);
+      n = __popc(have);
+      __syncwarp();
+      if (ref != kInvalid) {
+        const uint32_t q = __popc(have & lt_mask);
+        S.b0[q] = b0;
+        S.b1[q] = b1;
+        S.id[q] = make_uint2(ref, label);
+      }
+      if (lane >= n) {
+        S.b0[lane] = make_float4(-kPlocFar, -kPlocFar, -kPlocFar, kPlocFar);
+        S.b1[lane] = make_float2(kPlocFar, kPlocFar);
+      }
+      __syncwarp();
+      b0 = S.b0[lane];
+      b1 = S.b1[lane];
+      ref = S.id[lane].x;
+      label = S.id[lane].y;
+    }
+    while (n > keep) {
+      // Nearest neighbour within the radius: the least of 16 keys, a merged area
+      // (not negative, so its bits are in order) with the low four bits replaced by
+      // the neighbour's place, earlier first.
+      uint32_t near = 0x7FFFFFFFu, d[kPlocRadius];
+#pragma unroll
+      for (uint32_t r = 1; r <= kPlocRadius; ++r) {
+        const float4 o0 = S.b0[lane + r];
+        const float2 o1 = S.b1[lane + r];
+        const float x = fmaxf(b0.w, o0.w) - fminf(b0.x, o0.x), y = fmaxf(b1.x, o1.x) - fminf(b0.y, o0.y),
+                    z = fmaxf(b1.y, o1.y) - fminf(b0.z, o0.z);
+        d[r - 1] = __float_as_uint(__fmaf_rn(x, y, __fmaf_rn(y, z, z * x)));
+        near = min(near, (d[r - 1] & ~15u) | (kPlocRadius - 1 + r));
+      }
+#pragma unroll
+      for (uint32_t r = 1; r <= kPlocRadius; ++r)
+        near = min(near, (__shfl_up_sync(kAll, d[r - 1], r) & ~15u) | back_code[r - 1]);
+      uint32_t nn = lane + (near & 15u) - kPlocRadius;
+      if ((near & 15u) >= kPlocRadius) ++nn;
+      const uint32_t back = __shfl_sync(kAll, nn, nn & 31u);
+      bool mutual = lane < n && nn < n && back == lane;
+      if (__ballot_sync(kAll, mutual) == 0) {  // (no order among the areas, as with NaN: the first two)
+        mutual = lane < 2;
+        nn = lane ^ 1u;
+      }
+      const bool merge = mutual && lane < nn, gone = mutual && nn < lane;
+      if (merge) {
+        const float4 o0 = S.b0[nn];
+        const float2 o1 = S.b1[nn];
+        const uint2 other = S.id[nn];
+        const uint32_t id = other.y - 1u;  // the label retired (label 0 never is)
+        // binary node: child boxes as (lo.x, hi.x, lo.y, hi.y) x 2, (lo.z, hi.z) x 2, refs
+        nodes[4 * (size_t)id + 0] = make_float4(b0.x, b0.w, b0.y, b1.x);
+        nodes[4 * (size_t)id + 1] = make_float4(o0.x, o0.w, o0.y, o1.x);
+        nodes[4 * (size_t)id + 2] = make_float4(b0.z, b1.y, o0.z, o1.y);
+        nodes[4 * (size_t)id + 3] = make_float4(__uint_as_float(ref), __uint_as_float(other.x), 0.f, 0.f);
+        if (ref & kLeafBit) parent_leaf[ref & ~kLeafBit] = id; else parent_int[ref] = id;
+        if (other.x & kLeafBit) parent_leaf[other.x & ~kLeafBit] = id; else parent_int[other.x] = id;
+        b0 = make_float4(fminf(b0.x, o0.x), fminf(b0.y, o0.y), fminf(b0.z, o0.z), fmaxf(b0.w, o0.w));
+        b1 = make_float2(fmaxf(b1.x, o1.x), fmaxf(b1.y, o1.y));
+        float2* s = reinterpret_cast<float2*>(ibox + 6 * (size_t)id);
+        s[0] = make_float2(b0.x, b0.y);
+        s[1] = make_float2(b0.z, b0.w);
+        s[2] = b1;
+        ref = id;
+      }
+      // close the gaps, in order
+      const uint32_t km = __ballot_sync(kAll, lane < n && !gone);
+      __syncwarp();
+      if (lane < n && !gone) {
+        const uint32_t q = __popc(km & lt_mask);
+        S.b0[q] = b0;
+        S.b1[q] = b1;
+        S.id[q] = make_uint2(ref, label);
+      }
+      n = __popc(km);
+      if (lane >= n) {
+        S.b0[lane] = make_float4(-kPlocFar, -kPlocFar, -kPlocFar, kPlocFar);
+        S.b1[lane] = make_float2(kPlocFar, kPlocFar);
+      }
+      __syncwarp();
+      b0 = S.b0[lane];
+      b1 = S.b1[lane];
+      ref = S.id[lane].x;
+      label = S.id[lane].y;
+    }
+    if (keep == 1u) {
+      if (lane == 0) {
+        *root = ref;
+        parent_int[ref] = kInvalid;
+      }
+      return;
+    }
+    if (lane < kPlocKeep) {  // (the node has more leaves than that)
+      float4* o = cluster + 2 * (size_t)(L + lane);
+      o[0] = make_float4(__uint_as_float(lane < n ? ref : kInvalid), __uint_as_float(label), b0.x, b0.y);
+      o[1] = make_float4(b0.z, b0.w, b1.x, b1.y);
+    }
+    __threadfence();  // the clusters and boxes before the arrival
+    __syncwarp();
+    // the first child to arrive at the parent leaves its far end there
+    uint32_t other = 0;
+    if (lane == 0) other = left ? atomicExch(link + H, L) : atomicExch(link + L - 1, H);
+    other = __shfl_sync(kAll, other, 0);
+    if (other == kInvalid) return;  // its sibling goes on
+    P = left ? H + 1 : L;
+    if (left) H = other; else L = other;
+    __threadfence();  // the arrival before the reads of what it announced
+  }
 }
 
 Err build_ploc(const uint32_t* keys, const float* leaf_box, uint32_t m, cudaStream_t st, float4* nodes, float* ibox,
                uint32_t* parent_int, uint32_t* parent_leaf, uint32_t* root, uint64_t* launches) {
   if (m < 2) return Err{};
-  uint2* cluster = nullptr;  // m clusters, then m links
-  GT_CUDA_TRY(cudaMallocAsync(&cluster, (size_t)m * 12, st));
-  uint32_t* link = reinterpret_cast<uint32_t*>(cluster + m);
-  k_hploc_init<<<(m + 255) / 256, 256, 0, st>>>(m, cluster, link);
-  k_hploc<<<(m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(keys, m, leaf_box, cluster, link, nodes, ibox,
-                                                                   parent_int, parent_leaf, root);
+  const uint32_t most = m / (kPlocKeep + 1) + 1;  // tasks: their nodes are disjoint (one when m <= kPlocKeep)
+  uint4* tasks = nullptr;  // `most` tasks, m clusters (reference, label, box), m links, the count
+  GT_CUDA_TRY(cudaMallocAsync(&tasks, (size_t)most * 16 + (size_t)m * 36 + 4, st));
+  float4* cluster = reinterpret_cast<float4*>(tasks + most);
+  uint32_t* link = reinterpret_cast<uint32_t*>(cluster + 2 * (size_t)m);
+  uint32_t* count = link + m;
+  GT_CUDA_TRY(cudaMemsetAsync(count, 0, 4, st));
+  k_hploc_find<<<(m + kFindBlock - 1) / kFindBlock, kFindBlock, 0, st>>>(keys, m, link, tasks, count);
+  const uint32_t warps = kPlocBlock / 32;
+  k_hploc<<<(most + warps - 1) / warps, kPlocBlock, 0, st>>>(keys, m, leaf_box, cluster, link, tasks, count, nodes,
+                                                             ibox, parent_int, parent_leaf, root);
   *launches += 2;
   cudaError_t e = cudaGetLastError();
-  cudaFreeAsync(cluster, st);
+  cudaFreeAsync(tasks, st);
   GT_CUDA_TRY(e);
   return Err{};
 }
