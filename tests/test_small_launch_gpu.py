@@ -1,0 +1,33 @@
+"""The warp-per-ray kernel's build and k-buffer sizes for launches of few rays
+(below 64 and 160 rays an SM) against the oracle's float render, bit for bit,
+on either side of the lines that choose them, and batches of one shape that
+replay one graph although their views ask for other k-buffers."""
+import numpy as np
+import pytest
+
+from conftest import small_scene, view
+from oracle import oracle
+from gtrace.tracer import Scene
+from test_stream_gpu import _bits, _same
+
+pytestmark = pytest.mark.gpu
+
+
+# 148 SMs: 9,472 rays (64 an SM) and 23,680 (160 an SM)
+@pytest.mark.parametrize("w,h", [(1, 1), (37, 256), (74, 128), (111, 86), (185, 127), (185, 129)])
+@pytest.mark.parametrize("k", [7, 8, 16, 17, 32])
+def test_lines_between_builds_and_buffers(ctx, w, h, k):
+    pg = small_scene(n=2500, seed=83)
+    _same(ctx, pg.gaussiansBuffer, 0.01, view(w, h, k=k, T_min=0.002).uniforms, w, h)
+
+
+def test_one_graph_for_several_buffers(ctx):
+    pg = small_scene(n=2500, seed=84)
+    s, o = Scene(ctx, pg.gaussiansBuffer, 0.01), oracle.Scene(pg.gaussiansBuffer, 0.01, "f32")
+    for w, h in [(60, 50), (100, 90)]:
+        for ks in [(4, 7), (8, 3), (5, 5), (16, 2), (9, 12), (32, 1), (17, 30)]:
+            views = [(s, view(w, h, k=k, pos=(0.1 * k, 0.3, 4.0)).uniforms, w, h) for k in ks]
+            outs, _ = ctx.render_batch(views)
+            for (_, u, ww, hh), out in zip(views, outs):
+                assert np.array_equal(_bits(out), o.render(u, ww, hh)[0].view(np.uint32)), ks
+    s.close()

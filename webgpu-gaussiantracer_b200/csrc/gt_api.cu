@@ -1011,7 +1011,7 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
   // the view table is rebuilt on every call: it takes the shape's k-buffer
   // size and leaf batch here, and the graph's kernel matches its slot count
   const bool packet = !lists.cap && packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, shape, false);
-  apply_shape(ctx->h_views, count, shape);
+  const bool wide = apply_shape(ctx->h_views, count, shape, lists.cap != 0, packet, ctx->num_sms);
   uint32_t kb_max = 1, pkb_max = 1;
   bool any_debug = false;  // the graph's kernel is the debug-mode instantiation
   for (uint32_t q = 0; q < count; ++q) {
@@ -1024,7 +1024,7 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
   auto key = std::make_tuple(count, total_tiles,
                              kmax | (any_debug ? 0x10000u : 0u) | (packet ? 0x20000u : 0u) | (colours ? 0x40000u : 0u) |
                                  (lists.cap ? (lists.rays << 20) | 0x80000u : 0u),
-                             shape.blocks_per_sm,
+                             shape.blocks_per_sm | (wide ? 0x100u : 0u),
                              ((kb_max + 31u) / 32u) | (packet ? (pkb_max << 8) | (shape.handoff_after << 16) : 0u));
   auto it = ctx->graphs.find(key);
   if (it == ctx->graphs.end()) {

@@ -952,7 +952,7 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
   BWD_TRY(talloc((void**)&d_ev, sizeof(ExpandView) * count));
   std::vector<ExpandView> hev(count);
   const LaunchShape shape = api_shape_for(ctx, views[0].scene, views[0].w, views[0].h, views[0].u.k);
-  apply_shape(vd.data(), count, shape);
+  apply_shape(vd.data(), count, shape, false, true, ctx->num_sms);  // (the adjoints use the leaf batch)
   sst = api_assign_colours(ctx, vd.data(), count);  // filled before the first adjoint launch
   if (sst != GT_OK) {
     cleanup();

@@ -306,8 +306,10 @@ struct Lists {
 // Whether launch_trace renders these views with the tile-packet kernel.
 bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, int num_sms,
                    const LaunchShape& shape, bool ckpt);
-// Sets each view's k-buffer size and leaf batch for a launch of either kernel.
-void apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape);
+// Sets each view's k-buffer size and leaf batch for a launch of either kernel
+// (lists: by proxy lists; packet: by tile packets).  True: the warp-per-ray
+// kernel runs in its build for few rays.
+bool apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape, bool lists, bool packet, int num_sms);
 // Fills the colour table of every view that has one (ViewDev::rgb) from the
 // device copy of the view table.
 Err launch_view_colours(const ViewDev* views, const ViewDev* d_views, uint32_t n_views, int num_sms,

@@ -293,6 +293,8 @@ __device__ __forceinline__ float4 trace_ray_warp(const ViewDev& V, const FaceTab
   return make_float4(R.L0, R.L1, R.L2, 1.0f);
 }
 
+constexpr int kWideBlocks = 5;
+
 // Persistent kernel: each warp takes one pixel slot at a time from a global
 // counter (slot = 32 * tile + position in the 8x4 tile, views back to back),
 // so neighbouring pixels run on neighbouring warps at the same time.  With
@@ -303,8 +305,10 @@ __device__ __forceinline__ float4 trace_ray_warp(const ViewDev& V, const FaceTab
 // without spills by 12% on the 1M-Gaussian 1080p view: the kernel is bound by
 // dependent latencies, and more warps hide them better than the spill loads
 // cost (measured 4/5/6/8/10/12/16 blocks: 111/105/104/98/112/121/140 ms).
-template <bool RECORD, bool CKPT, int NB, bool DEBUG>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_trace8(const ViewDev* __restrict__ views, uint32_t n_views,
+// Launches with few rays end with their slowest ray instead: WIDE is the build
+// for those, 5 blocks of 96 registers without the spills (apply_shape).
+template <bool RECORD, bool CKPT, int NB, bool DEBUG, bool WIDE>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, WIDE ? kWideBlocks : 8) k_trace8(const ViewDev* __restrict__ views, uint32_t n_views,
                                                                   uint32_t total_tiles, DevCounters* ctr,
                                                                   const __grid_constant__ FaceTable F,
                                                                   const uint32_t* pixels, uint32_t n_pix,
@@ -393,12 +397,35 @@ bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles,
   return (uint64_t)total_tiles >= (uint64_t)kPacketTilesPerSm * (uint64_t)std::max(1, num_sms);
 }
 
-void apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape) {
+// Launches whose rays go a warp each from the start, by default: 96 registers
+// below 64 rays an SM, and a k-buffer for fewer traversals, below 160 rays an SM
+// (launches of more have lists or keep 64 entries).  B200, us, 8 blocks x 64
+// registers / 5 x 96, each with 64, 96 and 128 entries:
+//             uniform 16k k 6          clusters 1M k 16         clusters 200k k 32
+//   64x64      70  73  74 / 65  65  66  649 583 570 / 597 531 516  241 276 244 / 216 248 215
+//   100x75    101 104 107 / 95  95  97  654 599 613 / 653 588 607  340 289 312 / 299 267 271
+//   160x90    149 154 165 /153 154 159  911 791 842 / 872 769 818  369 443 364 / 377 443 367
+//   256x192   362 380 411 /385 392 402 1757 1647 1928/1844 1847 2094  809 852 887 / 887 891 937
+// (200k k 8 as 1M; 100k k 6 at 160x120: 217 us with 64 entries, 232 with 96.)
+// The rays that list launches hand over have many hits: 96 registers and 128
+// entries (481x271 of 1M Gaussians 1.95 -> 1.70 ms, 960x540 3.35 -> 3.26).
+bool apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape, bool lists, bool packet, int num_sms) {
+  uint64_t rays = 0;
+  bool debug = false;
   for (uint32_t i = 0; i < n_views; ++i) {
     views[i].kbuf = std::max(1u, std::min(kMaxKbuf, std::max(shape.kbuf, views[i].u.k)));
     views[i].pkbuf = std::max(1u, std::min(kMaxPacketKbuf, std::max(shape.packet_kbuf, views[i].u.k)));
     views[i].leaf_batch = std::min(32u, std::max(1u, shape.leaf_batch));
+    rays += (uint64_t)views[i].w * views[i].h;
+    debug = debug || views[i].u.debug != 0;
   }
+  const uint64_t sms = (uint64_t)std::max(1, num_sms);
+  if (debug || packet || (!lists && (shape.packet != 2 || rays >= 160 * sms))) return false;
+  for (uint32_t i = 0; i < n_views; ++i) {
+    const uint32_t k = views[i].u.k;
+    views[i].kbuf = std::max(views[i].kbuf, lists || k > 16 ? 128u : k >= 8 ? 96u : 64u);
+  }
+  return lists || rays < 64 * sms;
 }
 
 // The colour table of each view that has one: thread p of row v writes view
@@ -439,7 +466,7 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
                  uint64_t* launches, ViewDev* d_views, const Ckpt* ckpt, const Handoff* handoff, const Lists* lists) {
   const bool stream_lists = lists && lists->cap && handoff && handoff->rays && handoff->redo;
   const bool packet = !stream_lists && packet_launch(views, n_views, total_tiles, num_sms, shape, ckpt != nullptr);
-  apply_shape(views, n_views, shape);
+  const bool wide = apply_shape(views, n_views, shape, stream_lists, packet, num_sms);
   GT_CUDA_TRY(cudaMemcpyAsync(d_views, views, sizeof(ViewDev) * n_views, cudaMemcpyHostToDevice, stream));
   Err ce = launch_view_colours(views, d_views, n_views, num_sms, stream, launches);
   if (ce.code != GT_OK) return ce;
@@ -455,7 +482,8 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
     if (e.code != GT_OK || !hand) return e;
   }
   uint32_t block = kWarpsPerBlock * 32;
-  uint32_t grid = (uint32_t)num_sms * std::max(1u, shape.blocks_per_sm);
+  const uint32_t per_sm = wide ? (uint32_t)kWideBlocks : std::max(1u, shape.blocks_per_sm);
+  uint32_t grid = (uint32_t)num_sms * per_sm;
   uint64_t warps_needed = (uint64_t)total_tiles * 32u;
   uint64_t max_grid = (warps_needed + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (grid > max_grid) grid = (uint32_t)std::max<uint64_t>(1, max_grid);
@@ -468,21 +496,28 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
   bool debug = false;
   for (uint32_t i = 0; i < n_views; ++i) debug = debug || views[i].u.debug != 0;
   const void* fn;
-  if (ckpt)  // checkpointing renders have debugMode 0
-    fn = nb <= 1   ? (const void*)k_trace8<false, true, 1, false>
-         : nb == 2 ? (const void*)k_trace8<false, true, 2, false>
-         : nb == 3 ? (const void*)k_trace8<false, true, 3, false>
-                   : (const void*)k_trace8<false, true, 4, false>;
+  if (wide)  // (64 entries or more)
+    fn = ckpt ? (nb == 2   ? (const void*)k_trace8<false, true, 2, false, true>
+                 : nb == 3 ? (const void*)k_trace8<false, true, 3, false, true>
+                           : (const void*)k_trace8<false, true, 4, false, true>)
+              : (nb == 2   ? (const void*)k_trace8<false, false, 2, false, true>
+                 : nb == 3 ? (const void*)k_trace8<false, false, 3, false, true>
+                           : (const void*)k_trace8<false, false, 4, false, true>);
+  else if (ckpt)  // checkpointing renders have debugMode 0
+    fn = nb <= 1   ? (const void*)k_trace8<false, true, 1, false, false>
+         : nb == 2 ? (const void*)k_trace8<false, true, 2, false, false>
+         : nb == 3 ? (const void*)k_trace8<false, true, 3, false, false>
+                   : (const void*)k_trace8<false, true, 4, false, false>;
   else if (debug)
-    fn = nb <= 1   ? (const void*)k_trace8<false, false, 1, true>
-         : nb == 2 ? (const void*)k_trace8<false, false, 2, true>
-         : nb == 3 ? (const void*)k_trace8<false, false, 3, true>
-                   : (const void*)k_trace8<false, false, 4, true>;
+    fn = nb <= 1   ? (const void*)k_trace8<false, false, 1, true, false>
+         : nb == 2 ? (const void*)k_trace8<false, false, 2, true, false>
+         : nb == 3 ? (const void*)k_trace8<false, false, 3, true, false>
+                   : (const void*)k_trace8<false, false, 4, true, false>;
   else
-    fn = nb <= 1   ? (const void*)k_trace8<false, false, 1, false>
-         : nb == 2 ? (const void*)k_trace8<false, false, 2, false>
-         : nb == 3 ? (const void*)k_trace8<false, false, 3, false>
-                   : (const void*)k_trace8<false, false, 4, false>;
+    fn = nb <= 1   ? (const void*)k_trace8<false, false, 1, false, false>
+         : nb == 2 ? (const void*)k_trace8<false, false, 2, false, false>
+         : nb == 3 ? (const void*)k_trace8<false, false, 3, false, false>
+                   : (const void*)k_trace8<false, false, 4, false, false>;
   const ViewDev* dv = d_views;
   const uint32_t* no_pix = nullptr;
   uint32_t zero = 0;
@@ -490,7 +525,7 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
   const HandoffRay* resume = hand ? handoff->rays : nullptr;
   const uint32_t resume_cap = hand ? handoff->cap : 0u;
   const uint32_t* redo = stream_lists ? handoff->redo : nullptr;
-  if (hand) grid = (uint32_t)num_sms * std::max(1u, shape.blocks_per_sm);
+  if (hand) grid = (uint32_t)num_sms * per_sm;
   void* args[] = {(void*)&dv, (void*)&n_views, (void*)&total_tiles, (void*)&counters, (void*)&faces,
                   (void*)&no_pix, (void*)&zero, (void*)&ho, (void*)&ck, (void*)&resume, (void*)&resume_cap, (void*)&redo};
   GT_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, stream));
@@ -507,7 +542,7 @@ Err launch_trace_hits(const ViewDev& view, ViewDev* d_views, const uint32_t* pix
   GT_CUDA_TRY(cudaMemcpyAsync(d_views, &view, sizeof(ViewDev), cudaMemcpyHostToDevice, stream));
   HitOut ho{out_pidx, out_t, out_alpha, out_count, out_rounds, out_rgba, max_entries};
   uint32_t grid = std::min<uint32_t>((n_pix + kWarpsPerBlock - 1) / kWarpsPerBlock, 148u * 8u);
-  k_trace8<true, false, 1, true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(d_views, 1, 0, counters, faces, pixels, n_pix, ho,
+  k_trace8<true, false, 1, true, false><<<grid, kWarpsPerBlock * 32, 0, stream>>>(d_views, 1, 0, counters, faces, pixels, n_pix, ho,
                                                                   Ckpt{}, nullptr, 0u, nullptr);
   ++*launches;
   GT_CUDA_TRY(cudaGetLastError());
