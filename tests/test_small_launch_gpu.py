@@ -31,3 +31,18 @@ def test_one_graph_for_several_buffers(ctx):
             for (_, u, ww, hh), out in zip(views, outs):
                 assert np.array_equal(_bits(out), o.render(u, ww, hh)[0].view(np.uint32)), ks
     s.close()
+
+
+@pytest.mark.parametrize("w,h", [(5, 5), (25, 25), (26, 25), (25, 26)])
+def test_line_of_the_colour_table(ctx, w, h):
+    """625 rays of 2,500 particles have no colour table, a ray more has one;
+    as one view, and as a batch whose views count together."""
+    pg = small_scene(n=2500, seed=85)
+    u = view(w, h, k=6).uniforms
+    _same(ctx, pg.gaussiansBuffer, 0.01, u, w, h)
+    s, o = Scene(ctx, pg.gaussiansBuffer, 0.01), oracle.Scene(pg.gaussiansBuffer, 0.01, "f32")
+    ref = o.render(u, w, h)[0].view(np.uint32)
+    for _ in range(2):
+        for out in ctx.render_batch([(s, u, w, h)] * 2)[0]:
+            assert np.array_equal(_bits(out), ref)
+    s.close()

@@ -203,14 +203,21 @@ static gt_status ensure_staging(gt_context* ctx, size_t bytes) {
 // (ViewDev::rgb, filled by k_view_colours before the trace kernels) in the
 // context's colour buffer, grown as needed.  A launch whose tables would
 // take more than kColourBudget bytes, or that has more views than a grid has
-// rows, keeps the per-entry evaluation (same image bits either way).
+// rows, keeps the per-entry evaluation (same image bits either way), and so
+// does a render of few rays, which meets a small part of the particles and
+// waits for the table: below 64 rays an SM and 4 particles a ray (B200, us,
+// with / without the table: 64x64 of 16k k 6 64 / 60, alpha_min 0.01 140 / 144,
+// of 1M 531 / 473, 100x75 of 16k 187 / 195, of 50k 121 / 116, of 1M 585 / 536,
+// 160x90 of 50k 181 / 196, of 1M 795 / 809).
 constexpr uint64_t kColourBudget = 2ull << 30;
-static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n) {
-  uint64_t need = 0;
+static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n, bool render) {
+  uint64_t need = 0, rays = 0;
   for (uint32_t i = 0; i < n; ++i) {
     views[i].rgb = nullptr;
     if (views[i].u.debug == 0) need += views[i].n_particles;
+    rays += (uint64_t)views[i].w * views[i].h;
   }
+  if (render && rays < 64ull * (uint64_t)ctx->num_sms && 4 * rays <= need) return GT_OK;
   if (need == 0 || n > 65535u || need * sizeof(float4) > kColourBudget) return GT_OK;
   if (need > ctx->colours_cap) {
     API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -428,7 +435,9 @@ gt_status api_ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t
                            const LaunchShape& shape, Lists* lists, Handoff* hand) {
   return ensure_lists(ctx, views, n, total_tiles, rays, shape, lists, hand);
 }
-gt_status api_assign_colours(gt_context* ctx, ViewDev* views, uint32_t n) { return assign_colours(ctx, views, n); }
+gt_status api_assign_colours(gt_context* ctx, ViewDev* views, uint32_t n) {
+  return assign_colours(ctx, views, n, false);
+}
 }  // namespace gt
 
 // ============================================================== context
@@ -804,7 +813,7 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
   if (st != GT_OK) return st;
   ViewDev v = make_view(scene, *u, w, h, out, 0);
   v.u.aa = aa ? 1u : 0u;
-  st = assign_colours(ctx, &v, 1);
+  st = assign_colours(ctx, &v, 1, true);
   if (st != GT_OK) return st;
   API_CUDA(ctx, cudaEventRecord(ctx->call0, ctx->stream));
   API_CUDA(ctx, cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), ctx->stream));
@@ -992,7 +1001,7 @@ extern "C" gt_status gt_render_batch(gt_context* ctx, const gt_batch_item* items
       if (st != GT_OK) return st;
     }
   }
-  st = assign_colours(ctx, ctx->h_views, count);
+  st = assign_colours(ctx, ctx->h_views, count, true);
   if (st != GT_OK) return st;
   bool colours = false;  // (the graph holds the colour kernel or not)
   for (uint32_t q = 0; q < count; ++q) colours = colours || ctx->h_views[q].rgb != nullptr;
@@ -1090,7 +1099,7 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
   st = ensure_views(ctx, 1);
   if (st != GT_OK) return st;
   ViewDev v = make_view(scene, *u, w, h, ctx->staging, 0);
-  st = assign_colours(ctx, &v, 1);  // as gt_render renders it
+  st = assign_colours(ctx, &v, 1, true);  // as gt_render renders it
   if (st != GT_OK) return st;
   Handoff hand;
   st = ensure_handoff(ctx, (uint64_t)w * h, &hand);
@@ -1256,7 +1265,7 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
     total_tiles += ctx->h_views[q].n_tiles;
     off += (size_t)it.w * it.h;
   }
-  st = assign_colours(ctx, ctx->h_views, count);  // as gt_render_batch renders it
+  st = assign_colours(ctx, ctx->h_views, count, true);  // as gt_render_batch renders it
   if (st != GT_OK) return st;
   Lists lists;
   st = ensure_lists(ctx, ctx->h_views, count, total_tiles, pixels, LaunchShape(), &lists, &hand);
