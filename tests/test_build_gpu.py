@@ -74,3 +74,29 @@ def test_clustering_tasks_at_block_edges(ctx, n, spread):
     s = Scene(ctx, rec, 0.01)
     _check(s, rec, 0.01)
     s.close()
+
+
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 2049, 151_551, 151_553, 310_007])
+def test_sort_at_block_edges(ctx, n):
+    """Stretches of the sort that are full, one short and one over (148 blocks
+    of 1,024 pairs), with many equal codes: leaves in Morton order, equal codes
+    in the order of the particles."""
+    rng = np.random.default_rng(n)
+    rec = np.zeros((n, 80), np.float32)
+    rec[:, 0:3] = rng.integers(0, 40, size=(n, 3))
+    rec[0, 0:3], rec[1, 0:3] = 0.0, 39.0
+    rec[:, 4:7] = 0.01
+    rec[:, 8] = 1.0
+    rec[:, 12] = 0.5
+    for fast in (False, True):
+        s = Scene(ctx, rec, 0.01, fast_build=fast)
+        _, leaves, info = s.export_bvh()
+        b = np.asarray(s.info()["bounds"], np.float64).reshape(2, 3)
+        s.close()
+        u = (rec[:, 0:3] - b[0]) / (b[1] - b[0]) * 1023.0
+        assert np.abs(u - np.round(u)).min() > 1e-3  # no cell is decided by rounding
+        q, code = np.floor(u).astype(np.uint32), np.zeros(n, np.uint32)
+        for bit in range(10):
+            for a in range(3):
+                code |= ((q[:, a] >> bit) & 1) << (3 * bit + 2 - a)
+        assert np.array_equal(leaves, np.argsort(code, kind="stable"))
