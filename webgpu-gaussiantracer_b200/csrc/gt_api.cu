@@ -205,19 +205,30 @@ static gt_status ensure_staging(gt_context* ctx, size_t bytes) {
 // take more than kColourBudget bytes, or that has more views than a grid has
 // rows, keeps the per-entry evaluation (same image bits either way), and so
 // does a render of few rays, which meets a small part of the particles and
-// waits for the table: below 64 rays an SM and 4 particles a ray (B200, us,
-// with / without the table: 64x64 of 16k k 6 64 / 60, alpha_min 0.01 140 / 144,
-// of 1M 531 / 473, 100x75 of 16k 187 / 195, of 50k 121 / 116, of 1M 585 / 536,
-// 160x90 of 50k 181 / 196, of 1M 795 / 809).
+// waits for the table.  A round evaluates the colours of its k entries at once,
+// so it takes k of 6 or more, and either few entries a ray (a large alpha_min) or
+// very few rays.  B200, time without the table against with it, k 1 / 6 / 16:
+//   64x64 of 16k alpha_min 0.2  -0 /  -5 / -9 %   0.01  +8 / +3 / -1 %
+//   64x64 of 38k alpha_min 0.2  +3 /  -4 / -5 %   0.01  +9 / +3 / -2 %
+//   32x24 of 50k                                  0.01  +3 / -0 / -5 %
+//   100x75 of 200k         0.05  0 /  -3 / -9 %   of 1M 0.01  -2 / -4 / -8 %
+// (64x64 of 16k, k 6, alpha_min 0.2: 64 -> 60 us; of 1M, k 16: 531 -> 473 us).
 constexpr uint64_t kColourBudget = 2ull << 30;
 static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n, bool render) {
   uint64_t need = 0, rays = 0;
+  uint32_t k = 32;
+  float alpha_min = 1.0f;
   for (uint32_t i = 0; i < n; ++i) {
     views[i].rgb = nullptr;
     if (views[i].u.debug == 0) need += views[i].n_particles;
     rays += (uint64_t)views[i].w * views[i].h;
+    k = std::min(k, views[i].u.k);
+    alpha_min = std::min(alpha_min, views[i].u.alpha_min);
   }
-  if (render && rays < 64ull * (uint64_t)ctx->num_sms && 4 * rays <= need) return GT_OK;
+  const uint64_t sms = (uint64_t)ctx->num_sms;
+  if (render && rays < 64 * sms && 4 * rays <= need && k >= 6 &&
+      (alpha_min >= 0.05f || 64 * rays <= need || (k >= 16 && rays < 32 * sms)))
+    return GT_OK;
   if (need == 0 || n > 65535u || need * sizeof(float4) > kColourBudget) return GT_OK;
   if (need > ctx->colours_cap) {
     API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
