@@ -161,7 +161,7 @@ struct LaunchShape {
 };
 constexpr uint32_t kMaxPacketKbuf = 64;
 // A tile packet is a coarse work item: a few tiles whose rays have many
-// hits take several times the mean, so with few tiles per resident warp (16
+// hits take several times the mean, so with few tiles per resident warp (15
 // warps an SM) their tail outweighs the packets' gain even with the handoff
 // (1M-Gaussian view, ms as packets / a ray per warp, with the early handoff
 // once every tile is taken: 480x270 (35 tiles an SM) 14.9 / 5.2; 640x360
