@@ -150,7 +150,7 @@ def make_workload(name: str):
     elif name == "clusters-1m-960x540":
         pg, amin, v = synth.clusters_1m_config()
         v = synth.view(960, 540, (0.0, 0.0, 12.0), k=16)
-        desc = ("1M Gaussians (64 clusters), 960x540 (profiling size of the tile-packet kernel), k=16, "
+        desc = ("1M Gaussians (64 clusters), 960x540 (profiling size of the large-view kernels), k=16, "
                 "alpha_min=0.01, T_min=0.01, SH3")
     elif name == "small-256":
         pg, amin, v = synth.small_config()
@@ -249,9 +249,7 @@ def extra_batched(ctx, reps: int = 2):
                         "240-1080, k=16, alpha_min per scene in {0.01, 0.05, 0.1}, camera radius 8-14",
             "rays": rays, "batched_ms": tb, "plain_ms": tp, "batched_mrays": rays / tb / 1e3,
             "plain_mrays": rays / tp / 1e3, "default_shape_ms": tdef,
-            "shape": {"kernel": "tile packets" if tune["block_threads"] == 32 else "warp per ray",
-                      "kbuf": tune["kbuf"], "handoff_after": tune["handoff_after"],
-                      "blocks_per_sm": tune["blocks_per_sm"], "tile": "8x4", "stack": 256},
+            "shape": shape_label(tune),
             "tuner_default_ms": tune["default_ms"], "tuner_best_ms": tune["best_ms"]}
 
 
@@ -363,9 +361,22 @@ def extra_batched_fwd_bwd(ctx, pg, amin, reps: int = 1, n_views: int = 32):
                         "L2 loss vs perturbed scene",
             "rays": rays, "batched_fwd_bwd_ms": tfb, "plain_fwd_ms": tp, "ratio": tfb / tp,
             "checkpoint_fwd_ms": tfc, "adjoint_ms": info.get("bwd_ms"),
-            "shape": {"kernel": "tile packets" if tune["block_threads"] == 32 else "warp per ray",
-                      "kbuf": tune["kbuf"], "handoff_after": tune["handoff_after"]},
+            "shape": shape_label(tune),
             "mode": "checkpoint" if info.get("used_mode") == 1 else "replay"}
+
+
+DEFAULT_SHAPE = {"block_threads": 32, "kbuf": 0, "handoff_after": 0, "blocks_per_sm": 8, "best_ms": None,
+                 "default_ms": None}
+
+
+def shape_label(tune):
+    """The kernels a tuning result stands for.  A default launch shape that won
+    has the tuner's two times equal: the list tracer for the views timed here."""
+    if not tune["kbuf"] or tune["best_ms"] is not None and tune["best_ms"] == tune["default_ms"]:
+        return {"kernel": "default (proxy lists)"}
+    if tune["block_threads"] == 32:
+        return {"kernel": "tile packets", "kbuf": tune["kbuf"], "handoff_after": tune["handoff_after"]}
+    return {"kernel": "warp per ray", "kbuf": tune["kbuf"], "blocks_per_sm": tune["blocks_per_sm"]}
 
 
 def main():
@@ -380,7 +391,8 @@ def main():
     ap.add_argument("--ref-step-budget", type=float, default=0.0,
                     help="--impl reference: seconds of CPU work per step (0: 60 s spread over the steps)")
     ap.add_argument("--shape", default=None,
-                    help="packets:KBUF:HANDOFF_AFTER or warp:KBUF: this launch shape instead of the tuner's")
+                    help="default, packets:KBUF:HANDOFF_AFTER or warp:KBUF: this launch shape instead of the "
+                         "tuner's")
     ap.add_argument("--no-extras", action="store_true",
                     help="skip the batched and forward+backward measurements")
     ap.add_argument("--extra", choices=["fwd_bwd", "batched", "batched_fwd_bwd"], default=None,
@@ -469,25 +481,25 @@ def main():
     warm_wall_ms = (time.perf_counter() - t_sc) * 1e3
     warm_info = scene.info()
     out_dev = ctx.device_alloc(rays * 16)
-    # the launch shape for this view from the library's tuner (gt_autotune:
-    # k-buffer size and hand-off point of the tile packets, blocks, k-buffer
-    # and leaf batch of the warp-per-ray kernel), cached by the context and
-    # used by every render below
+    # the launch shape for this view from the library's tuner (gt_autotune: the
+    # default, which for this view is the list tracer, against k-buffer sizes and
+    # hand-off points of the tile packets and blocks, k-buffer and leaf batch of
+    # the warp-per-ray kernel), cached by the context and used by every render
+    # below
     # (--shape installs a given shape instead, without the tuner's launches:
     # the profiling commands use it so that their launch lists hold renders)
-    if args.shape:
+    if args.shape == "default":
+        tune = dict(DEFAULT_SHAPE)
+    elif args.shape:
         kind, kb, ha = (args.shape.split(":") + ["0", "0"])[:3]
         bt = 32 if kind == "packets" else 128
-        ctx.set_tune(scene, v.uniforms, w, h, block_threads=bt, kbuf=int(kb) or (32 if bt == 32 else 64),
-                     handoff_after=int(ha), blocks_per_sm=8)
-        tune = {"block_threads": bt, "kbuf": int(kb), "handoff_after": int(ha), "blocks_per_sm": 8,
+        kb = int(kb) or (32 if bt == 32 else 64)
+        ctx.set_tune(scene, v.uniforms, w, h, block_threads=bt, kbuf=kb, handoff_after=int(ha), blocks_per_sm=8)
+        tune = {"block_threads": bt, "kbuf": kb, "handoff_after": int(ha), "blocks_per_sm": 8,
                 "best_ms": None, "default_ms": None}
     else:
         tune = ctx.autotune(scene, v.uniforms, w, h)
-    shape = {"kernel": "tile packets" if tune["block_threads"] == 32 else "warp per ray", "kbuf": tune["kbuf"],
-             "handoff_after": tune["handoff_after"] if tune["block_threads"] == 32 else None,
-             "blocks_per_sm": tune["blocks_per_sm"] if tune["block_threads"] == 128 else None,
-             "tuned_ms": tune["best_ms"], "default_shape_ms": tune["default_ms"],
+    shape = {**shape_label(tune), "tuned_ms": tune["best_ms"], "default_shape_ms": tune["default_ms"],
              "source": "--shape " + args.shape if args.shape else "gt_autotune"}
     # one synchronous render: counters for the algorithmic byte count
     st0 = ctx.render_device(scene, v.uniforms, w, h, out_dev)
@@ -582,13 +594,13 @@ def main():
                          "l2_hit_pct": prof.get("l2_hit_pct"), "l2_hit_source": prof.get("l2_hit_source"),
                          "issue": issue,
                          # warp execution efficiency: active lanes per warp instruction of the
-                         # tile-packet kernel (a full ncu capture of the 960x540 case)
+                         # main trace kernel (an ncu capture of the 960x540 case)
                          "warp_exec_eff": ({"lanes_per_inst": prof["lanes_per_inst"],
                                             "frac": prof["lanes_per_inst"] / 32.0,
                                             "source": prof.get("lanes_source")}
                                            if prof.get("lanes_per_inst") else None),
-                         "timed": "a render's trace launches (large views: the tile-packet kernel and the "
-                                  "warp-per-ray launch that finishes the rays it hands over)"},
+                         "timed": "a render's trace launches (large views: the proxy lists, the kernel that "
+                                  "streams them and the warp-per-ray launch that finishes the rays it hands over)"},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e, "unit": "Mrays/s", "h2d_bytes_per_step": 112 + 256,
                     "d2h_bytes_per_step": rays * 16},

@@ -109,13 +109,16 @@ typedef struct gt_render_stats {
   uint64_t entries;       /* valid hit entries composited (any alpha)             */
   uint64_t contributing;  /* entries with alpha > alpha_min                       */
   uint64_t proxy_tests;   /* ray-proxy tests                                      */
-  uint64_t node_visits;   /* BVH nodes popped                                     */
+  uint64_t node_visits;   /* BVH nodes popped; by proxy lists: chunks of 32 list
+                             entries scanned (plus the nodes of handed rays)       */
   uint64_t anyhits;       /* front-face proxy hits offered to the k-buffer         */
   uint32_t status_flags;  /* device status word (0 = clean)                       */
-  uint32_t handed;        /* rays that reached the tile packets' traversal limit: the
-                             warp-per-ray kernel finishes those that fit the handoff
-                             buffer (a quarter of the launch's rays), the packets the
-                             rest (0 when the warp-per-ray kernel traced the views)   */
+  uint32_t handed;        /* rays the warp-per-ray kernel finished: of the list tracer,
+                             those still tracing when most of its warps are idle or
+                             whose waiting hits did not fit; of tile packets, those
+                             that reached the traversal limit and fit the handoff
+                             buffer (a quarter of the launch's rays).  0 when the
+                             warp-per-ray kernel traced the views from the start      */
 } gt_render_stats;
 
 typedef struct gt_scene_info {
@@ -137,9 +140,13 @@ uint32_t gt_version(void);
 /* Creates a context on CUDA device `device`.  Replaces the adapter/device
  * request of src/main.ts:396-427.  Besides its scenes, a context keeps the
  * scratch of its largest call so far: staging images, the hand-off buffer,
- * checkpoints, and the colour tables of plain renders (16 bytes per
- * particle per view of a call, at most 2 GiB; each particle's SH colour as
- * seen from the view's camera, computed once per call before tracing). */
+ * checkpoints, the proxy lists of views they serve (52 bytes a proxy and view,
+ * 24 bytes a list entry, 25 entries a proxy to begin with, 57 MB of waiting
+ * hits; at most 8 GiB in all), and the colour tables of plain renders (16
+ * bytes per particle per view of a call, at most 2 GiB; each particle's SH
+ * colour as seen from the view's camera, computed once per call before
+ * tracing; renders of few rays evaluate the colours of their entries instead).
+ * Where a buffer does not fit, the call runs without it, with the same result. */
 gt_status gt_context_create(int device, gt_context** out);
 /* Destroys the context and every scene still alive on it (their handles
  * become invalid). */
@@ -393,7 +400,13 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * No counterpart in the reference.  Times the tracer's launch shapes on the
  * given view and caches the fastest per (GPU, scene-size bucket, image-size
  * bucket, k).  gt_render and gt_render_batch use the cached choice.
- * Two kernels render the plain image (debugMode 0), with identical results:
+ * Three ways render the plain image (debugMode 0), with identical results.
+ * The default for views of at least 160 rays per SM (23,680 on a 148-SM B200):
+ * per-view lists of the proxies that each bin of 16x8 or 32x16 pixels may show,
+ * ordered by distance, which the bin's tiles stream through.  They serve
+ * unsheared cameras with t_min >= 0 and the limits of gt_set_limits at their
+ * defaults, and need the context's scratch (see gt_context_create).  The
+ * others are chosen by block_threads, or by default where lists do not serve:
  *   block_threads 32:  a warp traces the 32 rays of an 8x4 tile together;
  *                      kbuf = k-buffer entries per ray (k..64, default 32),
  *                      handoff_after as below (the tuner times 2 to 8
@@ -402,15 +415,19 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  *   block_threads 128: a warp traces one ray; kbuf = k-buffer entries of a
  *                      traversal (k..128, default 64), blocks_per_sm and
  *                      leaf_batch as below.
- * Without a cached shape a launch takes the first kernel when it has at
- * least 48 8x4 tiles per SM (about 0.23 Mpixels on a 148-SM B200) and the
- * second otherwise: tiles are coarse work items, and with few of them per
- * warp the slowest ones decide the time.  With the first kernel, the rays
- * of a tile that still need hits after three traversals (or after the
- * current one, once every tile of the launch is taken) are finished by
- * the second one (a second launch).  The same choice holds for the
- * checkpointing forward of gt_backward; debug modes and hit recording
- * always use the second kernel. */
+ * Without a cached shape and without lists a launch takes the first of these
+ * when it has at least 48 8x4 tiles per SM (about 0.23 Mpixels on a 148-SM
+ * B200) and the second otherwise: tiles are coarse work items, and with few of
+ * them per warp the slowest ones decide the time.  The rays of a tile packet
+ * that still need hits after three traversals (or after the current one, once
+ * every tile of the launch is taken) are finished by the second one (a second
+ * launch).  The same choice holds for the checkpointing forward of gt_backward;
+ * debug modes and hit recording always use the second.  The default's few-ray
+ * launches of the second kernel (below 160 rays per SM, and the rays that lists
+ * hand over) choose their k-buffer and occupancy themselves.
+ * When the default is fastest, the result names it in _pad (copy the whole
+ * struct to install it again with gt_set_tune); kbuf, blocks_per_sm and the
+ * other fields are then those of a default launch without lists. */
 typedef struct gt_tune_result {
   uint32_t block_threads; /* 32: a warp per 8x4 tile; 128: a warp per ray      */
   uint32_t blocks_per_sm; /* resident blocks per SM of the persistent grid      */
@@ -422,7 +439,7 @@ typedef struct gt_tune_result {
   uint32_t handoff_after; /* block_threads 32: traversals after which a tile   *
                            * hands its unfinished rays to a warp-per-ray       *
                            * launch (0: the default, 3)                         */
-  uint32_t _pad;
+  uint32_t _pad;          /* 0, or the mark of the default launch (see above)   */
 } gt_tune_result;
 
 gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const gt_uniforms* u,
@@ -432,7 +449,7 @@ gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const gt_uniforms*
  * context, out_rgba is not written) and caches the fastest for batches of
  * that shape (the same view count, tile count and k bucket), which
  * gt_render_batch and the checkpointing forward of a batch then use ahead of
- * the per-view cache.  Tried: the tile packets with k-buffers of k, 24, 32,
+ * the per-view cache.  Tried: the default launch, the tile packets with k-buffers of k, 24, 32,
  * 48 and 64 entries and hand-offs after 2, 3, 4 and 6 traversals, and a warp
  * per ray at 4 and 8 blocks per SM.  The tile (8 x 4) and the traversal stack
  * (256 entries) are fixed: other tiles measured within 0.3 %, and a smaller
