@@ -401,7 +401,8 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * given view and caches the fastest per (GPU, scene-size bucket, image-size
  * bucket, k).  gt_render and gt_render_batch use the cached choice.
  * Three ways render the plain image (debugMode 0), with identical results.
- * The default for views of at least 160 rays per SM (23,680 on a 148-SM B200):
+ * The default for views of at least 160 rays per SM (23,680 on a 148-SM B200;
+ * with k of 4 or more, one more for every 14,000 proxies):
  * per-view lists of the proxies that each bin of 16x8 or 32x16 pixels may show,
  * ordered by distance, which the bin's tiles stream through.  They serve
  * unsheared cameras with t_min >= 0 and the limits of gt_set_limits at their
@@ -423,7 +424,7 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * every tile of the launch is taken) are finished by the second one (a second
  * launch).  The same choice holds for the checkpointing forward of gt_backward;
  * debug modes and hit recording always use the second.  The default's few-ray
- * launches of the second kernel (below 160 rays per SM, and the rays that lists
+ * launches of the second kernel (below 240 rays per SM, and the rays that lists
  * hand over) choose their k-buffer and occupancy themselves.
  * When the default is fastest, the result names it in _pad (copy the whole
  * struct to install it again with gt_set_tune); kbuf, blocks_per_sm and the

@@ -1,5 +1,5 @@
 """The warp-per-ray kernel's build and k-buffer sizes for launches of few rays
-(below 56 and 160 rays an SM) against the oracle's float render, bit for bit,
+(below 56 and 240 rays an SM) against the oracle's float render, bit for bit,
 on either side of the lines that choose them, and batches of one shape that
 replay one graph although their views ask for other k-buffers."""
 import numpy as np
@@ -14,7 +14,7 @@ from test_stream_gpu import _bits, _same
 pytestmark = pytest.mark.gpu
 
 
-# 148 SMs: 8,288 rays (56 an SM), 9,472 (64, the colour table's line) and 23,680 (160)
+# 148 SMs: 8,288 rays (56 an SM), 9,472 (64, the colour table's line) and 23,680 (160, where lists begin)
 @pytest.mark.parametrize("w,h", [(1, 1), (37, 256), (74, 128), (111, 86), (185, 127), (185, 129)])
 @pytest.mark.parametrize("k", [7, 8, 16, 17, 32])
 def test_lines_between_builds_and_buffers(ctx, w, h, k):
@@ -64,3 +64,12 @@ def test_lines_of_the_colour_table_and_the_deep_buffer(ctx, k, amin, w, h):
     for out, uu in zip(ctx.render_batch([(s, u, w, h), (s, u2, w, h)])[0], (u, u2)):
         assert np.array_equal(_bits(out), o.render(uu, w, h)[0].view(np.uint32))
     s.close()
+
+
+@pytest.mark.parametrize("k", [3, 4])
+@pytest.mark.parametrize("w,h", [(163, 146), (163, 147)])
+def test_lists_of_larger_scenes(ctx, k, w, h):
+    """160 and 161 rays an SM of 14,100 proxies: with k 4 the lists begin one
+    ray an SM later."""
+    pg = small_scene(n=14_100, seed=89)
+    _same(ctx, pg.gaussiansBuffer, 0.01, view(w, h, k=k, T_min=0.05).uniforms, w, h)

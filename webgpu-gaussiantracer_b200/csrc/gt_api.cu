@@ -264,14 +264,16 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
                               const LaunchShape& shape, Lists* out, Handoff* hand) {
   *out = Lists{};
   if (shape.packet != 2 || !stream_views(views, n, total_tiles, ctx->faces)) return GT_OK;
-  const StreamPlan plan = stream_plan(rays, ctx->num_sms);
-  if (plan.rays == 0) return GT_OK;
-  const uint64_t bins = total_tiles >> plan.shift;
   uint64_t recs = 0;
+  uint32_t k_min = 32;
   for (uint32_t i = 0; i < n; ++i) {
     views[i].rec_begin = (uint32_t)recs;
     recs += views[i].s.n_kept;
+    k_min = std::min(k_min, views[i].u.k);
   }
+  const StreamPlan plan = stream_plan(rays, recs, k_min, ctx->num_sms);
+  if (plan.rays == 0) return GT_OK;
+  const uint64_t bins = total_tiles >> plan.shift;
   constexpr uint64_t kRec = 3 * sizeof(float4) + sizeof(float), kEnt = sizeof(float4) + sizeof(uint2);
   constexpr uint64_t kBin = (4ull << kListBucketBits) + 8;
   // Everything grows with room to spare, so that a scene with a few more proxies

@@ -324,7 +324,7 @@ struct StreamPlan {
   uint32_t rays = 0;   // rays per warp (0: the hierarchy kernels are faster)
   uint32_t shift = 4;  // bins of 2^shift tiles
 };
-StreamPlan stream_plan(uint64_t rays, int num_sms);
+StreamPlan stream_plan(uint64_t rays, uint64_t proxies, uint32_t k_min, int num_sms);
 Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n_views, uint32_t total_tiles,
                         DevCounters* counters, const FaceTable& faces, int num_sms, cudaStream_t stream,
                         uint64_t* launches, const Lists& lists, const Handoff& handoff, const Ckpt* ckpt);

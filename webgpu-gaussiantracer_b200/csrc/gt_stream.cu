@@ -1065,10 +1065,14 @@ static Err launch_stream_r(const ViewDev* d_views, uint32_t n_views, uint32_t to
   const uint32_t items = total_tiles * (32 / R);
   if (grid > items) grid = std::max(1u, items);
   grid = std::min(grid, (uint32_t)(L.spill_bytes / (sizeof(unsigned long long) * kStreamSpill * R)));
-  // (idle warps at which the tiles still tracing hand over, 50 / 75 / 90 / 95 %
-  // / never: 481x271 of 1M Gaussians 2.14 / 2.00 / 2.09 / 2.04 / 2.79 ms,
-  // 256x256 of 16k 440 / 444 / 435 / 418 / 420 us, 1080p within 1 %)
-  hand.late = grid / 10 * 9;
+  // idle warps at which the tiles still tracing hand over: the rays of a
+  // quarter tile lose less to one another, so theirs leave earlier (us with 50 /
+  // 62 / 75 / 90 / 95 % idle: 200x150 of 1M Gaussians 1240 / 1248 / 1237 / 1268 /
+  // 1331, of 200k 394 / 398 / 406 / 426 / 441, 256x256 of 1M 1556 / 1538 / 1590 /
+  // 1599 / 1548, of 16k 353 / 347 / 348 / 348 / 348; with 32 rays a warp 481x271 of
+  // 1M 1992 / 1760 / 1589 / 1693 / 1756, 640x360 2236 / 2123 / 2072 / 2010 / 2132,
+  // 400x300 of 200k 701 / 626 / 560 / 554 / 590, 1080p within 1 %)
+  hand.late = R == 8 ? grid / 8 * 5 : grid / 10 * 9;
   k_trace_stream<R, CKPT><<<grid, 32, smem, stream>>>(d_views, L.views, n_views, total_tiles, counters, faces, L,
                                                       hand, ck);
   ++*launches;
@@ -1122,11 +1126,17 @@ bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, 
 //   400x300      1946 /  646 /  501   1491 /  559 /  614    3951 / 2138 / 1916
 //   800x600      7472 / 1980 / 1155   5542 / 1362 /  970   14931 / 5222 / 3504
 // With few tiles the warps with the most hits decide the time, so fewer rays
-// share one; below 160 rays an SM even those are too few warps.
-StreamPlan stream_plan(uint64_t rays, int num_sms) {
+// share one; below 160 rays an SM even those are too few warps, and the lists of
+// many proxies need a few more rays to pay (warp per ray / 8 rays per warp, us:
+//   179x150 (181 an SM): 200k k 8 418 / 407, 360k k 7 531 / 618, 1M k 8 809 / 951
+//   200x150 (203 an SM): 360k k 7 579 / 570, 700k k 8 535 / 627, 1M k 6 623 / 715
+//   220x160 (238 an SM): 700k k 8 604 / 568, 1M k 8 1084 / 971, k 16 1407 / 1159),
+// unless rounds are so short that a ray per warp pays for each (1M k 1, 200x150:
+// 1852 / 1356).
+StreamPlan stream_plan(uint64_t rays, uint64_t proxies, uint32_t k_min, int num_sms) {
   StreamPlan p;
   const uint64_t per_sm = rays / (uint64_t)std::max(1, num_sms);
-  if (per_sm >= 160) {
+  if (per_sm >= 160 + (k_min >= 4 ? proxies / 14000 : 0)) {
     p.rays = per_sm < 640 ? 8 : 32;
     p.shift = p.rays == 8 ? 2u : 4u;
   }

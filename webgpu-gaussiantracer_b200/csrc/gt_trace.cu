@@ -398,7 +398,7 @@ bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles,
 }
 
 // Launches whose rays go a warp each from the start, by default: 96 registers
-// below 56 rays an SM, and a k-buffer for fewer traversals, below 160 rays an SM
+// below 56 rays an SM, and a k-buffer for fewer traversals, below 240 rays an SM
 // (launches of more have lists or keep 64 entries), where rounds are long enough
 // that 64 entries hold only a few (k 8 to 16) and rays have many entries (a small
 // alpha_min).  B200, us, 8 blocks x 64 registers / 5 x 96, each with 64, 96 and
@@ -423,7 +423,7 @@ bool apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape, boo
     debug = debug || views[i].u.debug != 0;
   }
   const uint64_t sms = (uint64_t)std::max(1, num_sms);
-  if (debug || packet || (!lists && (shape.packet != 2 || rays >= 160 * sms))) return false;
+  if (debug || packet || (!lists && (shape.packet != 2 || rays >= 240 * sms))) return false;
   for (uint32_t i = 0; i < n_views; ++i) {
     const uint32_t k = views[i].u.k;
     const bool deep = k >= 8 && k <= 16 && views[i].u.alpha_min < 0.1f;
