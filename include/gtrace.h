@@ -424,7 +424,7 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * every tile of the launch is taken) are finished by the second one (a second
  * launch).  The same choice holds for the checkpointing forward of gt_backward;
  * debug modes and hit recording always use the second.  The default's few-ray
- * launches of the second kernel (below 240 rays per SM, and the rays that lists
+ * launches of the second kernel (below 56 rays per SM, and the rays that lists
  * hand over) choose their k-buffer and occupancy themselves.
  * When the default is fastest, the result names it in _pad (copy the whole
  * struct to install it again with gt_set_tune); kbuf, blocks_per_sm and the

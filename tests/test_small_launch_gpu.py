@@ -1,5 +1,5 @@
 """The warp-per-ray kernel's build and k-buffer sizes for launches of few rays
-(below 56 and 240 rays an SM) against the oracle's float render, bit for bit,
+(below 56 rays an SM) against the oracle's float render, bit for bit,
 on either side of the lines that choose them, and batches of one shape that
 replay one graph although their views ask for other k-buffers."""
 import numpy as np

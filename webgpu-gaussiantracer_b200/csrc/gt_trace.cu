@@ -398,8 +398,7 @@ bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles,
 }
 
 // Launches whose rays go a warp each from the start, by default: 96 registers
-// below 56 rays an SM, and a k-buffer for fewer traversals, below 240 rays an SM
-// (launches of more have lists or keep 64 entries), where rounds are long enough
+// below 56 rays an SM, and there a k-buffer for fewer traversals, where rounds are long enough
 // that 64 entries hold only a few (k 8 to 16) and rays have many entries (a small
 // alpha_min).  B200, us, 8 blocks x 64 registers / 5 x 96, each with 64, 96 and
 // 128 entries:
@@ -408,7 +407,8 @@ bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles,
 //   100x75    101 104 107 / 95  95  97  654 599 613 / 653 588 607  340 289 312 / 299 267 271
 //   160x90    149 154 165 /153 154 159  911 791 842 / 872 769 818  369 443 364 / 377 443 367
 //   256x192   362 380 411 /385 392 402 1757 1647 1928/1844 1847 2094  809 852 887 / 887 891 937
-// (106x89, 64 rays an SM, 8 blocks against 5: uniform 16k to 65k -6 to +8 %;
+// (160x90 to 220x160, 64 against 96 entries: 250k to 1M k 8 and 16 -14 to +20 %.
+// 106x89, 64 rays an SM, 8 blocks against 5: uniform 16k to 65k -6 to +8 %;
 // 64x64 of 65k, alpha_min 0.2, 64 entries against 96: -10 %.)
 // The rays that list launches hand over have many hits: 96 registers and 128
 // entries (481x271 of 1M Gaussians 1.95 -> 1.70 ms, 960x540 3.35 -> 3.26).
@@ -423,13 +423,13 @@ bool apply_shape(ViewDev* views, uint32_t n_views, const LaunchShape& shape, boo
     debug = debug || views[i].u.debug != 0;
   }
   const uint64_t sms = (uint64_t)std::max(1, num_sms);
-  if (debug || packet || (!lists && (shape.packet != 2 || rays >= 240 * sms))) return false;
+  if (debug || packet || (!lists && (shape.packet != 2 || rays >= 56 * sms))) return false;
   for (uint32_t i = 0; i < n_views; ++i) {
     const uint32_t k = views[i].u.k;
     const bool deep = k >= 8 && k <= 16 && views[i].u.alpha_min < 0.1f;
     views[i].kbuf = std::max(views[i].kbuf, lists ? 128u : deep ? 96u : 64u);
   }
-  return lists || rays < 56 * sms;
+  return true;
 }
 
 // The colour table of each view that has one: thread p of row v writes view
