@@ -1,0 +1,41 @@
+"""Room for the per-view proxy lists (gt_stream.cu, gt_api.cu): lists whose
+lengths pass 2^32 together.  The hierarchy kernels' image of the same view is
+the reference (bit-equal to the oracle, test_parity_gpu.py, test_packet_gpu.py)."""
+import numpy as np
+import pytest
+
+from gtrace.tracer import Context, Scene
+from gtrace.uniforms import look_at, pack_uniforms
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits(a):
+    return np.ascontiguousarray(a, dtype=np.float32).reshape(-1, 4).view(np.uint32)
+
+
+def test_more_list_entries_than_32_bits_count():
+    """135,000 proxies that each cover all 32,768 bins of a 2^20 x 1 image:
+    4.4e9 list entries.  The proxies lie one behind another (0.007 apart, 50 to
+    1,050 from the camera, a field of view of 1 degree), so a ray ends at the
+    first few."""
+    n, w, h = 135_000, 1 << 20, 1
+    rng = np.random.default_rng(91)
+    rec = np.zeros((n, 80), np.float32)
+    rec[:, 0:2] = 0.5 * rng.normal(size=(n, 2))
+    rec[:, 2] = -np.linspace(50.0, 1050.0, n)
+    rec[:, 4:7] = 4.0
+    rec[:, 8] = 1.0
+    rec[:, 12] = 0.6
+    rec[:, 16:19] = rng.normal(size=(n, 3))
+    u = pack_uniforms(look_at((0.0, 0.0, 0.0), (0.0, 0.0, -1.0)), w, h, hfov=1.0, k=4, alpha_min=0.01, T_min=0.02)
+    u.view(np.float32)[17] = u.view(np.float32)[16]  # (anisotropic pixels)
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        got = [c.render(s, u, w, h) for _ in range(2)]
+        c.set_tune(s, u, w, h, kbuf=64, blocks_per_sm=8, block_threads=128)
+        ref = c.render(s, u, w, h)
+        s.close()
+    assert (ref[..., :3].max(axis=-1) > 0).mean() > 0.5
+    for img in got:
+        assert np.array_equal(_bits(img), _bits(ref))

@@ -68,7 +68,7 @@ struct DevCounters {
   unsigned int work2;    // the same for the second kernel of a launch
   unsigned int handoff;  // rays the tile kernels handed to the warp-per-ray kernel
   unsigned int redo;       // rays that kernel traces from the start
-  unsigned int list_pairs; // list entries the launch needed (gt_stream.cu)
+  unsigned int list_pairs; // list entries the launch needed, at most 2^31 - 1 (gt_stream.cu)
 };
 
 // Scene as the kernels see it.  Records of kept proxies are in BVH leaf

@@ -425,6 +425,12 @@ __global__ void __launch_bounds__(128) k_list_rows(const Lists L) {
 // are ordered by length (in powers of two, longest first).  Tiles of long lists
 // take longest, and the launch's end waits on those taken last (256x256 of 16k
 // Gaussians 483 -> 435 us, 960x540 of 1M 3.86 -> 3.67 ms, 1080p unchanged).
+// The sums stop at kListFull, above every capacity (proxies times bins has no
+// bound below 2^32): lists from there on count as not fitting, and a list is
+// shorter than 2^31, so that no position past them wraps either.
+constexpr uint32_t kListFull = 0x7FFFFFFFu;
+__device__ __forceinline__ uint32_t list_add(uint32_t a, uint32_t b) { return min(a + b, kListFull); }
+
 __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bins, DevCounters* ctr) {
   __shared__ uint32_t ws[32];
   __shared__ uint32_t carry;
@@ -436,13 +442,14 @@ __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bi
   for (uint32_t base = 0; base < n_bins; base += 1024) {
     const uint32_t i = base + threadIdx.x;
     const uint32_t v = i < n_bins ? L.bin_base[i] : 0u;
-    if (i < n_bins) atomicAdd(&place[__clz(v)], 1u);
     uint32_t x = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const uint32_t y = __shfl_up_sync(kFull, x, off);
-      if ((int)lane >= off) x += y;
+      if ((int)lane >= off) x = list_add(x, y);
     }
+    uint32_t pre = __shfl_up_sync(kFull, x, 1);
+    if (lane == 0) pre = 0;
     if (lane == 31) ws[warp] = x;
     __syncthreads();
     if (warp == 0) {
@@ -450,15 +457,19 @@ __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bi
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const uint32_t y = __shfl_up_sync(kFull, s, off);
-        if ((int)lane >= off) s += y;
+        if ((int)lane >= off) s = list_add(s, y);
       }
       ws[lane] = s;
     }
     __syncthreads();
-    const uint32_t c = carry;
-    if (i < n_bins) L.bin_base[i] = c + (warp ? ws[warp - 1] : 0u) + x - v;
+    const uint32_t before = list_add(carry, warp ? ws[warp - 1] : 0u);
+    if (i < n_bins) {
+      const uint32_t at = list_add(before, pre);
+      L.bin_base[i] = at;
+      atomicAdd(&place[__clz(list_add(at, v) - at)], 1u);  // (the length that the starts give)
+    }
     __syncthreads();
-    if (threadIdx.x == 1023) carry = c + ws[31];
+    if (threadIdx.x == 1023) carry = list_add(carry, ws[31]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
