@@ -426,9 +426,10 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * debug modes and hit recording always use the second.  The default's few-ray
  * launches of the second kernel (below 56 rays per SM, and the rays that lists
  * hand over) choose their k-buffer and occupancy themselves.
- * When the default is fastest, the result names it in _pad (copy the whole
+ * When none of the timed shapes is faster than the default launch (which goes by
+ * the view, not by the bucket), the result names it in _pad (copy the whole
  * struct to install it again with gt_set_tune); kbuf, blocks_per_sm and the
- * other fields are then those of a default launch without lists. */
+ * other fields are then those of the fastest of these shapes. */
 typedef struct gt_tune_result {
   uint32_t block_threads; /* 32: a warp per 8x4 tile; 128: a warp per ray      */
   uint32_t blocks_per_sm; /* resident blocks per SM of the persistent grid      */

@@ -1,0 +1,22 @@
+"""The launch tuners (gt_autotune, gt_autotune_batch): the default launch is one
+of their candidates."""
+import pytest
+
+from conftest import small_scene, view
+from gtrace.tracer import Context, Scene
+
+pytestmark = pytest.mark.gpu
+
+
+# 148 SMs: below 56 rays an SM the default has a build of its own, lists begin
+# at 160
+@pytest.mark.parametrize("w,h,k,alpha_min", [(64, 64, 6, 0.2), (90, 60, 16, 0.2), (200, 150, 6, 0.01)])
+def test_a_tuned_view_is_no_slower_than_the_default_launch(w, h, k, alpha_min):
+    pg = small_scene(n=16384, seed=7)
+    with Context(0) as c:
+        s = Scene(c, pg.gaussiansBuffer, alpha_min)
+        u = view(w, h, k=k, alpha_min=alpha_min, T_min=0.03).uniforms
+        r = c.autotune(s, u, w, h)
+        assert r["best_ms"] <= r["default_ms"]
+        assert r["block_threads"] == 32 or r["kbuf"] >= k
+        s.close()

@@ -411,9 +411,8 @@ static std::tuple<uint64_t, uint32_t, uint32_t, uint32_t> tune_key(const gt_scen
                          (uint32_t)log2((double)std::max<uint64_t>((uint64_t)w * h, 1)), kmax_for(k), 0u);
 }
 
-// gt_tune_result::_pad of a result that stands for the default launch (over
-// per-view lists where they serve; gt_set_tune takes it back and ignores the
-// other fields).
+// gt_tune_result::_pad of a result that stands for the default launch (gt_set_tune
+// takes it back and ignores the other fields).
 constexpr uint32_t kTuneLists = 0x4C495354u;
 
 // The launch shape a tuning result stands for.
@@ -430,6 +429,25 @@ static LaunchShape shape_of(const gt_tune_result& r) {
   sh.leaf_batch = r.leaf_batch;
   if (r.handoff_after) sh.handoff_after = r.handoff_after;
   return sh;
+}
+
+// The result of a tuning: the fastest explicit shape, marked where the default
+// launch is no slower than that.
+static gt_tune_result tune_result(const LaunchShape& sh, bool is_default, float best_ms, float default_ms,
+                                  uint32_t k) {
+  gt_tune_result r;
+  memset(&r, 0, sizeof r);
+  r.block_threads = sh.packet ? 32u : 128u;
+  r.blocks_per_sm = sh.blocks_per_sm;
+  r.tile_w = 8;
+  r.tile_h = 4;
+  r.best_ms = best_ms;
+  r.default_ms = default_ms;
+  r.kbuf = std::max(sh.packet ? sh.packet_kbuf : sh.kbuf, k);
+  r.leaf_batch = sh.leaf_batch;
+  r.handoff_after = sh.handoff_after;
+  if (is_default) r._pad = kTuneLists;
+  return r;
 }
 
 static LaunchShape shape_for(gt_context* ctx, const gt_scene* s, uint32_t w, uint32_t h, uint32_t k) {
@@ -1145,14 +1163,14 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
     *out_ms = ms_min;
     return GT_OK;
   };
+  // 0. the default launch, whatever it takes (lists, tile packets or a build for few rays)
   const uint32_t k = u->k;
-  LaunchShape best_sh;
+  LaunchShape best_sh;  // the fastest of the others
   float best = 1e30f, def = 0.0f;
   st = time_shape(LaunchShape(), 3, &def);
   if (st != GT_OK) return st;
   float pk_best = 1e30f;
   LaunchShape pk_sh;
-  if (lists.cap) best = def;  // 0. the default: per-view lists
   // 1. tile packets: k-buffer entries per ray, then the hand-off point of
   // the fastest
   const uint32_t pkbufs[] = {k, 24u, 32u, 48u, 64u};
@@ -1227,18 +1245,7 @@ extern "C" gt_status gt_autotune(gt_context* ctx, const gt_scene* scene, const g
     best = warp_best;
     best_sh = warp_sh;
   }
-  gt_tune_result r;
-  memset(&r, 0, sizeof r);
-  if (best_sh.packet == 2) r._pad = kTuneLists;
-  r.block_threads = best_sh.packet ? 32u : 128u;
-  r.blocks_per_sm = best_sh.blocks_per_sm;
-  r.tile_w = 8;
-  r.tile_h = 4;
-  r.best_ms = best;
-  r.default_ms = def;
-  r.kbuf = std::max(best_sh.packet ? best_sh.packet_kbuf : best_sh.kbuf, k);
-  r.leaf_batch = best_sh.leaf_batch;
-  r.handoff_after = best_sh.handoff_after;
+  const gt_tune_result r = tune_result(best_sh, def <= best, std::min(best, def), def, k);
   ctx->tune[tune_key(scene, w, h, k)] = r;
   if (result) *result = r;
   return GT_OK;
