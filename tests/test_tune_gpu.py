@@ -20,3 +20,18 @@ def test_a_tuned_view_is_no_slower_than_the_default_launch(w, h, k, alpha_min):
         assert r["best_ms"] <= r["default_ms"]
         assert r["block_threads"] == 32 or r["kbuf"] >= k
         s.close()
+
+
+def test_a_batch_result_names_the_shape_that_won(ctx):
+    """A small far view, which lists serve: a warp per ray takes half their time
+    and a tenth of the tile packets', and the result says so."""
+    pg = small_scene(n=16384, seed=7)
+    s = Scene(ctx, pg.gaussiansBuffer, 0.01)
+    u = view(160, 150, pos=(0.0, 0.0, 60.0), k=32).uniforms
+    try:
+        r = ctx.autotune_batch([(s, u, 160, 150)])
+        assert r["block_threads"] == 128
+    finally:
+        ctx._lib.gt_autotune_reset(ctx._h)
+        s.close()
+

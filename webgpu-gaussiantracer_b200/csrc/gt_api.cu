@@ -1321,8 +1321,10 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
   if (st != GT_OK) return st;
   st = time_shape(def_sh, 2, &def);
   if (st != GT_OK) return st;
+  // the fastest of the explicit shapes, beside the default launch
+  const bool plain = def_sh.packet == 2;
   LaunchShape best_sh = def_sh;
-  float best = def;
+  float best = plain ? 1e30f : def;
   const uint32_t pkbufs[] = {kmin, 24u, 32u, 48u, 64u};
   const uint32_t hands[] = {2u, 3u, 4u, 6u};
   for (int i = 0; i < 5; ++i) {
@@ -1353,19 +1355,7 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
       best_sh = sh;
     }
   }
-  gt_tune_result r;
-  memset(&r, 0, sizeof r);
-  if (best_sh.packet == 2) r._pad = kTuneLists;
-  const bool pk = lists.cap || packet_launch(ctx->h_views, count, total_tiles, ctx->num_sms, best_sh, false);
-  r.block_threads = pk ? 32u : 128u;
-  r.blocks_per_sm = best_sh.blocks_per_sm;
-  r.tile_w = 8;
-  r.tile_h = 4;
-  r.best_ms = best;
-  r.default_ms = def;
-  r.kbuf = pk ? best_sh.packet_kbuf : best_sh.kbuf;
-  r.leaf_batch = best_sh.leaf_batch;
-  r.handoff_after = best_sh.handoff_after;
+  const gt_tune_result r = tune_result(best_sh, plain && def <= best, std::min(best, def), def, kmin);
   ctx->batch_tune[std::make_tuple(count, total_tiles, kmax)] = r;
   if (result) *result = r;
   return GT_OK;
