@@ -365,14 +365,14 @@ def extra_batched_fwd_bwd(ctx, pg, amin, reps: int = 1, n_views: int = 32):
             "mode": "checkpoint" if info.get("used_mode") == 1 else "replay"}
 
 
-DEFAULT_SHAPE = {"block_threads": 32, "kbuf": 0, "handoff_after": 0, "blocks_per_sm": 8, "best_ms": None,
-                 "default_ms": None}
+DEFAULT_SHAPE = {"default": True, "block_threads": 32, "kbuf": 0, "handoff_after": 0, "blocks_per_sm": 8,
+                 "best_ms": None, "default_ms": None}
 
 
 def shape_label(tune):
-    """The kernels a tuning result stands for.  A default launch shape that won
-    has the tuner's two times equal: the list tracer for the views timed here."""
-    if not tune["kbuf"] or tune["best_ms"] is not None and tune["best_ms"] == tune["default_ms"]:
+    """The kernels a tuning result stands for (the default launch is the list
+    tracer for the views timed here)."""
+    if tune["default"]:
         return {"kernel": "default (proxy lists)"}
     if tune["block_threads"] == 32:
         return {"kernel": "tile packets", "kbuf": tune["kbuf"], "handoff_after": tune["handoff_after"]}
@@ -495,7 +495,7 @@ def main():
         bt = 32 if kind == "packets" else 128
         kb = int(kb) or (32 if bt == 32 else 64)
         ctx.set_tune(scene, v.uniforms, w, h, block_threads=bt, kbuf=kb, handoff_after=int(ha), blocks_per_sm=8)
-        tune = {"block_threads": bt, "kbuf": kb, "handoff_after": int(ha), "blocks_per_sm": 8,
+        tune = {"default": False, "block_threads": bt, "kbuf": kb, "handoff_after": int(ha), "blocks_per_sm": 8,
                 "best_ms": None, "default_ms": None}
     else:
         tune = ctx.autotune(scene, v.uniforms, w, h)

@@ -77,6 +77,7 @@ class TuneResult(C.Structure):
                 ("tile_h", C.c_uint32), ("best_ms", C.c_float), ("default_ms", C.c_float),
                 ("kbuf", C.c_uint32), ("leaf_batch", C.c_uint32), ("handoff_after", C.c_uint32),
                 ("_pad", C.c_uint32)]
+    DEFAULT = 0x4C495354  # _pad of a result that stands for the default launch
 
 
 class BvhInfo(C.Structure):

@@ -39,6 +39,12 @@ def _uniforms(u) -> L.Uniforms:
     return L.Uniforms.from_buffer_copy(b)
 
 
+def _tune_dict(r: L.TuneResult) -> dict:
+    d = {name: getattr(r, name) for name, _ in r._fields_ if not name.startswith("_")}
+    d["default"] = r._pad == r.DEFAULT
+    return d
+
+
 class Context:
     """A CUDA device, its stream and the library state (one per GPU)."""
 
@@ -219,10 +225,13 @@ class Context:
         return loss.value
 
     def autotune(self, scene: "Scene", uniforms, width: int, height: int):
+        """Times the launch shapes on a view and caches the fastest (gt_autotune).
+        ``default`` in the result says that it is the default launch; the other
+        fields are then those of the fastest explicit shape."""
         r = L.TuneResult()
         self.check(self._lib.gt_autotune(self._h, scene.handle, C.byref(_uniforms(uniforms)), width, height,
                                          C.byref(r)))
-        return {name: getattr(r, name) for name, _ in r._fields_ if not name.startswith("_")}
+        return _tune_dict(r)
 
     def autotune_batch(self, views):
         """views: list of (scene, uniforms, width, height) -> the fastest launch
@@ -234,15 +243,19 @@ class Context:
             items[i].w, items[i].h = w, h
         r = L.TuneResult()
         self.check(self._lib.gt_autotune_batch(self._h, items, len(views), C.byref(r)))
-        return {name: getattr(r, name) for name, _ in r._fields_ if not name.startswith("_")}
+        return _tune_dict(r)
 
     def set_tune(self, scene: "Scene", uniforms, width: int, height: int, blocks_per_sm: int = 4,
-                 kbuf: int = 32, leaf_batch: int = 32, block_threads: int = 128, handoff_after: int = 0):
+                 kbuf: int = 32, leaf_batch: int = 32, block_threads: int = 128, handoff_after: int = 0,
+                 default: bool = False):
         """Installs a launch shape for this (scene, k, image size) bucket:
         block_threads 32 traces 8x4 tiles of rays per warp (kbuf entries per
         ray, rays handed to a warp-per-ray launch after handoff_after
-        traversals, 0: the default), 128 one ray per warp (gt_set_tune)."""
-        r = L.TuneResult(block_threads, blocks_per_sm, 8, 4, 0.0, 0.0, kbuf, leaf_batch, handoff_after, 0)
+        traversals, 0: the default), 128 one ray per warp (gt_set_tune).
+        default=True (as in a result of ``autotune``) stands for the default
+        launch, whatever the other values."""
+        r = L.TuneResult(block_threads, blocks_per_sm, 8, 4, 0.0, 0.0, kbuf, leaf_batch, handoff_after,
+                         L.TuneResult.DEFAULT if default else 0)
         self.check(self._lib.gt_set_tune(self._h, scene.handle, C.byref(_uniforms(uniforms)), width, height,
                                          C.byref(r)))
 
