@@ -35,3 +35,17 @@ def test_a_batch_result_names_the_shape_that_won(ctx):
         ctx._lib.gt_autotune_reset(ctx._h)
         s.close()
 
+
+def test_a_batch_tries_the_default_launch_beside_a_cached_shape(ctx):
+    """With tile packets cached for the view, the lists (twice as fast as any
+    other launch here) are still tried, and win."""
+    pg = small_scene(n=16384, seed=7)
+    s = Scene(ctx, pg.gaussiansBuffer, 0.01)
+    w, h = 640, 400
+    u = view(w, h, k=6).uniforms
+    try:
+        ctx.set_tune(s, u, w, h, block_threads=32, kbuf=32)
+        assert ctx.autotune_batch([(s, u, w, h)])["default"]
+    finally:
+        ctx._lib.gt_autotune_reset(ctx._h)
+        s.close()

@@ -1321,10 +1321,17 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
   if (st != GT_OK) return st;
   st = time_shape(def_sh, 2, &def);
   if (st != GT_OK) return st;
-  // the fastest of the explicit shapes, beside the default launch
-  const bool plain = def_sh.packet == 2;
-  LaunchShape best_sh = def_sh;
-  float best = plain ? 1e30f : def;
+  // the default launch, and the fastest of the explicit shapes (the per-view
+  // result, where there is one, among them)
+  float plain = def;
+  LaunchShape best_sh;
+  float best = 1e30f;
+  if (def_sh.packet != 2) {
+    best_sh = def_sh;
+    best = def;
+    st = time_shape(LaunchShape(), 3, &plain);
+    if (st != GT_OK) return st;
+  }
   const uint32_t pkbufs[] = {kmin, 24u, 32u, 48u, 64u};
   const uint32_t hands[] = {2u, 3u, 4u, 6u};
   for (int i = 0; i < 5; ++i) {
@@ -1355,7 +1362,7 @@ extern "C" gt_status gt_autotune_batch(gt_context* ctx, const gt_batch_item* ite
       best_sh = sh;
     }
   }
-  const gt_tune_result r = tune_result(best_sh, plain && def <= best, std::min(best, def), def, kmin);
+  const gt_tune_result r = tune_result(best_sh, plain <= best, std::min(best, plain), def, kmin);
   ctx->batch_tune[std::make_tuple(count, total_tiles, kmax)] = r;
   if (result) *result = r;
   return GT_OK;
