@@ -279,6 +279,7 @@ struct ListView {
   double X[3], Y[3], Z[3];  // camera frame: right, up, view direction
   double sx, sy, ox, oy;    // pixel x = u sx + ox
   double inv_bw, inv_bh;    // 1 / bin size in pixels
+  double reach;             // 1 + largest |u| + largest |v|
   float Xf[3], Yf[3], Zf[3];
   uint32_t bins_x, bins_y;  // bins that cover the image
   uint32_t bin_begin, rec_begin;
