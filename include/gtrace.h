@@ -402,7 +402,9 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  * bucket, k).  gt_render and gt_render_batch use the cached choice.
  * Three ways render the plain image (debugMode 0), with identical results.
  * The default for views of at least 160 rays per SM (23,680 on a 148-SM B200;
- * with k of 4 or more, one more for every 14,000 proxies):
+ * with k of 4 or more, one more for every 14,000 proxies; rays outside the
+ * image of the scene's box do not count where it has 4,096 proxies or more,
+ * unless there are 200,000 rays and six more for every proxy):
  * per-view lists of the proxies that each bin of 16x8 or 32x16 pixels may show,
  * ordered by distance, which the bin's tiles stream through.  They serve
  * unsheared cameras with t_min >= 0 and the limits of gt_set_limits at their
@@ -417,8 +419,8 @@ gt_status gt_l2_loss(gt_context* ctx, const float* rgba, const float* target, ui
  *                      traversal (k..128, default 64), blocks_per_sm and
  *                      leaf_batch as below.
  * Without a cached shape and without lists a launch takes the first of these
- * when it has at least 48 8x4 tiles per SM (about 0.23 Mpixels on a 148-SM
- * B200) and the second otherwise: tiles are coarse work items, and with few of
+ * when it has at least 48 8x4 tiles per SM within the image of the scene's box
+ * (about 0.23 Mpixels on a 148-SM B200) and the second otherwise: tiles are coarse work items, and with few of
  * them per warp the slowest ones decide the time.  The rays of a tile packet
  * that still need hits after three traversals (or after the current one, once
  * every tile of the launch is taken) are finished by the second one (a second

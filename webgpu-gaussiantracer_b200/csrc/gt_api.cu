@@ -264,14 +264,15 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
                               const LaunchShape& shape, Lists* out, Handoff* hand) {
   *out = Lists{};
   if (shape.packet != 2 || !stream_views(views, n, total_tiles, ctx->faces)) return GT_OK;
-  uint64_t recs = 0;
+  uint64_t recs = 0, met = 0;
   uint32_t k_min = 32;
   for (uint32_t i = 0; i < n; ++i) {
     views[i].rec_begin = (uint32_t)recs;
     recs += views[i].s.n_kept;
+    met += views[i].met;
     k_min = std::min(k_min, views[i].u.k);
   }
-  const StreamPlan plan = stream_plan(rays, recs, k_min, ctx->num_sms);
+  const StreamPlan plan = stream_plan(rays, met, recs, k_min, ctx->num_sms);
   if (plan.rays == 0) return GT_OK;
   const uint64_t bins = total_tiles >> plan.shift;
   constexpr uint64_t kRec = 3 * sizeof(float4) + sizeof(float), kEnt = sizeof(float4) + sizeof(uint2);
@@ -376,6 +377,7 @@ static ViewDev make_view(const gt_scene* s, const gt_uniforms& u, uint32_t w, ui
   v.n_tiles = v.tiles_x * (((h + 3) / 4 + 15) / 16 * 16);
   v.tile_begin = tile_begin;
   v.n_particles = s->n;
+  v.met = s->b.n_kept ? pixels_of_box(v.u, w, h, s->b.bounds) : 0;
   v.kbuf = 32;
   v.leaf_batch = 32;
   return v;

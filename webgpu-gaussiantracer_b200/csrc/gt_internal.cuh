@@ -131,6 +131,7 @@ struct ViewDev {
   float4* grad_sh;      // backward: this view's per-particle sums of the colour weights (1 float4 a particle)
   uint64_t n_particles;
   uint32_t rec_begin;   // first projection record of this view (gt_stream.cu)
+  uint32_t met;         // pixels of the scene's box, by which the kernels are chosen
   // this view's colour of every particle, max(0, SH(normalize(mu - camera)))
   // per channel (k_view_colours, before the trace launch), or null: the
   // trace kernels evaluate the SH per composited entry
@@ -319,13 +320,16 @@ Err launch_trace(ViewDev* views, uint32_t n_views, uint32_t total_tiles, DevCoun
                  const FaceTable& faces, const LaunchShape& shape, int num_sms, cudaStream_t stream,
                  uint64_t* launches, ViewDev* d_views_scratch, const Ckpt* ckpt = nullptr,
                  const Handoff* handoff = nullptr, const Lists* lists = nullptr);
+// Pixels of a w x h view inside the image rectangle of a box (lo, hi): all of them
+// where the box reaches the camera plane.
+uint32_t pixels_of_box(const RayUniforms& u, uint32_t w, uint32_t h, const float* box);
 // Whether per-view lists can serve these views (gt_stream.cu).
 bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, const FaceTable& faces);
 struct StreamPlan {
   uint32_t rays = 0;   // rays per warp (0: the hierarchy kernels are faster)
   uint32_t shift = 4;  // bins of 2^shift tiles
 };
-StreamPlan stream_plan(uint64_t rays, uint64_t proxies, uint32_t k_min, int num_sms);
+StreamPlan stream_plan(uint64_t rays, uint64_t met, uint64_t proxies, uint32_t k_min, int num_sms);
 Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n_views, uint32_t total_tiles,
                         DevCounters* counters, const FaceTable& faces, int num_sms, cudaStream_t stream,
                         uint64_t* launches, const Lists& lists, const Handoff& handoff, const Ckpt* ckpt);

@@ -1136,6 +1136,36 @@ static Err launch_stream_r(const ViewDev* d_views, uint32_t n_views, uint32_t to
   return Err{};
 }
 
+uint32_t pixels_of_box(const RayUniforms& u, uint32_t w, uint32_t h, const float* box) {
+  double axis[3][3], len[3];  // right, up, view direction
+  for (int r = 0; r < 3; ++r) {
+    len[r] = 0.0;
+    for (int q = 0; q < 3; ++q) {
+      axis[r][q] = (r == 1 ? 1.0 : -1.0) * (double)u.tw[4 * r + q];
+      len[r] += axis[r][q] * axis[r][q];
+    }
+    len[r] = sqrt(len[r]);
+  }
+  // x and y in half images from the centre, as ray_gen places the pixels
+  double lo[2] = {1.0, 1.0}, hi[2] = {-1.0, -1.0};
+  for (int c = 0; c < 8; ++c) {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int q = 0; q < 3; ++q) {
+      const double p = (double)box[(c >> q & 1) * 3 + q] - (double)u.tw[12 + q];
+      for (int r = 0; r < 3; ++r) v[r] += axis[r][q] * p;
+    }
+    if (!(v[2] > 1e-3 * len[2] * (fabs(v[0]) / len[0] + fabs(v[1]) / len[1]))) return w * h;
+    for (int a = 0; a < 2; ++a) {
+      const double x = v[a] / len[a] / (v[2] / len[2]) * len[2] / (len[a] * (double)u.asp[a]);
+      if (!(fabs(x) < 1e30)) return w * h;
+      lo[a] = std::min(lo[a], std::max(-1.0, x));
+      hi[a] = std::max(hi[a], std::min(1.0, x));
+    }
+  }
+  const double part = std::max(0.0, hi[0] - lo[0]) * std::max(0.0, hi[1] - lo[1]) / 4.0;
+  return (uint32_t)(part * (double)w * (double)h + 0.5);
+}
+
 bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, const FaceTable& faces) {
   if (n_views == 0 || n_views > 65535u || (uint64_t)total_tiles * 32u > kStreamMaxSlots) return false;
   // lowered limits (gt_set_limits) act on the hierarchy's loops
@@ -1189,11 +1219,23 @@ bool stream_views(const ViewDev* views, uint32_t n_views, uint32_t total_tiles, 
 //   220x160 (238 an SM): 700k k 8 604 / 568, 1M k 8 1084 / 971, k 16 1407 / 1159),
 // unless rounds are so short that a ray per warp pays for each (1M k 1, 200x150:
 // 1852 / 1356).
-StreamPlan stream_plan(uint64_t rays, uint64_t proxies, uint32_t k_min, int num_sms) {
+// The rays that count are those that may meet the scene (`met`, pixels_of_box):
+// a far scene fills few tiles, whose warps go through long lists while the others
+// are idle (lists of a few thousand proxies are short: 400 that fill a sixth of
+// 180x140, 846 / 583; warp per ray / lists, us):
+//   481x271, radius 60:  200k k 8 401 / 609, 1M k 16 822 / 2206; radius 300: 1M
+//   626 / 12920; 200x150: uniform 65k k 6 radius 12 288 / 349, radius 30 246 / 461.
+// A warp for each of many rays that meet nothing costs more (2M rays 1.9 ms) than
+// the lists of a few proxies (radius 100, k 6, 960x540: 16k 542 / 288, 65k
+// 562 / 567; 1080p: 16k 1872 / 363, 65k 1943 / 538; radius 300, 960x540: 200k
+// 636 / 1093, 1M 769 / 5570; 1080p: 200k 1881 / 740, 1M 1984 / 2355).
+StreamPlan stream_plan(uint64_t rays, uint64_t met, uint64_t proxies, uint32_t k_min, int num_sms) {
   StreamPlan p;
-  const uint64_t per_sm = rays / (uint64_t)std::max(1, num_sms);
-  if (per_sm >= 160 + (k_min >= 4 ? proxies / 14000 : 0)) {
-    p.rays = per_sm < 640 ? 8 : 32;
+  const uint64_t sms = (uint64_t)std::max(1, num_sms);
+  if (proxies < 4096) met = rays;
+  const bool near = met / sms >= 160 + (k_min >= 4 ? proxies / 14000 : 0);
+  if (near || rays >= 200000 + 6 * proxies) {
+    p.rays = (near ? met : rays) / sms < 640 ? 8 : 32;
     p.shift = p.rays == 8 ? 2u : 4u;
   }
   return p;

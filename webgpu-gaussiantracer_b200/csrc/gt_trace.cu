@@ -394,7 +394,15 @@ bool packet_launch(const ViewDev* views, uint32_t n_views, uint32_t total_tiles,
   for (uint32_t i = 0; i < n_views; ++i)
     if (views[i].u.debug != 0) return false;
   if (shape.packet == 1) return true;
-  return (uint64_t)total_tiles >= (uint64_t)kPacketTilesPerSm * (uint64_t)std::max(1, num_sms);
+  // (the tiles of a far scene's part of the image: 960x540, radius 300, 1M
+  // Gaussians 16.2 ms as packets, 0.77 as a warp per ray)
+  uint64_t met = 0, rays = 0;
+  for (uint32_t i = 0; i < n_views; ++i) {
+    met += views[i].met;
+    rays += (uint64_t)views[i].w * views[i].h;
+  }
+  const uint64_t tiles = met < rays ? (uint64_t)((double)total_tiles * (double)met / (double)rays) : total_tiles;
+  return tiles >= (uint64_t)kPacketTilesPerSm * (uint64_t)std::max(1, num_sms);
 }
 
 // Launches whose rays go a warp each from the start, by default: 96 registers
