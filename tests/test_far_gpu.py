@@ -31,3 +31,22 @@ def test_far_scenes(ctx, distance, lists, w, h, target):
     assert np.array_equal(_bits(img), oracle.Scene(pg.gaussiansBuffer, 0.01, "f32").render(u, w, h)[0].view(np.uint32))
     same = (st["node_visits"], st["proxy_tests"]) == (warp["node_visits"], warp["proxy_tests"])
     assert same != lists  # (the warp-per-ray kernel's own counts)
+
+
+# (16 quarter tiles of 8 rays, 16 tiles of 32: those of the four bins in the middle)
+@pytest.mark.parametrize("w,h,rays", [(230, 170, 128), (400, 300, 512)])
+def test_far_scene_with_outliers(ctx, w, h, rays):
+    """Eight proxies far out stretch the scene's box over the image, so lists
+    serve; the few tiles that show the rest, or lie beside it, hand their rays
+    over instead of going through lists of 30,000 proxies while all others are
+    idle."""
+    rec = small_scene(n=30000, seed=8).gaussiansBuffer.copy().reshape(-1, 80)
+    for i in range(8):
+        rec[i, 0:3] = [1e3 * (1 if i >> a & 1 else -1) for a in range(3)]
+        rec[i, 12] = 0.9
+    s = Scene(ctx, rec, 0.01)
+    u = view(w, h, pos=(0.0, 0.0, 150.0), k=6).uniforms
+    img, st = ctx.render(s, u, w, h, stats=True)
+    s.close()
+    assert np.array_equal(_bits(img), oracle.Scene(rec, 0.01, "f32").render(u, w, h)[0].view(np.uint32))
+    assert 0.75 * rays <= st["handed"] <= 2 * rays

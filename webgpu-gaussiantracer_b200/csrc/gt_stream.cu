@@ -544,6 +544,11 @@ __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bi
 constexpr int kStreamKb = 32;
 constexpr int kStreamHot = 24;
 constexpr uint32_t kStreamStep = 10;
+// Chunks of a list after which a tile looks whether every tile is taken (481x271 of
+// 1M Gaussians from radius 300 with a few proxies far out, so that their box fills
+// the image: 13.5 ms without, 1.57 / 1.62 / 1.71 at 32 / 64 / 128; 1080p of the
+// scene alone 9.31 -> 9.33).
+constexpr uint32_t kStreamLook = 32;
 
 template <int R>
 struct StreamScratch {
@@ -1054,7 +1059,14 @@ __global__ void __launch_bounds__(32, 16) k_trace_stream(const ViewDev* __restri
           nbx = __ldg(L.ent_box + pos + lane);
           nen = __ldg(L.ent + pos + lane);
         }
-        ++scanned;
+        // a tile that goes through a long list without many hits looks up now and
+        // then whether the others are done (it then hands its rays over, above)
+        if ((++scanned & (kStreamLook - 1)) == 0 && hand.rays) {
+          uint32_t taken = 0;
+          if (lane == 0) taken = *reinterpret_cast<volatile const uint32_t*>(&ctr->work);
+          hot = __shfl_sync(kFull, taken, 0) >= total + hand.late;
+          if (hot) break;
+        }
       }
       __syncwarp();
       sv_i = 0;
