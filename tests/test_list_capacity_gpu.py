@@ -1,9 +1,10 @@
 """Room for the per-view proxy lists (gt_stream.cu, gt_api.cu): lists whose
-lengths pass 2^32 together.  The hierarchy kernels' image of the same view is
+lengths pass 2^32 together, and buffers that grow to what launches needed.  The hierarchy kernels' image of the same view is
 the reference (bit-equal to the oracle, test_parity_gpu.py, test_packet_gpu.py)."""
 import numpy as np
 import pytest
 
+from conftest import view
 from gtrace.tracer import Context, Scene
 from gtrace.uniforms import look_at, pack_uniforms
 
@@ -39,3 +40,42 @@ def test_more_list_entries_than_32_bits_count():
     assert (ref[..., :3].max(axis=-1) > 0).mean() > 0.5
     for img in got:
         assert np.array_equal(_bits(img), _bits(ref))
+
+
+W, H = 320, 200
+
+
+def _wide_proxies(n):
+    """Proxies that each cover the whole image, one behind another, and the view
+    that shows them: a ray ends at the third or fourth."""
+    rng = np.random.default_rng(92)
+    rec = np.zeros((n, 80), np.float32)
+    rec[:, 0:2] = 0.3 * rng.normal(size=(n, 2))
+    rec[:, 2] = -np.linspace(50.0, 500.0, n)
+    rec[:, 4:7] = 4.0
+    rec[:, 8] = 1.0
+    rec[:, 12] = 0.9
+    rec[:, 16:19] = rng.normal(size=(n, 3))
+    return rec, view(W, H, pos=(0.0, 0.0, 0.0), target=(0.0, 0.0, -1.0), k=4, T_min=0.01, hfov=1.5).uniforms
+
+
+# 3,500 proxies in 500 bins: 1.75 million entries, room for 1.4 million at
+# first: the rays of more than 80 bins (128 each) go to the warp-per-ray kernel,
+# and once all fit, those at the launch's end
+@pytest.mark.parametrize("how", ["another view between", "queued"])
+def test_a_need_is_kept_and_told_without_waiting(how):
+    rec, u = _wide_proxies(3500)
+    small = view(64, 48, pos=(0.0, 0.0, 0.0), target=(0.0, 0.0, -1.0), k=4, hfov=1.5).uniforms
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        out = c.device_alloc(W * H * 16)
+        if how == "queued":
+            for _ in range(2):
+                c.render_device(s, u, W, H, out, asynchronous=True)
+            c.synchronize()
+        else:
+            assert c.render_device(s, u, W, H, out)["handed"] > 10_000
+            c.render_device(s, small, 64, 48, out)
+        assert c.render_device(s, u, W, H, out)["handed"] < 4_000
+        c.device_free(out)
+        s.close()

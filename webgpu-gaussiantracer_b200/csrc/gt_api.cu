@@ -254,9 +254,10 @@ static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n, boo
 // Buffers of the per-view proxy lists (gt_stream.cu) for a launch of these
 // views, grown as needed and kept by the context (at most kListBudget bytes).
 // Entries: 25 per proxy and view to begin with (a proxy meets 2 to 4 bins of a
-// 1080p view of the 1M-Gaussian scene), more once a call that was waited for
-// has reported a larger need; the tiles of bins whose lists do not fit are
-// traced by the warp-per-ray kernel.  Views the lists cannot serve, and
+// 1080p view of the 1M-Gaussian scene), more once a launch that did not have
+// room has left its need in Lists::need (it is read here without waiting, so
+// queued launches count too, and the largest is kept, so views may take turns);
+// the tiles of bins whose lists do not fit are traced by the warp-per-ray kernel.  Views the lists cannot serve, and
 // launches whose projection records or bins alone would take half the
 // budget, get none (the hierarchy kernels trace them).
 constexpr uint64_t kListBudget = 8ull << 30;
@@ -284,6 +285,8 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
   const uint64_t fixed = spare(recs) * kRec + spare(bins) * kBin;
   if (fixed > kListBudget / 2 || recs >= (1ull << 31)) return GT_OK;
   const uint64_t most = std::min<uint64_t>((kListBudget - fixed) / kEnt, 1ull << 30);
+  const uint32_t told = *reinterpret_cast<volatile uint32_t*>(ctx->lists.need);
+  ctx->lists_need = std::max(ctx->lists_need, told);
   const uint64_t need = std::max<uint64_t>(recs * 20 + (1u << 20), ctx->lists_need);
   const uint64_t want = std::min<uint64_t>(need + need / 4, most);
   Lists& L = ctx->lists;
@@ -516,6 +519,8 @@ extern "C" gt_status gt_context_create(int device, gt_context** out) {
   }
   CTX_TRY(cudaMalloc(&ctx->d_ctr, sizeof(DevCounters)));
   CTX_TRY(cudaHostAlloc((void**)&ctx->h_ctr, sizeof(DevCounters), cudaHostAllocDefault));
+  CTX_TRY(cudaHostAlloc((void**)&ctx->lists.need, sizeof(uint32_t), cudaHostAllocDefault));
+  *ctx->lists.need = 0;
   CTX_TRY(cudaEventCreate(&ctx->call0));
   CTX_TRY(cudaEventCreate(&ctx->call1));
   CTX_TRY(cudaEventCreate(&ctx->timer0));
@@ -547,6 +552,7 @@ extern "C" gt_status gt_context_destroy(gt_context* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);  // the frees are stream-ordered
   cudaFree(ctx->d_ctr);
   cudaFreeHost(ctx->h_ctr);
+  cudaFreeHost(ctx->lists.need);
   cudaFree(ctx->d_views);
   cudaFree(ctx->d_handoff);
   cudaFreeHost(ctx->h_views);
@@ -776,7 +782,6 @@ static gt_status finish_call(gt_context* ctx, gt_render_stats* stats, uint64_t k
   API_CUDA(ctx, cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
   API_CUDA(ctx, cudaEventRecord(ctx->call1, ctx->stream));
   API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->lists_need = ctx->h_ctr->list_pairs;
   if (stats) {
     memset(stats, 0, sizeof *stats);
     fill_stats(*ctx->h_ctr, stats);

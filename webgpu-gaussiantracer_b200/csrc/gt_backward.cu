@@ -794,7 +794,6 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     CK_TRY(cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
     CK_TRY(cudaStreamSynchronize(st));
     cudaEventElapsedTime(&ck.fwd_ms, ctx->int0, ctx->int1);
-    ctx->lists_need = ctx->h_ctr->list_pairs;
     sst = api_status_to_error(ctx, ctx->h_ctr->status);
     if (sst != GT_OK) return sst;
     if (stats) {

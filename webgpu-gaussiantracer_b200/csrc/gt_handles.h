@@ -71,7 +71,7 @@ struct gt_context {
   gt::Lists lists;                      // per-view proxy lists (gt_stream.cu)
   uint32_t lists_views = 0;             // capacities: views, projection records, bins, redo slots
   uint64_t lists_recs = 0, lists_bins = 0, redo_cap = 0;
-  uint32_t lists_need = 0;              // entries the last list launch that was waited for needed
+  uint32_t lists_need = 0;              // the most entries a launch needed without having room for them
   uint32_t* d_redo = nullptr;
   cudaEvent_t call0 = nullptr, call1 = nullptr, timer0 = nullptr, timer1 = nullptr;
   cudaEvent_t int0 = nullptr, int1 = nullptr;  // library-internal timing (never the user's timer)

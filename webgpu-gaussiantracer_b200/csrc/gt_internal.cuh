@@ -68,7 +68,6 @@ struct DevCounters {
   unsigned int work2;    // the same for the second kernel of a launch
   unsigned int handoff;  // rays the tile kernels handed to the warp-per-ray kernel
   unsigned int redo;       // rays that kernel traces from the start
-  unsigned int list_pairs; // list entries the launch needed, at most 2^31 - 1 (gt_stream.cu)
 };
 
 // Scene as the kernels see it.  Records of kept proxies are in BVH leaf
@@ -298,6 +297,7 @@ struct Lists {
   uint2* ent = nullptr;          // proxy, bits of its bucket's lower bound
   unsigned long long* spill = nullptr;  // waiting hits past a ray's column in shared memory
   uint64_t spill_bytes = 0;
+  uint32_t* need = nullptr;      // page-locked: entries a launch needed that had no room for them
   uint32_t cap = 0;              // entries that fit
   uint32_t shift = 4;            // tiles per bin: 2^shift
   uint32_t rays = 32;            // rays per warp

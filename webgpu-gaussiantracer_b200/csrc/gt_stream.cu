@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(128) k_list_rows(const Lists L) {
 constexpr uint32_t kListFull = 0x7FFFFFFFu;
 __device__ __forceinline__ uint32_t list_add(uint32_t a, uint32_t b) { return min(a + b, kListFull); }
 
-__global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bins, DevCounters* ctr) {
+__global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bins) {
   __shared__ uint32_t ws[32];
   __shared__ uint32_t carry;
   __shared__ uint32_t place[33];  // bins per class, then their first places
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(1024) k_list_bins(const Lists L, uint32_t n_bi
   }
   if (threadIdx.x == 0) {
     L.bin_base[n_bins] = carry;
-    atomicMax(&ctr->list_pairs, carry);
+    if (carry > L.cap) *reinterpret_cast<volatile uint32_t*>(L.need) = carry;
     uint32_t at = 0;
     for (int c = 0; c < 33; ++c) {
       const uint32_t k = place[c];
@@ -1268,7 +1268,7 @@ Err launch_trace_stream(const ViewDev* views, const ViewDev* d_views, uint32_t n
                        n_views);
   k_list_pass<false><<<pass_grid, kPassBlock, 0, stream>>>(d_views, L.views, faces.r_circ, per_warp, L);
   k_list_rows<<<n_bins, 128, 0, stream>>>(L);
-  k_list_bins<<<1, 1024, 0, stream>>>(L, n_bins, counters);
+  k_list_bins<<<1, 1024, 0, stream>>>(L, n_bins);
   k_list_pass<true><<<pass_grid, kPassBlock, 0, stream>>>(d_views, L.views, faces.r_circ, per_warp, L);
   *launches += 6;
   GT_CUDA_TRY(cudaGetLastError());
