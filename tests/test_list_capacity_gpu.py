@@ -79,3 +79,22 @@ def test_a_need_is_kept_and_told_without_waiting(how):
         assert c.render_device(s, u, W, H, out)["handed"] < 4_000
         c.device_free(out)
         s.close()
+
+
+def test_every_ray_is_handed_over_once():
+    """Thousands of faint proxies about one place: more rays give up their
+    waiting hits than the hand-over buffer takes (a quarter of them)."""
+    rng = np.random.default_rng(93)
+    n = 3500
+    d = rng.normal(size=(n, 3))
+    rec = np.zeros((n, 80), np.float32)
+    rec[:, 0:3] = 3.0 * d / np.linalg.norm(d, axis=1, keepdims=True) + (0.0, 0.0, -3.0)
+    rec[:, 4:7] = 4.0
+    rec[:, 8] = 1.0
+    rec[:, 12] = 0.02
+    u = view(W, H, pos=(0.0, 0.0, 30.0), k=16, T_min=0.01, hfov=3.0).uniforms
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        st = c.render(s, u, W, H, stats=True)[1]
+        s.close()
+    assert W * H // 4 < st["handed"] <= W * H == st["rays"]

@@ -398,7 +398,7 @@ ViewDev api_make_view(const gt_scene* s, const gt_uniforms& u, uint32_t w, uint3
 
 static uint64_t ring_slot(gt_context* ctx) { return (ctx->ring_head++) % kEventRing; }
 
-static void fill_stats(const DevCounters& c, gt_render_stats* st) {
+static void fill_stats(const gt_context* ctx, const DevCounters& c, gt_render_stats* st) {
   st->rays = c.rays;
   st->rounds = c.rounds;
   st->entries = c.entries;
@@ -407,7 +407,8 @@ static void fill_stats(const DevCounters& c, gt_render_stats* st) {
   st->node_visits = c.node_visits;
   st->anyhits = c.anyhits;
   st->status_flags = c.status;
-  st->handed = c.handoff + c.redo;
+  // (rays past the buffer are counted in `handoff` too, and go on elsewhere)
+  st->handed = std::min(c.handoff, ctx->handoff_cap) + c.redo;
 }
 
 static std::tuple<uint64_t, uint32_t, uint32_t, uint32_t> tune_key(const gt_scene* s, uint32_t w, uint32_t h,
@@ -471,7 +472,7 @@ LaunchShape api_batch_shape_for(gt_context* ctx, const gt_scene* const* scenes, 
   auto bt = ctx->batch_tune.find(std::make_tuple(count, total_tiles, kmax));
   return bt != ctx->batch_tune.end() ? shape_of(bt->second) : shape_for(ctx, scenes[0], ws[0], hs[0], us[0].k);
 }
-void api_fill_stats(const DevCounters& c, gt_render_stats* st) { fill_stats(c, st); }
+void api_fill_stats(const gt_context* ctx, const DevCounters& c, gt_render_stats* st) { fill_stats(ctx, c, st); }
 gt_status api_ensure_views(gt_context* ctx, uint32_t n) { return ensure_views(ctx, n); }
 gt_status api_ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out) { return ensure_handoff(ctx, rays, out); }
 gt_status api_ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
@@ -784,7 +785,7 @@ static gt_status finish_call(gt_context* ctx, gt_render_stats* stats, uint64_t k
   API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (stats) {
     memset(stats, 0, sizeof *stats);
-    fill_stats(*ctx->h_ctr, stats);
+    fill_stats(ctx, *ctx->h_ctr, stats);
     cudaEventElapsedTime(&stats->kernel_ms, ctx->ring[2 * kslot], ctx->ring[2 * kslot + 1]);
     cudaEventElapsedTime(&stats->total_ms, ctx->call0, ctx->call1);
   }

@@ -798,7 +798,7 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     if (sst != GT_OK) return sst;
     if (stats) {
       memset(stats, 0, sizeof *stats);
-      api_fill_stats(*ctx->h_ctr, stats);
+      api_fill_stats(ctx, *ctx->h_ctr, stats);
       stats->kernel_ms = ck.fwd_ms;
       stats->total_ms = ck.fwd_ms;
     }
@@ -1063,7 +1063,7 @@ gt_status backward_impl(gt_context* ctx, const BwdView* views, uint32_t count, c
   sst = api_status_to_error(ctx, ctx->h_ctr->status);
   if (stats) {
     memset(stats, 0, sizeof *stats);
-    api_fill_stats(*ctx->h_ctr, stats);
+    api_fill_stats(ctx, *ctx->h_ctr, stats);
     stats->kernel_ms = bwd_ms;
     stats->total_ms = fwd_ms + bwd_ms;
   }

@@ -114,7 +114,7 @@ LaunchShape api_batch_shape_for(gt_context* ctx, const gt_scene* const* scenes, 
 // returns; the download has arrived once the stream is waited for.
 gt_status api_upload(gt_context* ctx, void* dev, const void* host, size_t bytes);
 gt_status api_download(gt_context* ctx, void* host, const void* dev, size_t bytes);
-void api_fill_stats(const DevCounters& c, gt_render_stats* st);
+void api_fill_stats(const gt_context* ctx, const DevCounters& c, gt_render_stats* st);
 gt_status api_ensure_views(gt_context* ctx, uint32_t n);
 gt_status api_ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out);
 // Proxy lists for a launch of these views (shape.packet == 2 and views the

@@ -115,7 +115,7 @@ extern "C" gt_status gt_render_batch_noalloc(gt_context* ctx, const gt_batch_ite
   if (e != cudaSuccess) return api_fail(ctx, GT_ERR_CUDA, cudaGetErrorString(e));
   if (stats) {
     memset(stats, 0, sizeof *stats);
-    api_fill_stats(*ctx->h_ctr, stats);
+    api_fill_stats(ctx, *ctx->h_ctr, stats);
     cudaEventElapsedTime(&stats->kernel_ms, ctx->int0, ctx->int1);
     cudaEventElapsedTime(&stats->total_ms, ctx->call0, ctx->call1);
   }
