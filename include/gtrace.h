@@ -140,9 +140,9 @@ uint32_t gt_version(void);
 /* Creates a context on CUDA device `device`.  Replaces the adapter/device
  * request of src/main.ts:396-427.  Besides its scenes, a context keeps the
  * scratch of its largest call so far: staging images, the hand-off buffer,
- * checkpoints, the proxy lists of views they serve (52 bytes a proxy and view,
+ * checkpoints, the proxy lists of views they serve (48 bytes a proxy and view,
  * 24 bytes a list entry, 25 entries a proxy to begin with, 57 MB of waiting
- * hits; at most 8 GiB in all), and the colour tables of plain renders (16
+ * hits; at most 8 GiB for one launch), and the colour tables of plain renders (16
  * bytes per particle per view of a call, at most 2 GiB; each particle's SH
  * colour as seen from the view's camera, computed once per call before
  * tracing; renders of few rays evaluate the colours of their entries instead).

@@ -276,7 +276,7 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
   const StreamPlan plan = stream_plan(rays, met, recs, k_min, ctx->num_sms);
   if (plan.rays == 0) return GT_OK;
   const uint64_t bins = total_tiles >> plan.shift;
-  constexpr uint64_t kRec = 3 * sizeof(float4) + sizeof(float), kEnt = sizeof(float4) + sizeof(uint2);
+  constexpr uint64_t kRec = 3 * sizeof(float4), kEnt = sizeof(float4) + sizeof(uint2);
   constexpr uint64_t kBin = (4ull << kListBucketBits) + 8;
   // Everything grows with room to spare, so that a scene with a few more proxies
   // or a view with a few more entries than the last does not allocate again
@@ -312,7 +312,6 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
       const uint64_t c = spare(recs);
       e = grow(&L.rec, 2 * c);
       if (e == cudaSuccess) e = grow(&L.box, c);
-      if (e == cudaSuccess) e = grow(&L.far, c);
       if (e == cudaSuccess) ctx->lists_recs = c;
     }
     if (e == cudaSuccess && bins > ctx->lists_bins) {
@@ -559,7 +558,7 @@ extern "C" gt_status gt_context_destroy(gt_context* ctx) {
   cudaFreeHost(ctx->h_views);
   cudaFree(ctx->staging);
   cudaFree(ctx->colours);
-  for (void* p : {(void*)ctx->lists.views, (void*)ctx->lists.rec, (void*)ctx->lists.box, (void*)ctx->lists.far, (void*)ctx->lists.range,
+  for (void* p : {(void*)ctx->lists.views, (void*)ctx->lists.rec, (void*)ctx->lists.box, (void*)ctx->lists.range,
                   (void*)ctx->lists.cells, (void*)ctx->lists.bin_base, (void*)ctx->lists.order, (void*)ctx->lists.ent_box,
                   (void*)ctx->lists.ent, (void*)ctx->lists.spill, (void*)ctx->d_redo})
     cudaFree(p);

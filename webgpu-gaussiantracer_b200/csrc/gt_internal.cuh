@@ -288,7 +288,6 @@ struct Lists {
   ListView* views = nullptr;
   float4* rec = nullptr;         // 2 per (view, proxy): (u0, v0, slope, g11), (g22, bound, bins x, bins y)
   float4* box = nullptr;         // outline rectangle (u lo, u hi, v lo, v hi)
-  float* far = nullptr;          // per (view, proxy): no point of it is farther from the camera
   uint32_t* range = nullptr;     // per view: bits of the smallest and largest bound
   uint32_t* cells = nullptr;     // per bin 2^kListBucketBits counts, then places
   uint32_t* bin_base = nullptr;  // start of each bin's list (one more than bins)
