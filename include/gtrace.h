@@ -141,12 +141,15 @@ uint32_t gt_version(void);
  * request of src/main.ts:396-427.  Besides its scenes, a context keeps the
  * scratch of its largest call so far: staging images, the hand-off buffer,
  * checkpoints, the proxy lists of views they serve (48 bytes a proxy and view,
- * 24 bytes a list entry, 25 entries a proxy to begin with, 57 MB of waiting
- * hits; at most 8 GiB for one launch), and the colour tables of plain renders (16
+ * 4 KB a bin, 24 bytes a list entry, 25 entries a proxy to begin with, 57 MB of
+ * waiting hits, 4 bytes a ray; records and bins take at most 4 GiB and all lists at
+ * most 8 GiB of one launch, and each of these buffers is kept at its largest), and
+ * the colour tables of plain renders (16
  * bytes per particle per view of a call, at most 2 GiB; each particle's SH
  * colour as seen from the view's camera, computed once per call before
  * tracing; renders of few rays evaluate the colours of their entries instead).
- * Where a buffer does not fit, the call runs without it, with the same result. */
+ * Where lists or colour tables do not fit, the call runs without them, with the
+ * same result. */
 gt_status gt_context_create(int device, gt_context** out);
 /* Destroys the context and every scene still alive on it (their handles
  * become invalid). */

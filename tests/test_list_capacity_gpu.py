@@ -4,7 +4,7 @@ the reference (bit-equal to the oracle, test_parity_gpu.py, test_packet_gpu.py).
 import numpy as np
 import pytest
 
-from conftest import view
+from conftest import small_scene, view
 from gtrace.tracer import Context, Scene
 from gtrace.uniforms import look_at, pack_uniforms
 
@@ -98,3 +98,40 @@ def test_every_ray_is_handed_over_once():
         st = c.render(s, u, W, H, stats=True)[1]
         s.close()
     assert W * H // 4 < st["handed"] <= W * H == st["rays"]
+
+
+def test_lists_that_cannot_be_had():
+    """A batch whose lists need more memory than the GPU has left renders
+    without them, and replays its graph instead of asking again each time; once
+    memory is freed it has them."""
+    import torch
+    rec = small_scene(n=60_000, seed=94).gaussiansBuffer
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        u = view(160, 150, k=6, alpha_min=0.2, T_min=0.2).uniforms
+        out = c.device_alloc(160 * 150 * 16)
+        views = [(s, u, 160, 150, out)] * 40
+        ref = np.empty((150, 160, 4), np.float32)
+        with_lists = c.render_batch(views, device_outputs=True)[1]
+        c.memcpy(ref.ctypes.data, out, ref.nbytes, 1)
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        out = c.device_alloc(160 * 150 * 16)
+        views = [(s, u, 160, 150, out)] * 40
+        # 40 x 60,000 proxies: 1.5 GB of lists
+        ballast = c.device_alloc(torch.cuda.mem_get_info(0)[0] - (1 << 30))
+        launches = []
+        for _ in range(4):
+            n0 = c.launch_count()
+            st = c.render_batch(views, device_outputs=True)[1]
+            launches.append(c.launch_count() - n0)
+        img = np.empty_like(ref)
+        c.memcpy(img.ctypes.data, out, img.nbytes, 1)
+        assert np.array_equal(_bits(img), _bits(ref))
+        assert st["proxy_tests"] != with_lists["proxy_tests"]
+        assert launches[1:] == [1, 1, 1]
+        c.device_free(ballast)
+        again = c.render_batch(views, device_outputs=True)[1]
+        c.memcpy(img.ctypes.data, out, img.nbytes, 1)
+        assert np.array_equal(_bits(img), _bits(ref))
+        assert abs(again["proxy_tests"] - with_lists["proxy_tests"]) < 0.1 * with_lists["proxy_tests"]

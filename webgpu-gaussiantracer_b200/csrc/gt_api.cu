@@ -252,15 +252,34 @@ static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n, boo
 }
 
 // Buffers of the per-view proxy lists (gt_stream.cu) for a launch of these
-// views, grown as needed and kept by the context (at most kListBudget bytes).
-// Entries: 25 per proxy and view to begin with (a proxy meets 2 to 4 bins of a
+// views, grown as needed and kept by the context (at most kListBudget bytes for a
+// launch).  Entries: 25 per proxy and view to begin with (a proxy meets 2 to 4 bins of a
 // 1080p view of the 1M-Gaussian scene), more once a launch that did not have
 // room has left its need in Lists::need (it is read here without waiting, so
 // queued launches count too, and the largest is kept, so views may take turns);
-// the tiles of bins whose lists do not fit are traced by the warp-per-ray kernel.  Views the lists cannot serve, and
-// launches whose projection records or bins alone would take half the
-// budget, get none (the hierarchy kernels trace them).
+// the tiles of bins whose lists do not fit are traced by the warp-per-ray kernel.
+// Views the lists cannot serve, and launches whose projection records or bins
+// alone would take half the budget, get none (the hierarchy kernels trace them).
+// So do launches that need as much memory as could not be had before (a try
+// waits for the stream, drops the captured graphs and, where it fails, gives all
+// list buffers back), until the program frees memory of the context, or for
+// kListRetry launches.
 constexpr uint64_t kListBudget = 8ull << 30;
+constexpr uint32_t kListRetry = 256;
+
+static void free_lists(gt_context* ctx) {
+  Lists& L = ctx->lists;
+  for (void* p : {(void*)L.views, (void*)L.rec, (void*)L.box, (void*)L.range, (void*)L.cells, (void*)L.bin_base,
+                  (void*)L.order, (void*)L.ent_box, (void*)L.ent, (void*)L.spill, (void*)ctx->d_redo})
+    cudaFree(p);
+  uint32_t* need = L.need;
+  L = Lists{};
+  L.need = need;
+  ctx->d_redo = nullptr;
+  ctx->lists_views = 0;
+  ctx->lists_recs = ctx->lists_bins = ctx->redo_cap = 0;
+}
+
 static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
                               const LaunchShape& shape, Lists* out, Handoff* hand) {
   *out = Lists{};
@@ -287,59 +306,59 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
   const uint64_t most = std::min<uint64_t>((kListBudget - fixed) / kEnt, 1ull << 30);
   const uint32_t told = *reinterpret_cast<volatile uint32_t*>(ctx->lists.need);
   ctx->lists_need = std::max(ctx->lists_need, told);
-  const uint64_t need = std::max<uint64_t>(recs * 20 + (1u << 20), ctx->lists_need);
+  const uint64_t first = recs * 20 + (1u << 20);
+  uint64_t need = std::min(std::max<uint64_t>(first, ctx->lists_need), most);
+  auto bytes = [&] { return fixed + spare(rays) * sizeof(uint32_t) + need * kEnt; };
+  if (bytes() >= ctx->lists_denied && ++ctx->lists_skipped >= kListRetry) ctx->lists_denied = ~0ull;
+  if (bytes() >= ctx->lists_denied) need = std::min(first, most);
+  if (bytes() >= ctx->lists_denied) return GT_OK;
   const uint64_t want = std::min<uint64_t>(need + need / 4, most);
   Lists& L = ctx->lists;
-  if (n > ctx->lists_views || recs > ctx->lists_recs || bins > ctx->lists_bins || std::min(need, most) > L.cap ||
+  if (n > ctx->lists_views || recs > ctx->lists_recs || bins > ctx->lists_bins || need > L.cap ||
       rays > ctx->redo_cap) {
     cudaStreamSynchronize(ctx->stream);
     drop_graphs(ctx);  // captured graphs hold the old addresses
-    auto grow = [](auto** p, uint64_t count) {
+    cudaError_t e = cudaSuccess;
+    auto grow = [&e](auto** p, uint64_t count) {
+      if (e != cudaSuccess) return;
       cudaFree(*p);
       *p = nullptr;
-      return cudaMalloc(p, count * sizeof(**p));
+      e = cudaMalloc(p, count * sizeof(**p));
     };
-    cudaError_t e = cudaSuccess;
     if (n > ctx->lists_views) {
-      ctx->lists_views = 0;
-      const uint32_t c = n + n / 2;
-      e = grow(&L.views, c);
-      if (e == cudaSuccess) e = grow(&L.range, 2ull * c);
-      if (e == cudaSuccess) ctx->lists_views = c;
+      ctx->lists_views = n + n / 2;
+      grow(&L.views, ctx->lists_views);
+      grow(&L.range, 2ull * ctx->lists_views);
     }
-    if (e == cudaSuccess && recs > ctx->lists_recs) {
-      ctx->lists_recs = 0;
-      const uint64_t c = spare(recs);
-      e = grow(&L.rec, 2 * c);
-      if (e == cudaSuccess) e = grow(&L.box, c);
-      if (e == cudaSuccess) ctx->lists_recs = c;
+    if (recs > ctx->lists_recs) {
+      ctx->lists_recs = spare(recs);
+      grow(&L.rec, 2 * ctx->lists_recs);
+      grow(&L.box, ctx->lists_recs);
     }
-    if (e == cudaSuccess && bins > ctx->lists_bins) {
-      ctx->lists_bins = 0;
-      const uint64_t c = spare(bins);
-      e = grow(&L.cells, c << kListBucketBits);
-      if (e == cudaSuccess) e = grow(&L.bin_base, c + 1);
-      if (e == cudaSuccess) e = grow(&L.order, c);
-      if (e == cudaSuccess) ctx->lists_bins = c;
+    if (bins > ctx->lists_bins) {
+      ctx->lists_bins = spare(bins);
+      grow(&L.cells, ctx->lists_bins << kListBucketBits);
+      grow(&L.bin_base, ctx->lists_bins + 1);
+      grow(&L.order, ctx->lists_bins);
     }
-    if (e == cudaSuccess && std::min(need, most) > L.cap) {
-      L.cap = 0;
-      e = grow(&L.ent_box, want);
-      if (e == cudaSuccess) e = grow(&L.ent, want);
-      if (e == cudaSuccess) L.cap = (uint32_t)want;
+    if (need > L.cap) {
+      L.cap = (uint32_t)want;
+      grow(&L.ent_box, want);
+      grow(&L.ent, want);
     }
-    if (e == cudaSuccess && !L.spill) {  // 16 warps an SM of 32 rays each
-      const uint64_t b = (uint64_t)ctx->num_sms * 16u * kStreamSpill * 32u * sizeof(unsigned long long);
-      e = cudaMalloc(&L.spill, b);
-      if (e == cudaSuccess) L.spill_bytes = b;
+    if (!L.spill) {  // 16 warps an SM of 32 rays each
+      L.spill_bytes = (uint64_t)ctx->num_sms * 16u * kStreamSpill * 32u * sizeof(unsigned long long);
+      grow(&L.spill, L.spill_bytes / sizeof(unsigned long long));
     }
-    if (e == cudaSuccess && rays > ctx->redo_cap) {
-      ctx->redo_cap = 0;
-      e = grow(&ctx->d_redo, spare(rays));
-      if (e == cudaSuccess) ctx->redo_cap = spare(rays);
+    if (rays > ctx->redo_cap) {
+      ctx->redo_cap = spare(rays);
+      grow(&ctx->d_redo, ctx->redo_cap);
     }
     if (e != cudaSuccess) {  // (no room: the hierarchy kernels)
       (void)cudaGetLastError();
+      free_lists(ctx);
+      ctx->lists_denied = bytes();
+      ctx->lists_skipped = 0;
       return GT_OK;
     }
   }
@@ -558,10 +577,7 @@ extern "C" gt_status gt_context_destroy(gt_context* ctx) {
   cudaFreeHost(ctx->h_views);
   cudaFree(ctx->staging);
   cudaFree(ctx->colours);
-  for (void* p : {(void*)ctx->lists.views, (void*)ctx->lists.rec, (void*)ctx->lists.box, (void*)ctx->lists.range,
-                  (void*)ctx->lists.cells, (void*)ctx->lists.bin_base, (void*)ctx->lists.order, (void*)ctx->lists.ent_box,
-                  (void*)ctx->lists.ent, (void*)ctx->lists.spill, (void*)ctx->d_redo})
-    cudaFree(p);
+  free_lists(ctx);
   delete ctx->copy_pool;
   for (int b = 0; b < 2; ++b) {
     if (ctx->up_pinned[b]) cudaFreeHost(ctx->up_pinned[b]);
@@ -737,6 +753,7 @@ extern "C" gt_status gt_scene_destroy(gt_scene* s) {
   ctx->scenes.erase(s);
   free_scene(&s->b, ctx->stream);
   delete s;
+  ctx->lists_denied = ~0ull;
   return GT_OK;
 }
 
@@ -1411,6 +1428,7 @@ extern "C" gt_status gt_device_free(gt_context* ctx, void* ptr) {
   if (!ctx) return GT_ERR_INVALID_ARG;
   API_CUDA(ctx, cudaSetDevice(ctx->device));
   API_CUDA(ctx, cudaFree(ptr));
+  ctx->lists_denied = ~0ull;
   return GT_OK;
 }
 extern "C" gt_status gt_host_alloc(gt_context* ctx, uint64_t bytes, void** out) {

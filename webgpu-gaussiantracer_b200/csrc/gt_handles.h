@@ -71,6 +71,8 @@ struct gt_context {
   gt::Lists lists;                      // per-view proxy lists (gt_stream.cu)
   uint32_t lists_views = 0;             // capacities: views, projection records, bins, redo slots
   uint64_t lists_recs = 0, lists_bins = 0, redo_cap = 0;
+  uint64_t lists_denied = ~0ull;        // bytes of list buffers that could not be had
+  uint32_t lists_skipped = 0;           // launches that did without since
   uint32_t lists_need = 0;              // the most entries a launch needed without having room for them
   uint32_t* d_redo = nullptr;
   cudaEvent_t call0 = nullptr, call1 = nullptr, timer0 = nullptr, timer1 = nullptr;
