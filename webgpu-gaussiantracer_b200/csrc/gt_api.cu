@@ -640,8 +640,9 @@ static gt_status ensure_chunks(gt_context* ctx) {
 namespace gt {
 gt_status api_upload(gt_context* ctx, void* dev, const void* host, size_t bytes) {
   if (bytes == 0) return GT_OK;
-  const bool locked = page_locked(host);
-  if (bytes <= kDirectCopy || locked) {
+  // (a buffer locked in part takes the chunks: one copy cannot span its ends)
+  const bool locked = page_locked(host), tail = page_locked(static_cast<const unsigned char*>(host) + bytes - 1);
+  if (locked == tail && (locked || bytes <= kDirectCopy)) {
     API_CUDA(ctx, cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     // (a page-locked source is read by the DMA engine, not staged by the call)
     if (locked) API_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
