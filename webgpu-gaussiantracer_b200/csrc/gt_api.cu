@@ -796,6 +796,24 @@ extern "C" gt_status gt_scene_get_info(const gt_scene* s, gt_scene_info* info) {
 }
 
 // =============================================================== render
+// The device's address of a host buffer that is page-locked on this GPU from
+// its first byte to its last, else null.
+static void* mapped_whole(gt_context* ctx, const void* host, size_t bytes) {
+  const unsigned char* p = static_cast<const unsigned char*>(host);
+  void* dev[2] = {nullptr, nullptr};
+  for (int end = 0; end < 2; ++end) {
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, end ? p + bytes - 1 : p) != cudaSuccess) {
+      (void)cudaGetLastError();  // (an unknown pointer)
+      return nullptr;
+    }
+    if (pa.type != cudaMemoryTypeHost || pa.device != ctx->device || !pa.devicePointer) return nullptr;
+    dev[end] = pa.devicePointer;
+  }
+  return static_cast<unsigned char*>(dev[1]) - static_cast<unsigned char*>(dev[0]) == (ptrdiff_t)(bytes - 1) ? dev[0]
+                                                                                                             : nullptr;
+}
+
 static gt_status finish_call(gt_context* ctx, gt_render_stats* stats, uint64_t kslot) {
   API_CUDA(ctx, cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
   API_CUDA(ctx, cudaEventRecord(ctx->call1, ctx->stream));
@@ -836,15 +854,10 @@ extern "C" gt_status gt_render(gt_context* ctx, const gt_scene* scene, const gt_
   // renders take the staging buffer.
   bool direct = false;
   if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !(flags & GT_FLAG_CHECKPOINT)) {
-    cudaPointerAttributes pa;
-    if (cudaPointerGetAttributes(&pa, out_rgba) == cudaSuccess) {
-      if (pa.type == cudaMemoryTypeHost && pa.device == ctx->device && pa.devicePointer &&
-          (uintptr_t)pa.devicePointer % 16 == 0) {
-        out = reinterpret_cast<float4*>(pa.devicePointer);
-        direct = true;
-      }
-    } else {
-      (void)cudaGetLastError();  // (an unknown pointer: the staging path)
+    void* dev = mapped_whole(ctx, out_rgba, bytes);
+    if (dev && (uintptr_t)dev % 16 == 0) {
+      out = reinterpret_cast<float4*>(dev);
+      direct = true;
     }
   }
   if (!(flags & GT_FLAG_OUTPUT_DEVICE) && !direct) {
