@@ -404,37 +404,35 @@ constexpr float kCore = 896.0f;
 __global__ void __launch_bounds__(kCoreSamples) k_core(const float* box, uint64_t n, const uint32_t* flags,
                                                        const uint32_t* bounds_ord, float* core) {
   __shared__ float c[kCoreSamples];
-  const uint64_t step = (n + kCoreSamples - 1) / kCoreSamples, p = threadIdx.x * step;
-  const bool on = p < n && flags[p];
-  for (int a = 0; a < 3; ++a) {
-    float x = on ? 0.5f * (box[6 * p + a] + box[6 * p + 3 + a]) : CUDART_INF_F;
-    if (!(fabsf(x) < 1e30f)) x = CUDART_INF_F;
-    c[threadIdx.x] = x;
-    const int m = __syncthreads_count(x < 1e30f);
-    for (int k = 2; k <= kCoreSamples; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        const int i = threadIdx.x, o = i ^ j;
-        if (o > i && (c[i] > c[o]) == ((i & k) == 0)) {
-          const float t = c[i];
-          c[i] = c[o];
-          c[o] = t;
-        }
-        __syncthreads();
+  const int a = blockIdx.x, i = threadIdx.x;  // a block an axis
+  const uint64_t p = i * ((n + kCoreSamples - 1) / kCoreSamples);
+  float x = CUDART_INF_F;
+  if (p < n && flags[p]) x = 0.5f * (box[6 * p + a] + box[6 * p + 3 + a]);
+  if (!(fabsf(x) < 1e30f)) x = CUDART_INF_F;
+  c[i] = x;
+  const int m = __syncthreads_count(x < 1e30f);
+  for (int k = 2; k <= kCoreSamples; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const int o = i ^ j;
+      if (o > i && (c[i] > c[o]) == ((i & k) == 0)) {
+        const float t = c[i];
+        c[i] = c[o];
+        c[o] = t;
       }
-    if (threadIdx.x == 0) {
-      float lo = ord2f(bounds_ord[a]), hi = ord2f(bounds_ord[3 + a]);
-      if (m >= 32) {
-        const float q0 = c[m * 3 / 100], q1 = c[m - 1 - m * 3 / 100], more = 0.25f * (q1 - q0);
-        const float l = fmaxf(lo, q0 - more), h = fminf(hi, q1 + more);
-        if (h > l && 4.0f * (h - l) < hi - lo) {
-          lo = l;
-          hi = h;
-        }
-      }
-      core[a] = lo;
-      core[3 + a] = hi;
+      __syncthreads();
     }
-    __syncthreads();
+  if (i == 0) {
+    float lo = ord2f(bounds_ord[a]), hi = ord2f(bounds_ord[3 + a]);
+    if (m >= 32) {
+      const float q0 = c[m * 3 / 100], q1 = c[m - 1 - m * 3 / 100], more = 0.25f * (q1 - q0);
+      const float l = fmaxf(lo, q0 - more), h = fminf(hi, q1 + more);
+      if (h > l && 4.0f * (h - l) < hi - lo) {
+        lo = l;
+        hi = h;
+      }
+    }
+    core[a] = lo;
+    core[3 + a] = hi;
   }
 }
 
@@ -1033,7 +1031,7 @@ Err build_scene(const void* packed_dev, uint64_t n, uint32_t stride, double alph
   GT_CUDA_TRY(cudaMallocAsync(&keys, (size_t)m * 4, st));
   GT_CUDA_TRY(cudaMallocAsync(&vals, (size_t)m * 4, st));
   float* core = reinterpret_cast<float*>(bounds + 16);
-  k_core<<<1, kCoreSamples, 0, st>>>(box, n, flags, bounds, core);
+  k_core<<<3, kCoreSamples, 0, st>>>(box, n, flags, bounds, core);
   k_morton<<<grid_for(n, B), B, 0, st>>>(box, n, flags, slots, bounds, core, keys, vals);
   *launches += 2;
   GT_CUDA_TRY(cudaGetLastError());
