@@ -79,14 +79,9 @@ void make_face_table(FaceTable* F) {
   for (int i = 0; i < 12; ++i)
     r = fmaxf(r, sqrtf(v[3 * i] * v[3 * i] + v[3 * i + 1] * v[3 * i + 1] + v[3 * i + 2] * v[3 * i + 2]));
   F->r_circ = r;
-  float em = 0.0f;
-  for (int f = 0; f < 20; ++f) {
-    em = fmaxf(em, fabsf(F->e0[f][0]) + fabsf(F->e0[f][1]) + fabsf(F->e0[f][2]));
-    em = fmaxf(em, fabsf(F->e1[f][0]) + fabsf(F->e1[f][1]) + fabsf(F->e1[f][2]));
-  }
-  F->emax = em;
+  float c[20];  // plane offsets
   for (int f = 0; f < 20; ++f)
-    F->c[f] = F->n[f][0] * F->p0[f][0] + F->n[f][1] * F->p0[f][1] + F->n[f][2] * F->p0[f][2];
+    c[f] = F->n[f][0] * F->p0[f][0] + F->n[f][1] * F->p0[f][1] + F->n[f][2] * F->p0[f][2];
   // antipodal pairs: the face whose vertices are the negated vertices of f
   int q = 0;
   bool used[20] = {false};
@@ -118,16 +113,15 @@ void make_face_table(FaceTable* F) {
     bool same = q == 10;
     for (int r = 0; r < q && same; ++r) {
       for (int x = 0; x < 3; ++x) same = same && F->n[F->pa[r]][x] == want[r][x];
-      same = same && F->c[F->pa[r]] == F->c[0] && F->c[F->pb[r]] == F->c[0];
+      same = same && c[F->pa[r]] == c[0] && c[F->pb[r]] == c[0];
     }
     if (!same) q = 0;  // (the context is not created)
+    F->na = a;
+    F->nb = bb;
+    F->nc = cc;
+    F->plane = c[0];
   }
   F->npairs = q;
-  for (int r = 0; r < q; ++r) {
-    for (int a = 0; a < 3; ++a) F->pn[r][a] = F->n[F->pa[r]][a];
-    F->pca[r] = F->c[F->pa[r]];
-    F->pcb[r] = F->c[F->pb[r]];
-  }
   F->lim_steps = 0xFFFFFFFFu;
   F->lim_stack = kWarpStack;
   F->lim_rounds = kMaxRounds;

@@ -42,11 +42,9 @@ struct FaceTable {
   float n[20][3];
   float nmax;      // max |n| component over all faces
   float r_circ;    // circumradius of the vertex set
-  float emax;      // max L1 norm of the edge vectors e0, e1
-  float c[20];     // plane offsets n . p0 (pre-check only)
   int pa[10], pb[10];  // antipodal face pairs: n[pb[q]] == -n[pa[q]] bit for bit
-  float pn[10][3];     // n[pa[q]], pair-major: the unrolled candidate pass reads them
-  float pca[10], pcb[10];  // c[pa[q]], c[pb[q]]   at fixed parameter offsets
+  float na, nb, nc;    // components of the normals: (+-na, +-na, +-na) and the cyclic (0, +-nb, +-nc)
+  float plane;         // n . p0, the same of every face
   int npairs;          // 10 (checked when the context is created)
   // Device loop limits of the trace kernels (this table is a kernel
   // parameter, so they cost no registers).  gt_set_limits lowers them to

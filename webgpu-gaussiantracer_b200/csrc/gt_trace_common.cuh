@@ -116,7 +116,7 @@ __device__ __forceinline__ void proxy_any_face(const FaceTable& F, const float4*
 
 // n_q . v of the ten pairs' normals, up to rounding.
 __device__ __forceinline__ void pair_dots(const FaceTable& F, V3 v, float out[10]) {
-  const float a = F.pn[5][0], b = F.pn[1][1], c = F.pn[1][2];
+  const float a = F.na, b = F.nb, c = F.nc;
   const float ax = a * v.x, ay = a * v.y, az = a * v.z;
   const float s = ay + ax, t = ay - ax;
   out[0] = t + az;
@@ -180,7 +180,7 @@ __device__ __forceinline__ void proxy_faces(const FaceTable& F, const FaceRows& 
 #pragma unroll
   for (int q = 0; q < 10; ++q) {
     // distance of the origin in front of the pair's front face: -(c + s n.o)
-    num[q] = -__uint_as_float(__float_as_uint(num[q]) ^ (__float_as_uint(dn[q]) & 0x80000000u)) - F.pca[0];
+    num[q] = -__uint_as_float(__float_as_uint(num[q]) ^ (__float_as_uint(dn[q]) & 0x80000000u)) - F.plane;
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(dn[q])));
     const float t = num[q] * r;
