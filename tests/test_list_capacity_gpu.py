@@ -135,3 +135,31 @@ def test_lists_that_cannot_be_had():
         c.memcpy(img.ctypes.data, out, img.nbytes, 1)
         assert np.array_equal(_bits(img), _bits(ref))
         assert abs(again["proxy_tests"] - with_lists["proxy_tests"]) < 0.1 * with_lists["proxy_tests"]
+
+
+def test_lists_make_room_for_other_buffers():
+    """With little memory left, a buffer of the program's own, then a larger
+    image, are had at the lists' cost; views and gradients stay the same."""
+    import torch
+    rec = small_scene(n=60_000, seed=94).gaussiansBuffer
+    w, h = 160, 150
+    u = view(w, h, k=6, alpha_min=0.2, T_min=0.2).uniforms
+    g = np.random.default_rng(94).normal(size=(h, w, 4)).astype(np.float32)
+    with Context(0) as c:
+        s = Scene(c, rec, 0.01)
+        out = c.device_alloc(w * h * 16)
+        views = [(s, u, w, h, out)] * 40
+        ballast = c.device_alloc(torch.cuda.mem_get_info(0)[0] - (3 << 30))
+        ref = c.render(s, u, w, h)
+        grad = c.backward(s, u, w, h, g, mode=1)[0]
+        assert c.render_batch(views, device_outputs=True)[1]["rays"] == 40 * w * h  # (1.5 GB of lists)
+        more = c.device_alloc(torch.cuda.mem_get_info(0)[0] + (1 << 29))
+        img = np.empty_like(ref)
+        assert c.render_batch(views, device_outputs=True)[1]["rays"] == 40 * w * h
+        c.memcpy(img.ctypes.data, out, img.nbytes, 1)
+        assert np.array_equal(_bits(img), _bits(ref))
+        got = c.backward(s, u, w, h, g, mode=1)[0]
+        assert np.abs(got - grad).max() <= 1e-4 * np.abs(grad).max()  # (sums in another order)
+        c.device_free(more)
+        c.device_free(ballast)
+        s.close()

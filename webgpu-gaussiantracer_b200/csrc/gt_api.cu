@@ -144,6 +144,35 @@ static void drop_graphs(gt_context* ctx) {
   ctx->graphs.clear();
 }
 
+static void free_lists(gt_context* ctx) {
+  Lists& L = ctx->lists;
+  for (void* p : {(void*)L.views, (void*)L.rec, (void*)L.box, (void*)L.range, (void*)L.cells, (void*)L.bin_base,
+                  (void*)L.order, (void*)L.ent_box, (void*)L.ent, (void*)L.spill, (void*)ctx->d_redo})
+    cudaFree(p);
+  uint32_t* need = L.need;
+  L = Lists{};
+  L.need = need;
+  ctx->d_redo = nullptr;
+  ctx->lists_bytes = ~0ull;
+  ctx->lists_views = 0;
+  ctx->lists_recs = ctx->lists_bins = ctx->redo_cap = 0;
+}
+
+// cudaMalloc, with the list buffers given back where there is no room otherwise
+// (launches then do without them until memory is freed).  Not to be called
+// between ensure_lists and the launch that has its pointers.
+static cudaError_t dev_alloc(gt_context* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !ctx->lists.cap) return e;
+  (void)cudaGetLastError();
+  ctx->lists_denied = ctx->lists_bytes;
+  ctx->lists_skipped = 0;
+  cudaStreamSynchronize(ctx->stream);
+  drop_graphs(ctx);  // captured graphs hold the old addresses
+  free_lists(ctx);
+  return cudaMalloc(p, bytes);
+}
+
 // Handoff buffer for a launch of `rays` rays: room for a quarter of them, at
 // most 4M rays (128 MB); a packet whose rays do not fit keeps tracing them
 // itself, so the cap changes only how the tail of a large batch is shared.
@@ -157,7 +186,7 @@ static gt_status ensure_handoff(gt_context* ctx, uint64_t rays, Handoff* out) {
     cudaFree(ctx->d_handoff);
     ctx->d_handoff = nullptr;
     ctx->handoff_cap = 0;
-    API_CUDA(ctx, cudaMalloc(&ctx->d_handoff, sizeof(HandoffRay) * (size_t)want));
+    API_CUDA(ctx, dev_alloc(ctx, (void**)&ctx->d_handoff, sizeof(HandoffRay) * (size_t)want));
     ctx->handoff_cap = want;
   }
   out->rays = ctx->d_handoff;
@@ -175,7 +204,7 @@ static gt_status ensure_views(gt_context* ctx, uint32_t n) {
     cudaFree(ctx->d_views);
     ctx->d_views = nullptr;
     uint32_t cap = std::max<uint32_t>(n, 2 * ctx->d_views_cap);
-    API_CUDA(ctx, cudaMalloc(&ctx->d_views, sizeof(ViewDev) * cap));
+    API_CUDA(ctx, dev_alloc(ctx, (void**)&ctx->d_views, sizeof(ViewDev) * cap));
     ctx->d_views_cap = cap;
   }
   if (n > ctx->h_views_cap) {
@@ -193,7 +222,7 @@ static gt_status ensure_staging(gt_context* ctx, size_t bytes) {
     cudaFree(ctx->staging);
     ctx->staging = nullptr;
     ctx->staging_bytes = 0;
-    API_CUDA(ctx, cudaMalloc(&ctx->staging, bytes));
+    API_CUDA(ctx, dev_alloc(ctx, (void**)&ctx->staging, bytes));
     ctx->staging_bytes = bytes;
   }
   return GT_OK;
@@ -266,19 +295,6 @@ static gt_status assign_colours(gt_context* ctx, ViewDev* views, uint32_t n, boo
 // kListRetry launches.
 constexpr uint64_t kListBudget = 8ull << 30;
 constexpr uint32_t kListRetry = 256;
-
-static void free_lists(gt_context* ctx) {
-  Lists& L = ctx->lists;
-  for (void* p : {(void*)L.views, (void*)L.rec, (void*)L.box, (void*)L.range, (void*)L.cells, (void*)L.bin_base,
-                  (void*)L.order, (void*)L.ent_box, (void*)L.ent, (void*)L.spill, (void*)ctx->d_redo})
-    cudaFree(p);
-  uint32_t* need = L.need;
-  L = Lists{};
-  L.need = need;
-  ctx->d_redo = nullptr;
-  ctx->lists_views = 0;
-  ctx->lists_recs = ctx->lists_bins = ctx->redo_cap = 0;
-}
 
 static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint32_t total_tiles, uint64_t rays,
                               const LaunchShape& shape, Lists* out, Handoff* hand) {
@@ -361,6 +377,7 @@ static gt_status ensure_lists(gt_context* ctx, ViewDev* views, uint32_t n, uint3
       ctx->lists_skipped = 0;
       return GT_OK;
     }
+    ctx->lists_bytes = std::min(ctx->lists_bytes, bytes());
   }
   *out = L;
   out->shift = plan.shift;
@@ -405,6 +422,7 @@ static ViewDev make_view(const gt_scene* s, const gt_uniforms& u, uint32_t w, ui
 }
 
 namespace gt {
+cudaError_t api_alloc(gt_context* ctx, void** p, size_t bytes) { return dev_alloc(ctx, p, bytes); }
 gt_status api_fail(gt_context* ctx, gt_status code, const std::string& msg) { return fail(ctx, code, msg); }
 gt_status api_status_to_error(gt_context* ctx, uint32_t status) { return status_to_error(ctx, status); }
 gt_status api_check_uniforms(gt_context* ctx, const gt_uniforms* u) { return check_uniforms(ctx, u); }
@@ -1435,7 +1453,7 @@ extern "C" gt_status gt_autotune_reset(gt_context* ctx) {
 extern "C" gt_status gt_device_alloc(gt_context* ctx, uint64_t bytes, void** out) {
   if (!ctx || !out) return fail(ctx, GT_ERR_INVALID_ARG, "NULL argument");
   API_CUDA(ctx, cudaSetDevice(ctx->device));
-  API_CUDA(ctx, cudaMalloc(out, bytes ? bytes : 1));
+  API_CUDA(ctx, dev_alloc(ctx, out, bytes ? bytes : 1));
   return GT_OK;
 }
 extern "C" gt_status gt_device_free(gt_context* ctx, void* ptr) {

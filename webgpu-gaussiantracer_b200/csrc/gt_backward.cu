@@ -692,7 +692,7 @@ gt_status grow(gt_context* ctx, void** p, size_t* have, size_t bytes) {
   *p = nullptr;
   *have = 0;
   const size_t want = bytes + bytes / 4;
-  CK_TRY(cudaMalloc(p, want ? want : 16));
+  CK_TRY(api_alloc(ctx, p, want ? want : 16));
   *have = want;
   return GT_OK;
 }
@@ -755,9 +755,6 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
   if (sst != GT_OK) return sst;
   sst = api_assign_colours(ctx, vd.data(), count);  // as a plain render's
   if (sst != GT_OK) return sst;
-  Lists lists;
-  sst = api_ensure_lists(ctx, vd.data(), count, total_tiles, rays, shape, &lists, &hand);
-  if (sst != GT_OK) return sst;
   for (int attempt = 0; attempt < 3; ++attempt) {
     if (want > 0xFFFFFFF0ull) return api_fail(ctx, GT_ERR_OOM, "checkpoint needs more than 2^32 records");
     if (own_budget && want * (kCkptHeader + kCkptChunk) * 4 > budget) {
@@ -774,6 +771,9 @@ gt_status api_forward_ckpt(gt_context* ctx, const gt_scene* const* scenes, const
     uint32_t m = mode == 1 ? 1u : (mode == 2 ? 2u : (want * (kCkptHeader + kCkptChunk) * 4 <= budget ? 1u : 2u));
     const uint32_t kc = m == 1 ? kCkptChunk : 0u;
     sst = grow(ctx, (void**)&ck.pool, &ck.pool_bytes, want * (kCkptHeader + kc) * 4);
+    if (sst != GT_OK) return sst;
+    Lists lists;  // (after every allocation of the launch: these may take the lists' room)
+    sst = api_ensure_lists(ctx, vd.data(), count, total_tiles, rays, shape, &lists, &hand);
     if (sst != GT_OK) return sst;
     Ckpt c;
     c.head = ck.head;

@@ -72,6 +72,7 @@ struct gt_context {
   uint32_t lists_views = 0;             // capacities: views, projection records, bins, redo slots
   uint64_t lists_recs = 0, lists_bins = 0, redo_cap = 0;
   uint64_t lists_denied = ~0ull;        // bytes of list buffers that could not be had
+  uint64_t lists_bytes = ~0ull;         // the least that a launch needed since the buffers are held
   uint32_t lists_skipped = 0;           // launches that did without since
   uint32_t lists_need = 0;              // the most entries a launch needed without having room for them
   uint32_t* d_redo = nullptr;
@@ -101,6 +102,7 @@ struct gt_scene {
 
 namespace gt {
 // shared by the C-ABI translation units (gt_api.cu)
+cudaError_t api_alloc(gt_context* ctx, void** p, size_t bytes);
 gt_status api_fail(gt_context* ctx, gt_status code, const std::string& msg);
 gt_status api_status_to_error(gt_context* ctx, uint32_t status);
 gt_status api_check_uniforms(gt_context* ctx, const gt_uniforms* u);
