@@ -148,7 +148,7 @@ struct LaunchShape {
   // hierarchy (gt_packet.cu) when packet is 1, one warp per ray when it is 0.
   // By default (2) they run over per-view proxy lists (gt_stream.cu) when the
   // launch has lists, else as tile packets when it has at least
-  // kPacketTilesPerSm tiles per SM.  The packet kernel's k-buffer has
+  // kPacketTilesPerSm tiles per SM within the image of the scene's box.  The packet kernel's k-buffer has
   // packet_kbuf entries per ray (raised to k; <= kMaxPacketKbuf).
   uint32_t packet = 2;
   uint32_t packet_kbuf = 32;
