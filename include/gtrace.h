@@ -141,7 +141,7 @@ uint32_t gt_version(void);
  * request of src/main.ts:396-427.  Besides its scenes, a context keeps the
  * scratch of its largest call so far: staging images, the hand-off buffer,
  * checkpoints, the proxy lists of views they serve (48 bytes a proxy and view,
- * 4 KB a bin, 24 bytes a list entry, 25 entries a proxy to begin with, 57 MB of
+ * 4 KB a bin, 24 bytes a list entry, 25 entries a proxy to begin with, 136 MB of
  * waiting hits, 4 bytes a ray; records and bins take at most 4 GiB and all lists at
  * most 8 GiB of one launch, and each of these buffers is kept at its largest), and
  * the colour tables of plain renders (16

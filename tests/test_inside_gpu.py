@@ -65,3 +65,29 @@ def test_proxies_across_and_beside_the_camera_plane(ctx, seed, hfov):
     img = ctx.render(s, u, w, h)
     s.close()
     assert np.array_equal(_bits(img), oracle.Scene(rec, 0.01, "f32").render(u, w, h)[0].view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h", [(200, 150), (330, 300)])
+def test_dense_scenes_stay_with_the_lists(ctx, w, h):
+    """Large proxies all around the camera, many of them about it: between 128 and
+    256 hits of every ray wait for the last of these, and its column holds them."""
+    rng = np.random.default_rng(710)
+    n = 20000
+    rec = np.zeros((n, 80), np.float32)
+    rec[:, 0:3] = np.clip(rng.normal(size=(n, 3)), -3, 3)
+    rec[:, 4:7] = np.exp(rng.uniform(-4.5, -2.5, size=(n, 3))) * 4.0
+    q = rng.normal(size=(n, 4))
+    rec[:, 8:12] = q / np.linalg.norm(q, axis=1, keepdims=True)
+    rec[:, 12] = rng.uniform(0.05, 0.99, size=n)
+    rec[:, 16:19] = rng.normal(size=(n, 3))
+    s = Scene(ctx, rec, 0.01)
+    u = view(w, h, pos=(0.0, 0.0, 0.0), target=(1.0, 0.2, -1.0), k=6).uniforms
+    img, st = ctx.render(s, u, w, h, stats=True)
+    ctx.set_tune(s, u, w, h, block_threads=128, kbuf=64, blocks_per_sm=8)
+    try:
+        ref = ctx.render(s, u, w, h)
+    finally:
+        ctx._lib.gt_autotune_reset(ctx._h)
+        s.close()
+    assert np.array_equal(_bits(img), _bits(ref))
+    assert st["handed"] < 0.5 * w * h

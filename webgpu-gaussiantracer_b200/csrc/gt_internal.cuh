@@ -271,7 +271,7 @@ struct Handoff {
 
 // Per-view proxy lists (gt_stream.cu).
 constexpr int kListBucketBits = 10;                // distance buckets per bin
-constexpr int kStreamSpill = 96;                   // rows of a ray's column in global memory
+constexpr int kStreamSpill = 224;                  // rows of a ray's column in global memory
 constexpr uint64_t kStreamMaxSlots = 1ull << 28;   // larger launches use the hierarchy kernels
 struct ListView {
   double X[3], Y[3], Z[3];  // camera frame: right, up, view direction

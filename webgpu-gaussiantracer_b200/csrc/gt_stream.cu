@@ -585,7 +585,12 @@ __device__ __forceinline__ float s_key_t(unsigned long long k) {
 
 // Rows of a ray's column: the first kStreamKb in shared memory, the next
 // kStreamSpill (rays with many hits at nearly one distance, a few in a
-// hundred) in the warp's part of a global buffer.
+// hundred; all rays of a dense scene whose proxies surround the camera, where no
+// hit is final before the last of these is tested) in the warp's part of a global
+// buffer.  96 / 224 / 480 rows: 1M uniform Gaussians from their centre, 960x540,
+// 82.7 / 12.8 / 12.9 ms (hierarchy kernels 57.1), 31k of four times the size
+// 100 / 22.8 / 19.0, 1M clusters from (4, 1, 3) 5.36 / 4.09 / 3.38; views from
+// outside are the same.  224 rows take 136 MB.
 template <int R>
 __device__ __forceinline__ unsigned long long* stream_row(StreamScratch<R>& W, unsigned long long* sp, uint32_t i,
                                                           uint32_t r) {
